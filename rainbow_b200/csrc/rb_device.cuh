@@ -127,6 +127,29 @@ __device__ __forceinline__ void prox_sphere(double zs, double zt, double ztau, d
     o[0] = zs * scale; o[1] = zt * scale; o[2] = ztau * scale;
 }
 
+// a / sqrt(v) with both operations rounded to nearest, as one chain without calls: from the hardware's estimate
+// of 1 / sqrt(v), Goldschmidt's coupled iteration for sqrt(v) and 1 / (2 sqrt(v)) with the final correction by the
+// exact residual, then one Newton step to the rounded reciprocal of the root and the quotient corrected by its exact
+// residual (Markstein, IBM J. Res. Dev. 34, 1990; Cornea, Harrison, Tang, 2002).  Operands outside 2^+-500, zeros and
+// NaN among them, take the plain operations.
+__device__ __forceinline__ double ratio_sqrt(double a, double v) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+    double g = v * y, h = 0.5 * y;
+    double r = fma(-g, h, 0.5);
+    g = fma(g, r, g); h = fma(h, r, h);
+    r = fma(-g, h, 0.5);
+    g = fma(g, r, g); h = fma(h, r, h);
+    const double root = fma(fma(-g, g, v), h, g);
+    y = h + h;
+    y = fma(fma(-root, y, 1.0), y, y);
+    double q = a * y;
+    q = fma(fma(-root, q, a), y, q);
+    const unsigned ev = (unsigned)__double2hiint(v) - 0x20b00000u, ea = (unsigned)__double2hiint(a) - 0x20b00000u;
+    if (max(ev, ea) > 0x3e800000u) q = a / sqrt(v);   // (exponent field + 500 - 1023) of either beyond 1000
+    return q;
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // Signed distance grid (grid3.py)
 // ---------------------------------------------------------------------------------------------------------

@@ -23,6 +23,7 @@
 // device counters; kernels that depend on them run grid-stride loops over those counters.
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdio>
 #include <algorithm>
 #include <atomic>
@@ -764,6 +765,24 @@ __device__ __forceinline__ double jrow_dot(const double* Jr, const double* wlo, 
     return s;
 }
 
+// Layout of a contact's 4 x 12 blocks of J and of W J^T (48 doubles, columns: six of the lo body, six of the hi
+// body).  The solver reads them by quads: lane q takes row q of J, and of W J^T the columns 2q, 2q + 1 and 8 + q in
+// all four rows, 12 doubles each as six 16-byte pieces.  Piece j of the four lanes is contiguous (64 bytes), so a
+// warp's load of one piece touches one line per contact; with rows stored whole the 32 lanes fell on up to 28 lines
+// (4096-body lattice, eight warps sweeping: 4948 against 4193 cycles a level; one warp on the 32-box tower is the
+// same either way).
+__device__ __forceinline__ int j_at(int row, int col) { return 8 * (col >> 1) + 2 * row + (col & 1); }
+__device__ __forceinline__ int w_at(int row, int col) {
+    const int q = col < 8 ? col >> 1 : col - 8, p = col < 8 ? col & 1 : 2;
+    return 16 * p + 8 * (row >> 1) + 2 * q + (row & 1);
+}
+// column col of W J^T (rows 0..3) as two 16-byte pieces
+__device__ __forceinline__ void w_column(const double* WJT, int k, int col, double* o) {
+    const double2* W = reinterpret_cast<const double2*>(WJT + 48 * (size_t)k + w_at(0, col));
+    const double2 t = W[0], u = W[4];
+    o[0] = t.x; o[1] = t.y; o[2] = u.x; o[3] = u.y;
+}
+
 __global__ void k_contacts(const StepArgs a) {
     // one thread per (contact, row): row q's J and W J^T blocks, b, Delassus diagonal, r and start impulse;
     // the row-0 thread also writes the contact's body pair and mu
@@ -780,11 +799,7 @@ __global__ void k_contacts(const StepArgs a) {
         d3 vs, vt, vn;
         make_orthonormal_vectors(ld3(a.out.contact_n + 3 * k), vs, vt, vn);   // (t, b, n)
         const int lo = min(A, B), hi = max(A, B);
-        const int offA = (A == lo) ? 0 : 6, offB = (B == lo) ? 0 : 6;
-        double* J = a.ws.J + 48 * (size_t)k + 12 * row;
-        double* W = a.ws.WJT + 48 * (size_t)k + 12 * row;
-        double* JA = J + offA;
-        double* JB = J + offB;
+        double JA[6], JB[6], J[12], W[12];
         if (row < 3) {   // contacts.py:140-147
             const d3 d = row == 0 ? vn : (row == 1 ? vs : vt);
             const d3 ca = cross_np(rA, d), cb = cross_np(rB, d);
@@ -794,7 +809,10 @@ __global__ void k_contacts(const StepArgs a) {
             JA[0] = -0.0; JA[1] = -0.0; JA[2] = -0.0; JA[3] = -vn.x; JA[4] = -vn.y; JA[5] = -vn.z;
             JB[0] = 0.0; JB[1] = 0.0; JB[2] = 0.0; JB[3] = vn.x; JB[4] = vn.y; JB[5] = vn.z;
         }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) { J[i] = A == lo ? JA[i] : JB[i]; J[6 + i] = A == lo ? JB[i] : JA[i]; }
         bool hasw[2];
+#pragma unroll
         for (int side = 0; side < 2; ++side) {   // WJT = W J^T (bsr_matmat order)
             const int bb = side ? hi : lo;
             hasw[side] = !a.bd.fixed[bb];
@@ -802,6 +820,7 @@ __global__ void k_contacts(const StepArgs a) {
             const double* Wi = a.ws.Winv + 9 * bb;
             const double* Jr = J + 6 * side;
             double* Wr = W + 6 * side;
+#pragma unroll
             for (int i = 0; i < 3; ++i) {
                 double s = 0.0;
                 s += (i == 0 ? m : 0.0) * Jr[0];
@@ -814,6 +833,14 @@ __global__ void k_contacts(const StepArgs a) {
                 Wr[i] = hasw[side] ? s : 0.0;
                 Wr[3 + i] = hasw[side] ? tt : 0.0;
             }
+        }
+        {
+            double2* Jk = reinterpret_cast<double2*>(a.ws.J + 48 * (size_t)k + j_at(row, 0));
+#pragma unroll
+            for (int j = 0; j < 6; ++j) Jk[4 * j] = make_double2(J[2 * j], J[2 * j + 1]);
+            double* Wk = a.ws.WJT + 48 * (size_t)k;
+#pragma unroll
+            for (int c = 0; c < 12; ++c) Wk[w_at(row, c)] = W[c];
         }
         // b = (1 + e) v + J (dt W f_ext) + g   (contacts.py:46)
         const int sc = scene_of(a.bd.scene_start, a.bd.n_scenes, A);
@@ -842,6 +869,7 @@ __global__ void k_contacts(const StepArgs a) {
         // Delassus diagonal: reduceat over the nonzero products J .* WJT^T in column order (contacts.py:49)
         double prods[12];
         int m = 0;
+#pragma unroll
         for (int c = 0; c < 12; ++c) {
             if (!hasw[c / 6]) continue;
             const double pr = J[c] * W[c];
@@ -919,48 +947,49 @@ __global__ void k_preds_init(const StepArgs a) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * K; i += gridDim.x * blockDim.x) a.ws.cpred[i] = -1;
 }
 
-// w[b] = (WJT x) rows of body b: sequential over its contacts (ascending) and their 4 columns.  The loads of
-// four contacts are issued before their products are accumulated (in order) to overlap their latency.
-__device__ __forceinline__ void body_wjt_dot(const Workspace& ws, int b, const double* x, double* out6) {
-    double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    const int e0 = ws.bc_ptr[b], e1 = ws.bc_ptr[b + 1];
+// component d of (WJT x) of a body, over its contacts bc_list[e0 .. e1): sequential over the contacts (ascending)
+// and their four rows.  The loads of four contacts are issued before their products are accumulated in order.
+__device__ __forceinline__ double body_wjt_dot(const Workspace& ws, int e0, int e1, int d, const double* x) {
+    double s = 0.0;
     int e = e0;
     for (; e + 4 <= e1; e += 4) {
         int code[4];
+        double W[4][4], xv[4][4];
+#pragma unroll
         for (int j = 0; j < 4; ++j) code[j] = ws.bc_list[e + j];
-        double xv[4][4];
-        const double* Wk[4];
+#pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int k = code[j] >> 1;
-            Wk[j] = ws.WJT + 48 * (size_t)k + 6 * (code[j] & 1);
-            for (int i = 0; i < 4; ++i) xv[j][i] = x[4 * k + i];
+            w_column(ws.WJT, k, 6 * (code[j] & 1) + d, W[j]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) xv[j][q] = x[4 * (size_t)k + q];
         }
-        for (int d = 0; d < 6; ++d) {
-            double t = s[d];
-            for (int j = 0; j < 4; ++j) {
-                t += Wk[j][d] * xv[j][0];
-                t += Wk[j][12 + d] * xv[j][1];
-                t += Wk[j][24 + d] * xv[j][2];
-                t += Wk[j][36 + d] * xv[j][3];
-            }
-            s[d] = t;
-        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s += W[j][q] * xv[j][q];
     }
     for (; e < e1; ++e) {
-        const int code = ws.bc_list[e];
-        const int k = code >> 1, side = code & 1;
-        const double* Wk = ws.WJT + 48 * (size_t)k + 6 * side;
-        const double x0 = x[4 * k], x1 = x[4 * k + 1], x2 = x[4 * k + 2], x3 = x[4 * k + 3];
-        for (int d = 0; d < 6; ++d) {
-            double t = s[d];
-            t += Wk[d] * x0;
-            t += Wk[12 + d] * x1;
-            t += Wk[24 + d] * x2;
-            t += Wk[36 + d] * x3;
-            s[d] = t;
-        }
+        const int code = ws.bc_list[e], k = code >> 1;
+        double W[4];
+        w_column(ws.WJT, k, 6 * (code & 1) + d, W);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s += W[q] * x[4 * (size_t)k + q];
     }
-    for (int d = 0; d < 6; ++d) out6[d] = s[d];
+    return s;
+}
+// six lanes of a warp per body, one velocity component each: this lane's body (-1: none) and component
+__device__ __forceinline__ int body_of_six(int n_bodies, int& d) {
+    const int lane = threadIdx.x & 31, slot = lane / 6;
+    d = lane - 6 * slot;
+    const int b = 5 * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) + slot;
+    return slot < 5 && b < n_bodies ? b : -1;
+}
+// the six components held by the lanes of this lane's body
+__device__ __forceinline__ void gather_six(double v, double* o) {
+    const int lane = threadIdx.x & 31, base = min(lane / 6, 4) * 6;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) o[i] = __shfl_sync(0xffffffffu, v, base + i);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -995,6 +1024,16 @@ struct WarpGroup {
         for (int o = 16; o > 0; o >>= 1) v = ::max(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
     }
+    // collect: the members whose flag is set take consecutive places after the n taken so far (every member
+    // calls it the same number of times); n is then the number taken in all
+    __device__ __forceinline__ int append_begin() const { return 0; }
+    __device__ __forceinline__ int append(bool flag, int& n) const {
+        const unsigned bal = __ballot_sync(0xffffffffu, flag);
+        const int at = n + __popc(bal & lanemask_lt());
+        n += __popc(bal);
+        return at;
+    }
+    __device__ __forceinline__ void append_end(int&) const { __syncwarp(); }
 };
 
 struct BlockGroup {
@@ -1026,60 +1065,392 @@ struct BlockGroup {
         __syncthreads();
         return m;
     }
+    __device__ int append_begin() const {
+        __syncthreads();
+        if (threadIdx.x == 0) ired[32] = 0;
+        __syncthreads();
+        return 0;
+    }
+    __device__ int append(bool flag, int&) const {
+        const unsigned bal = __ballot_sync(0xffffffffu, flag);
+        int at = 0;
+        if (bal && (threadIdx.x & 31) == 0) at = atomicAdd(ired + 32, __popc(bal));
+        return __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanemask_lt());
+    }
+    __device__ void append_end(int& n) const {
+        __syncthreads();
+        n = ired[32];
+        __syncthreads();
+    }
 };
 
-// Body accumulators w = WJT x of one scene: in shared memory when the scene fits, else in global memory.
-struct WView {
-    double* base;
-    int b0;
-    __device__ __forceinline__ double* at(int b) const { return base + 6 * (b - b0); }
+// the first `threads` threads of a block (a multiple of 32), with a barrier of their own
+struct SubGroup {
+    int threads;
+    __device__ __forceinline__ int rank() const { return threadIdx.x; }
+    __device__ __forceinline__ int size() const { return threads; }
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 };
 
-// w for every body of the scene from x (sequential over the body's contacts: the order of WJT.dot(x))
+// The working set of one scene's FP64 solve.  Only the free bodies with contacts have accumulators w = WJT x that
+// change; they are numbered ("slots", in any order) and their accumulators lie together, in shared memory when they
+// fit, else in global memory, followed by one zero slot that stands for every fixed body (a scene whose contacts
+// touch a fixed body has at most nb - 1 free ones, so nb slots hold them all).  In a lattice of 4096 bodies 547
+// contacts touch 302 of them.
+//   span  per slot the body's range in bc_list (at the scene's place of the w2 array)
+//   meta  per contact, in level order: contact, 6 x the slots of its lo and hi bodies, flags (bit 0 / 1: lo / hi is
+//         free; bit 2: an idle quad's stand-in), in the compact FP32 rows' room (c32), which no FP64 solve reads
+//   steps the sweep's sequence of steps, after the metas there (a meta and a step take 24 of a row's 208 bytes)
+struct Solve64 {
+    double* w;
+    const int2* span;
+    const int4* meta;
+    const int2* steps;
+    const int32_t* bc_list;
+    const double *J, *WJT, *mu;
+    int K, n_touched, n_steps;
+    int warps;       // warps that sweep (a block's; 1 for a warp)
+    bool w_shared;   // w lies in shared memory
+};
+constexpr int kMetaIdle = 4;
+constexpr int kStepEnds = 1 << 16;
+// accumulators i and i + 1 (i even), and single ones, by their own space's loads and stores
+template <bool kShared>
+struct W64 {
+    double* w;
+    uint32_t s;
+    __device__ __forceinline__ explicit W64(double* p) : w(p), s(kShared ? (uint32_t)__cvta_generic_to_shared(p) : 0u) {}
+    __device__ __forceinline__ double2 pair(int i) const {
+        double2 v;
+        if (kShared) asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(s + 8 * i) : "memory");
+        else v = *reinterpret_cast<const double2*>(w + i);
+        return v;
+    }
+    __device__ __forceinline__ double one(int i) const {
+        double v;
+        if (kShared) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(s + 8 * i) : "memory");
+        else v = w[i];
+        return v;
+    }
+    __device__ __forceinline__ void set(int i, double v) const {
+        if (kShared) asm volatile("st.shared.f64 [%0], %1;" ::"r"(s + 8 * i), "d"(v) : "memory");
+        else w[i] = v;
+    }
+    __device__ __forceinline__ void set(int i, double2 v) const {
+        if (kShared) asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(s + 8 * i), "d"(v.x), "d"(v.y) : "memory");
+        else *reinterpret_cast<double2*>(w + i) = v;
+    }
+};
+
+// numbers the scene's touched bodies: their spans, and body -> slot in bc_fill (free once bc_list is filled)
 template <class G>
-__device__ __forceinline__ void scene_wjt(const StepArgs& a, const G& g, const SceneRange& R, const double* x, WView w) {
-    for (int bb = R.b0 + g.rank(); bb < R.b1; bb += g.size()) {
-        double* o = w.at(bb);
-        if (a.bd.fixed[bb]) { for (int d = 0; d < 6; ++d) o[d] = 0.0; continue; }
-        body_wjt_dot(a.ws, bb, x, o);
+__device__ __forceinline__ int scene_touched(const StepArgs& a, const G& g, const SceneRange& R) {
+    int2* span = reinterpret_cast<int2*>(a.ws.w2 + 6 * (size_t)R.b0);
+    int n = g.append_begin();
+    for (int base = R.b0; base < R.b1; base += g.size()) {
+        const int bb = base + g.rank();
+        const int e0 = bb < R.b1 ? a.ws.bc_ptr[bb] : 0, e1 = bb < R.b1 ? a.ws.bc_ptr[bb + 1] : 0;
+        const int at = g.append(e1 > e0, n);   // fixed bodies have no list entries
+        if (e1 > e0) { span[at] = make_int2(e0, e1); a.ws.bc_fill[bb] = at; }
+    }
+    g.append_end(n);
+    return n;
+}
+
+// Warps that sweep a scene, eight contacts each: the number with the least cost over the scene's levels (ptr), a step
+// (a run of a level's contacts that the warps take at once) costing 1150 cycles with one warp and 100 more for every
+// further one: their FP64 and load instructions hold one another up even where they have no contact (64-box
+// lattice: 1420 with three; 4096-body lattice: 1870 with eight).  Every warp of the group counts for itself.
+__device__ __forceinline__ int sweep_warps(const int* ptr, int L, int max_warps) {
+    int steps[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int l = threadIdx.x & 31; l < L; l += 32) {
+        const int n = ptr[l + 1] - ptr[l];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) steps[w] += (n + 8 * w + 7) / (8 * w + 8);
+    }
+    int best = 1, cost = INT_MAX;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        const int c = __reduce_add_sync(0xffffffffu, steps[w]) * (23 + 2 * w);
+        if (w < max_warps && c < cost) { cost = c; best = w + 1; }
+    }
+    return best;
+}
+
+// the scene's working set once its contact order is known (L levels; 0: ascending order, no sweeps); w_smem holds
+// smem_bodies accumulators
+template <class G>
+__device__ __forceinline__ Solve64 scene_setup64(const StepArgs& a, const G& g, const SceneRange& R, int s, int L,
+                                                 double* w_smem, int smem_bodies) {
+    const int* order = L > 0 ? a.ws.lev_order + R.c0 : nullptr;
+    Solve64 v;
+    v.K = R.c1 - R.c0;
+    v.n_touched = scene_touched(a, g, R);
+    const int zero = v.n_touched < R.b1 - R.b0 ? v.n_touched : 0;
+    v.w_shared = w_smem != nullptr && v.n_touched + 1 <= smem_bodies;
+    v.w = v.w_shared ? w_smem : a.ws.w + 6 * (size_t)R.b0;
+    v.span = reinterpret_cast<const int2*>(a.ws.w2 + 6 * (size_t)R.b0);
+    int4* meta = reinterpret_cast<int4*>(a.ws.c32 + kS32Floats * (size_t)R.c0);
+    v.meta = meta;
+    v.bc_list = a.ws.bc_list;
+    v.J = a.ws.J; v.WJT = a.ws.WJT; v.mu = a.ws.mu;
+    for (int i = g.rank(); i < v.K; i += g.size()) {
+        const int k = order ? order[i] : R.c0 + i;
+        const int lo = a.ws.lohi[2 * k], hi = a.ws.lohi[2 * k + 1];
+        const bool fl = !a.bd.fixed[lo], fh = !a.bd.fixed[hi];
+        meta[i] = make_int4(k, 6 * (fl ? a.ws.bc_fill[lo] : zero), 6 * (fh ? a.ws.bc_fill[hi] : zero),
+                            (fl ? 1 : 0) | (fh ? 2 : 0));
+    }
+    if (zero == v.n_touched && g.rank() < 6) v.w[6 * zero + g.rank()] = 0.0;
+    // the steps: a level's contacts in runs of as many as the sweeping warps have quads
+    int2* steps = reinterpret_cast<int2*>(meta + v.K);
+    v.steps = steps;
+    const int* ptr = a.ws.lev_ptr + R.c0 + s;
+    v.warps = g.size() > 32 ? sweep_warps(ptr, L, g.size() >> 5) : 1;
+    v.n_steps = 0;
+    const int quads = 8 * v.warps;
+    for (int l0 = 0; l0 < L; l0 += 32) {   // every warp of the group counts; the group's first one writes
+        const int lane = threadIdx.x & 31, l = l0 + lane;
+        const int st = l < L ? ptr[l] : 0, n = l < L ? ptr[l + 1] - st : 0;
+        const int parts = (n + quads - 1) / quads;
+        int at = parts;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, at, 31);
+        if (g.rank() < 32)
+            for (int p = 0; p < parts; ++p)
+                steps[v.n_steps + at - parts + p] =
+                    make_int2(st + p * quads, min(quads, n - p * quads) | (p + 1 == parts ? kStepEnds : 0));
+        v.n_steps += total;
+    }
+    g.sync();
+    return v;
+}
+
+// w = WJT x, sequential over each body's contacts (the order of WJT.dot(x)).  A component's chain is 4 additions a
+// contact, so six lanes take a body, one component each; the next contacts' list codes are loaded while the current ones' products are accumulated in order.
+constexpr int kWjtAhead = 4;
+template <class G>
+__device__ __noinline__ void scene_wjt(const G g, const Solve64 v, const double* x) {
+    const int lane = g.rank() & 31, slot = lane / 6, d = lane - 6 * slot;
+    const int stride = 5 * (g.size() >> 5);
+    if (slot < 5) {
+        int i = 5 * (g.rank() >> 5) + slot;
+        int2 span = i < v.n_touched ? v.span[i] : make_int2(0, 0);
+        int code[kWjtAhead];
+#pragma unroll
+        for (int j = 0; j < kWjtAhead; ++j) code[j] = span.x + j < span.y ? v.bc_list[span.x + j] : -1;
+        while (i < v.n_touched) {
+            const int2 ahead = i + stride < v.n_touched ? v.span[i + stride] : make_int2(0, 0);
+            double t = 0.0;
+            for (int e = span.x; e < span.y; e += kWjtAhead) {
+                double Wv[kWjtAhead][4], xv[kWjtAhead][4];
+                bool on[kWjtAhead];
+#pragma unroll
+                for (int j = 0; j < kWjtAhead; ++j) {
+                    on[j] = code[j] >= 0;
+                    if (!on[j]) continue;
+                    const int k = code[j] >> 1;
+                    w_column(v.WJT, k, 6 * (code[j] & 1) + d, Wv[j]);
+                    const double2* xk = reinterpret_cast<const double2*>(x + 4 * (size_t)k);
+                    const double2 t0 = xk[0], t1 = xk[1];
+                    xv[j][0] = t0.x; xv[j][1] = t0.y; xv[j][2] = t1.x; xv[j][3] = t1.y;
+                }
+                const bool same = e + kWjtAhead < span.y;   // this body's next contacts, else the next body's first
+                const int e2 = same ? e + kWjtAhead : ahead.x, end2 = same ? span.y : ahead.y;
+#pragma unroll
+                for (int j = 0; j < kWjtAhead; ++j) code[j] = e2 + j < end2 ? v.bc_list[e2 + j] : -1;
+#pragma unroll
+                for (int j = 0; j < kWjtAhead; ++j)
+                    if (on[j])
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) t += Wv[j][q] * xv[j][q];
+            }
+            v.w[6 * i + d] = t;
+            span = ahead;
+            i += stride;
+        }
     }
     g.sync();
 }
 
-// One projected Gauss-Seidel update of contact k (contacts.py:78-107): z from the current w, normal impulse
-// clamped at zero, friction projected on the ball of radius mu x_n (or zeroed for post-stabilisation),
-// then w += WJT[:, block] delta with the reference's term order.
-__device__ __forceinline__ void gs_contact(const StepArgs& a, int k, const double* b, const double* r, double* x,
-                                           WView w, bool normal_only) {
-    const int lo = a.ws.lohi[2 * k], hi = a.ws.lohi[2 * k + 1];
-    const double* J = a.ws.J + 48 * (size_t)k;
-    const double* Wk = a.ws.WJT + 48 * (size_t)k;
-    const double* wlo = w.at(lo);
-    const double* whi = w.at(hi);
-    double xo[4], z[4];
-    for (int row = 0; row < 4; ++row) {
-        xo[row] = x[4 * k + row];
-        z[row] = xo[row] - r[4 * k + row] * (jrow_dot(J + 12 * row, wlo, whi) + b[4 * k + row]);
+// what lane q of a quad (four neighbouring lanes, one contact) reads of its contact ahead of time: row q of J with
+// its b and r (or, for the residual, the diagonal), the four impulses and mu
+struct Contact64 {
+    double J[12], x[4], xq, b, r, mu;
+    int4 me;
+};
+__device__ __forceinline__ void contact64_load(const Solve64& v, int4 me, int q, const double* b, const double* r,
+                                               const double* x, Contact64& c) {
+    const size_t k = (size_t)me.x;
+    c.me = me;
+    const double2* J = reinterpret_cast<const double2*>(v.J + 48 * k + 2 * q);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) { const double2 t = J[4 * i]; c.J[2 * i] = t.x; c.J[2 * i + 1] = t.y; }
+    c.b = b[4 * k + q];
+    c.r = r[4 * k + q];
+    const double2* xk = reinterpret_cast<const double2*>(x + 4 * k);
+    const double2 x0 = xk[0], x1 = xk[1];
+    c.x[0] = x0.x; c.x[1] = x0.y; c.x[2] = x1.x; c.x[3] = x1.y;
+    c.xq = x[4 * k + q];
+    c.mu = v.mu[k];
+}
+// the meta of position i of the level order, or an idle quad's stand-in (any contact, nothing written) past end
+__device__ __forceinline__ int4 contact64_meta(const Solve64& v, int i, int end) {
+    int4 me = v.meta[min(i, v.K - 1)];
+    if (i >= end) me.w = kMetaIdle;
+    return me;
+}
+// J_q . [w_lo; w_hi] of the quad's contact (jrow_dot's order), the accumulators read as 16-byte pairs
+template <bool kShared>
+__device__ __forceinline__ double contact64_jw(const Contact64& c, const W64<kShared> w) {
+    double u[12];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const double2 l = w.pair(c.me.y + 2 * i), h = w.pair(c.me.z + 2 * i);
+        u[2 * i] = l.x; u[2 * i + 1] = l.y; u[6 + 2 * i] = h.x; u[7 + 2 * i] = h.y;
     }
-    const double xn = z[0] > 0.0 ? z[0] : 0.0;
-    double f[3];
-    if (normal_only) { f[0] = 0.0; f[1] = 0.0; f[2] = 0.0; }
-    else prox_sphere(z[1], z[2], z[3], a.ws.mu[k], xn, f);
-    const double d0 = xn - xo[0], d1 = f[0] - xo[1], d2 = f[1] - xo[2], d3v = f[2] - xo[3];
-    x[4 * k] = xn; x[4 * k + 1] = f[0]; x[4 * k + 2] = f[1]; x[4 * k + 3] = f[2];
-    for (int side = 0; side < 2; ++side) {
-        const int bb = side ? hi : lo;
-        if (a.bd.fixed[bb]) continue;
-        double* wb = w.at(bb);
-        const double* Ws = Wk + 6 * side;
-        for (int d = 0; d < 6; ++d) {
-            double t = 0.0;
-            t += Ws[d] * d0;
-            t += Ws[12 + d] * d1;
-            t += Ws[24 + d] * d2;
-            t += Ws[36 + d] * d3v;
-            wb[d] = wb[d] + t;
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) s += c.J[i] * u[i];
+    return s;
+}
+// the quad's four values of z
+__device__ __forceinline__ void quad_gather(double z, double* o) {
+    const int base = (threadIdx.x & 31) & ~3;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = __shfl_sync(0xffffffffu, z, base | i);
+}
+// prox_sphere (prox_operators.py:14) of the tangential values z[1..3] as one factor kind: 0 takes none of z, 1 takes
+// z, 2 takes z * scale.
+__device__ __forceinline__ int prox_factor(const double* z, double mu, double xn, double& scale) {
+    const double radius = mu * xn;
+    const double sqr = z[1] * z[1] + z[2] * z[2] + z[3] * z[3];
+    const int kind = xn <= 0.0 ? 0 : (sqr <= radius * radius ? 1 : 2);
+    scale = ratio_sqrt(kind == 2 ? radius : 1.0, kind == 2 ? sqr : 1.0);   // zeros would leave its range
+    return kind;
+}
+__device__ __forceinline__ double prox_apply(int kind, double scale, double z) {
+    const double t = z * scale;
+    return kind == 0 ? 0.0 : (kind == 1 ? z : t);
+}
+
+// One projected Gauss-Seidel sweep (contacts.py:66-107) over the scene's levels, a quad per contact: lane q
+// computes z_q from the current w, the four z meet by shuffles, every lane applies the prox (normal impulse
+// clamped at zero, friction projected on the ball of radius mu x_n, or zeroed for post-stabilisation) and adds
+// three of the twelve components of WJT[:, block] delta to w -- 2q, 2q + 1 and 8 + q, six per body -- with the
+// reference's term order.  Reads the impulses x, writes the swept ones to y (which may be x).  Returns this
+// thread's largest |y - x|.
+//
+// Bound by one contact's chain (12 dependent additions of 8 cycles, two shuffles, the prox's root and quotient, 5
+// more additions: ~450 cycles) and by the ~290 instructions of a step, which one warp issues every ~4 cycles: what
+// does not depend on w is kept off the chain.  A level of the 32-box tower takes 1210 cycles and one of 150-250
+// boxes and spheres ~1500; with one thread per contact, its 96 matrix elements loaded after the level's barrier,
+// they took 2700 and 6300.  The sweep is one sequence of steps (a level, or as many of its contacts as there are
+// quads; steps[j] = first position, contacts, whether a level ends); each value of the next step's contact is
+// loaded into the register of the current one's as soon as that is used up, its meta a step before that, so one
+// copy of the loop body holds one contact and no register is moved.
+template <class G, bool kShared>
+__device__ __noinline__ double gs_sweep_quads(const G g, const Solve64 v, int n_steps, const double* b, const double* r,
+                                              const double* x, double* y, bool normal_only) {
+    const W64<kShared> w(v.w);
+    const int q = g.rank() & 3, slot = g.rank() >> 2;
+    const double* J = v.J + 2 * q;
+    const double* WJT = v.WJT + 2 * q;
+    b += q; r += q; y += q;
+    const double* xs = x + q;
+    double m = 0.0;
+    auto meta = [&](int2 st) {
+        int4 me = v.meta[min(st.x + slot, v.K - 1)];
+        if (slot >= (st.y & 0xffff)) me.w = kMetaIdle;
+        return me;
+    };
+    Contact64 c;
+    double W[12];   // columns 2q, 2q + 1, 8 + q, four rows each
+    auto load_w = [&](int k) {
+        const double2* p = reinterpret_cast<const double2*>(WJT + 48 * (size_t)k);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) { const double2 t = p[4 * i]; W[2 * i] = t.x; W[2 * i + 1] = t.y; }
+    };
+    auto load_j = [&](int k) {
+        const double2* p = reinterpret_cast<const double2*>(J + 48 * (size_t)k);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) { const double2 t = p[4 * i]; c.J[2 * i] = t.x; c.J[2 * i + 1] = t.y; }
+    };
+    auto load_x = [&](int k) {
+        const double2* p = reinterpret_cast<const double2*>(x + 4 * (size_t)k);
+        const double2 t = p[0], u = p[1];
+        c.x[0] = t.x; c.x[1] = t.y; c.x[2] = u.x; c.x[3] = u.y;
+    };
+    int2 st0 = v.steps[0], st1 = v.steps[min(1, n_steps - 1)];
+    c.me = meta(st0);
+    load_j(c.me.x);
+    load_x(c.me.x);
+    load_w(c.me.x);
+    c.xq = xs[4 * (size_t)c.me.x]; c.b = b[4 * (size_t)c.me.x]; c.r = r[4 * (size_t)c.me.x]; c.mu = v.mu[c.me.x];
+    int4 next = meta(st1);
+#pragma unroll 1
+    for (int j = 0; j < n_steps; ++j) {
+        const int2 st2 = v.steps[min(j + 2, n_steps - 1)];
+        const double jw = contact64_jw(c, w);
+        load_j(next.x);
+        const double xq = c.xq, zq = xq - c.r * (jw + c.b);
+        c.xq = xs[4 * (size_t)next.x]; c.b = b[4 * (size_t)next.x]; c.r = r[4 * (size_t)next.x];
+        double z[4];
+        quad_gather(zq, z);
+        const double xn = z[0] > 0.0 ? z[0] : 0.0;
+        double scale = 1.0;
+        const int kind = normal_only ? 0 : prox_factor(z, c.mu, xn, scale);
+        c.mu = v.mu[next.x];
+        const double d0 = xn - c.x[0], d1 = prox_apply(kind, scale, z[1]) - c.x[1];
+        const double d2 = prox_apply(kind, scale, z[2]) - c.x[2], d3v = prox_apply(kind, scale, z[3]) - c.x[3];
+        load_x(next.x);
+        const double yq = q == 0 ? xn : prox_apply(kind, scale, zq);
+        double ta = 0.0, tb = 0.0, tc = 0.0;
+        ta += W[0] * d0; tb += W[4] * d0; tc += W[8] * d0;
+        ta += W[1] * d1; tb += W[5] * d1; tc += W[9] * d1;
+        ta += W[2] * d2; tb += W[6] * d2; tc += W[10] * d2;
+        ta += W[3] * d3v; tb += W[7] * d3v; tc += W[11] * d3v;
+        load_w(next.x);
+        const int ia = q < 3 ? c.me.y + 2 * q : c.me.z, ic = c.me.z + 2 + q;
+        const double2 wa = w.pair(ia);
+        const double wc = w.one(ic);
+        if (c.me.w & (q < 3 ? 1 : 2)) w.set(ia, make_double2(wa.x + ta, wa.y + tb));
+        if (c.me.w & 2) w.set(ic, wc + tc);
+        if (!(c.me.w & kMetaIdle)) {
+            y[4 * (size_t)c.me.x] = yq;
+            m = nanmax(m, fabs(yq - xq));
         }
+        if (st0.y & kStepEnds) g.sync();   // the last step of its level
+        st0 = st1; st1 = st2;
+        c.me = next;
+        next = meta(st2);
+    }
+    return m;
+}
+
+// A block sweeps a scene with the number of its warps that scene_setup64 chose.  One warp has warp barriers between the
+// levels, several a barrier of their own, and the block meets at the end of the sweep.
+template <class G>
+__device__ __forceinline__ double gs_sweep_levels(const G& g, const Solve64& v, const double* b, const double* r,
+                                                  const double* x, double* y, bool normal_only) {
+    if constexpr (std::is_same_v<G, BlockGroup>) {
+        double m = 0.0;
+        if (v.warps == 1) {
+            if (threadIdx.x < 32) m = gs_sweep_levels(WarpGroup{}, v, b, r, x, y, normal_only);
+        } else if ((int)threadIdx.x < 32 * v.warps) {
+            const SubGroup sub = {32 * v.warps};
+            m = v.w_shared ? gs_sweep_quads<SubGroup, true>(sub, v, v.n_steps, b, r, x, y, normal_only)
+                           : gs_sweep_quads<SubGroup, false>(sub, v, v.n_steps, b, r, x, y, normal_only);
+        }
+        g.sync();
+        return m;
+    } else {
+        return v.w_shared ? gs_sweep_quads<G, true>(g, v, v.n_steps, b, r, x, y, normal_only)
+                          : gs_sweep_quads<G, false>(g, v, v.n_steps, b, r, x, y, normal_only);
     }
 }
 
@@ -1258,53 +1629,32 @@ __device__ int scene_colours(const StepArgs& a, const G& g, const SceneRange& R,
     return bucket_classes(a, g, R, s);
 }
 
-template <class G>
-__device__ __forceinline__ void gs_sweep_levels(const StepArgs& a, const G& g, const SceneRange& R, int s, int L,
-                                                const double* b, const double* r, double* x, WView w,
-                                                bool normal_only) {
-    const int* ptr = a.ws.lev_ptr + R.c0 + s;
-    for (int l = 1; l <= L; ++l) {
-        const int start = ptr[l - 1], end = ptr[l];
-        if (l < L) {   // pull the next level's Jacobian blocks into L1 while this level runs
-            const int i = end + g.rank();
-            if (i < ptr[l + 1]) {
-                const int kn = a.ws.lev_order[R.c0 + i];
-                const char* pj = reinterpret_cast<const char*>(a.ws.J + 48 * (size_t)kn);
-                const char* pw = reinterpret_cast<const char*>(a.ws.WJT + 48 * (size_t)kn);
-                for (int off = 0; off < 384; off += 128) {
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(pj + off));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(pw + off));
-                }
-            }
-        }
-        for (int i = start + g.rank(); i < end; i += g.size())
-            gs_contact(a, a.ws.lev_order[R.c0 + i], b, r, x, w, normal_only);
-        g.sync();
-    }
-}
-
 // complementarity residual ||x - prox(x - D^-1 (A x + b))||_inf / max(1, ||x||_inf), D = diag(A): the
 // tolerance the solver modes are compared at.  Every scheme scales the prox argument by a positive multiple of
 // D^-1, so they all share this map's zeros as fixed points.  A x = J W J^T x through w = WJT x (the
 // accumulators are rebuilt from x at the start of every sweep, so they are free to hold this product here).
 template <class G>
-__device__ double scene_residual(const StepArgs& a, const G& g, const SceneRange& R, const double* x, WView w) {
-    scene_wjt(a, g, R, x, w);
+__device__ double scene_residual(const StepArgs& a, const G& g, const Solve64& v, const double* x) {
+    scene_wjt(g, v, x);
+    const int q = g.rank() & 3, slot = g.rank() >> 2, nslot = g.size() >> 2;
     double m = 0.0, xm = 0.0;
-    for (int k = R.c0 + g.rank(); k < R.c1; k += g.size()) {
-        const int lo = a.ws.lohi[2 * k], hi = a.ws.lohi[2 * k + 1];
-        const double* J = a.ws.J + 48 * (size_t)k;
+    Contact64 c;
+    contact64_load(v, contact64_meta(v, slot, v.K), q, a.ws.b, a.ws.diag, x, c);
+    for (int i = 0; i < v.K; i += nslot) {   // a quad per contact, the next one's values loaded meanwhile
+        const double jw = contact64_jw(c, W64<false>(v.w));
+        const double xq = c.xq;
+        const double bq = c.b, dq = c.r, mu = c.mu;
+        const bool mine = !(c.me.w & kMetaIdle);
+        contact64_load(v, contact64_meta(v, i + nslot + slot, v.K), q, a.ws.b, a.ws.diag, x, c);
         double z[4];
-        for (int row = 0; row < 4; ++row)
-            z[row] = x[4 * k + row] -
-                     (1.0 / a.ws.diag[4 * k + row]) * (jrow_dot(J + 12 * row, w.at(lo), w.at(hi)) + a.ws.b[4 * k + row]);
+        const double zq = xq - (1.0 / dq) * (jw + bq);
+        quad_gather(zq, z);
         const double pn = z[0] > 0.0 ? z[0] : 0.0;
-        double f[3];
-        prox_sphere(z[1], z[2], z[3], a.ws.mu[k], pn, f);
-        const double d[4] = {x[4 * k] - pn, x[4 * k + 1] - f[0], x[4 * k + 2] - f[1], x[4 * k + 3] - f[2]};
-        for (int i = 0; i < 4; ++i) {
-            m = nanmax(m, fabs(d[i]));
-            xm = fmax(xm, fabs(x[4 * k + i]));
+        double scale;
+        const int kind = prox_factor(z, mu, pn, scale);
+        if (mine) {
+            m = nanmax(m, fabs(xq - (q == 0 ? pn : prox_apply(kind, scale, zq))));
+            xm = fmax(xm, fabs(xq));
         }
     }
     const double mres = g.max(m);
@@ -1529,7 +1879,7 @@ __device__ void solve_scene_hinges(const StepArgs& a, const G& g, int s, double*
     const double* b = a.ws.b;
     double* r = a.ws.r;
     const SceneRange R = scene_range(a, s);
-    const int K = R.c1 - R.c0, nb = R.b1 - R.b0;
+    const int K = R.c1 - R.c0;
     const int h0 = a.bd.scene_hinge_start[s], h1 = a.bd.scene_hinge_start[s + 1];
     rb_scene_stats* st = a.out.stats + s;
     double* hist = (a.out.residuals && a.pr.profiling) ? a.out.residuals + (size_t)s * a.caps.max_iterations : nullptr;
@@ -1539,9 +1889,9 @@ __device__ void solve_scene_hinges(const StepArgs& a, const G& g, int s, double*
         st->n_levels = 0; st->fp32_sweeps = 0;
     }
     if (hist) for (int i = g.rank(); i < max_it; i += g.size()) hist[i] = INFINITY;
-    const bool on_chip = w_smem != nullptr && nb <= smem_bodies;
-    const WView w = {on_chip ? w_smem : a.ws.w + 6 * R.b0, R.b0};
     const int L = K > 0 ? scene_levels(a, g, R, s) : 0;
+    Solve64 v = {};
+    if (K > 0) v = scene_setup64(a, g, R, s, L, w_smem, smem_bodies);
     const int HL = hinge_levels(a, g, R, s, h0, h1);
     if (g.rank() == 0) st->n_levels = L;
     const int* hptr = a.ws.hlev_ptr + h0 + s;
@@ -1550,11 +1900,9 @@ __device__ void solve_scene_hinges(const StepArgs& a, const G& g, int s, double*
     for (int it = 0; it < max_it; ++it) {
         double gm = 0.0;
         if (K > 0) {   // Contacts.sweep, then the accept / roll-back rule
-            scene_wjt(a, g, R, x, w);
-            gs_sweep_levels(a, g, R, s, L, b, r, x, w, false);
-            double m = 0.0;
-            for (int i = 4 * R.c0 + g.rank(); i < 4 * R.c1; i += g.size()) m = nanmax(m, fabs(x[i] - sol[i]));
-            const double merit = g.max(m);
+            scene_wjt(g, v, x);
+            // x = sol at the start of every sweep, so the sweep's largest change is the merit ||x - sol||_inf
+            const double merit = g.max(gs_sweep_levels(g, v, b, r, x, x, false));
             const bool reject = merit > last_c;
             const bool inc = !reject && last_c - merit < a.pr.too_small_merit_change;
             for (int i = 4 * R.c0 + g.rank(); i < 4 * R.c1; i += g.size()) {
@@ -1635,13 +1983,15 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
     const bool rigid = scheme == RB_SCHEME_RIGID_GS;
     const bool jacobi = scheme == RB_SCHEME_JACOBI || scheme == RB_SCHEME_JACOBI_HYBRID;
     const int max_it = a.pr.max_iterations;
+    // the accepted impulses x and the sweep's new ones y: two arrays that change places when a sweep is
+    // accepted (a rolled-back sweep leaves x as it is); the solution goes to sol at the end
     double* x = a.ws.x;
     double* sol = post ? a.ws.xold : a.out.contact_sol;
+    double* y = a.ws.xold;
     const double* b = a.ws.b;
     double* r = a.ws.r;
     const SceneRange R = scene_range(a, s);
     const int K = R.c1 - R.c0;
-    const int nb = R.b1 - R.b0;
     rb_scene_stats* st = a.out.stats + s;
     double* hist = (!post && a.out.residuals && a.pr.profiling) ? a.out.residuals + (size_t)s * a.caps.max_iterations
                                                                 : nullptr;
@@ -1661,8 +2011,6 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
         for (int k = R.c0 + g.rank(); k < R.c1; k += g.size()) any |= (b[4 * k] != 0.0);
         if (!g.any(any)) return;
     }
-    const bool on_chip = w_smem != nullptr && nb <= smem_bodies;
-    const WView w = {on_chip ? w_smem : a.ws.w + 6 * R.b0, R.b0};
     const bool coloured = !post && !jacobi &&
                           (scheme == RB_SCHEME_COLOURED_GS || a.pr.ordering == RB_ORDER_COLOURED);
     // FP32 modes: the scene's FP32 phase left its iterate in x and its level order in lev_order / lev_ptr
@@ -1670,6 +2018,7 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
     const int L = jacobi ? 0 : sweeps32 >= 0 ? a.ws.nlev[s]
                 : (coloured ? scene_colours(a, g, R, s) : scene_levels(a, g, R, s));
     if (!post && g.rank() == 0) st->n_levels = L;
+    const Solve64 v = scene_setup64(a, g, R, s, L, w_smem, smem_bodies);
     const bool by_residual = !post && a.pr.termination != RB_TERMINATE_MERIT;
     const bool fixed_r = !post && a.pr.termination == RB_TERMINATE_RESIDUAL_FIXED_R;
     const int interval = a.pr.residual_interval > 1 ? a.pr.residual_interval : 1;
@@ -1679,7 +2028,7 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
     // FP32 modes: test the FP32 iterate in FP64, then refine it in FP64 with the sweeps left
     int loop_max = max_it;
     if (sweeps32 >= 0) {
-        const double res0 = scene_residual(a, g, R, x, w);
+        const double res0 = scene_residual(a, g, v, x);
         w_is_wjt_x = true;
         shown = res0;
         if (g.rank() == 0) st->fp32_sweeps = sweeps32;
@@ -1699,34 +2048,40 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
         loop_max = max_it - sweeps32;   // the sweeps the FP32 phase left over
     }
     for (int it = 0; it < loop_max; ++it) {
-        if (!w_is_wjt_x) scene_wjt(a, g, R, x, w);   // every sweep starts from w = WJT x (contacts.py:72)
-        if (jacobi) {               // proximal_contact/jacobi_solver.py:41-79
+        if (!w_is_wjt_x) scene_wjt(g, v, x);   // every sweep starts from w = WJT x (contacts.py:72)
+        double m = 0.0;
+        if (jacobi) {               // proximal_contact/jacobi_solver.py:41-79, a quad per contact
             const bool hybrid = scheme == RB_SCHEME_JACOBI_HYBRID;
-            for (int k = R.c0 + g.rank(); k < R.c1; k += g.size()) {
-                const int lo = a.ws.lohi[2 * k], hi = a.ws.lohi[2 * k + 1];
-                const double* J = a.ws.J + 48 * (size_t)k;
+            const int q = g.rank() & 3, slot = g.rank() >> 2, nslot = g.size() >> 2;
+            Contact64 c;
+            contact64_load(v, contact64_meta(v, slot, K), q, b, r, x, c);
+            for (int i = 0; i < K; i += nslot) {
+                const double jw = contact64_jw(c, W64<false>(v.w));
+                const double xq = c.xq, xn_old = c.x[0];
+                const double bq = c.b, rq = c.r, mu = c.mu;
+                const int4 me = c.me;
+                contact64_load(v, contact64_meta(v, i + nslot + slot, K), q, b, r, x, c);
                 double z[4];
-                for (int row = 0; row < 4; ++row)
-                    z[row] = x[4 * k + row] - r[4 * k + row] * (jrow_dot(J + 12 * row, w.at(lo), w.at(hi)) + b[4 * k + row]);
+                const double zq = xq - rq * (jw + bq);
+                quad_gather(zq, z);
                 const double xn = z[0] > 0.0 ? z[0] : 0.0;
-                double f[3];
-                prox_sphere(z[1], z[2], z[3], a.ws.mu[k], hybrid ? xn : x[4 * k], f);
-                x[4 * k] = xn; x[4 * k + 1] = f[0]; x[4 * k + 2] = f[1]; x[4 * k + 3] = f[2];
+                double scale;
+                const int kind = prox_factor(z, mu, hybrid ? xn : xn_old, scale);
+                if (!(me.w & kMetaIdle)) {
+                    const double xnew = q == 0 ? xn : prox_apply(kind, scale, zq);
+                    y[4 * (size_t)me.x + q] = xnew;
+                    m = nanmax(m, fabs(xnew - xq));
+                }
             }
             g.sync();
         } else {
-            gs_sweep_levels(a, g, R, s, L, b, r, x, w, post != 0);
+            m = gs_sweep_levels(g, v, b, r, x, y, post != 0);
         }
-        // merit = ||x - sol||_inf (problem.py:53); the fixed-r rule never looks at it
-        double merit = 0.0;
-        if (!fixed_r) {
-            double m = 0.0;
-            for (int i = 4 * R.c0 + g.rank(); i < 4 * R.c1; i += g.size()) m = nanmax(m, fabs(x[i] - sol[i]));
-            merit = g.max(m);
-        }
+        // merit = ||y - x||_inf (problem.py:53); the fixed-r rule never looks at it
+        const double merit = fixed_r ? 0.0 : g.max(m);
         const bool check = by_residual && (!fixed_r || (it + 1) % interval == 0 || it + 1 == loop_max);
-        const double res = check ? scene_residual(a, g, R, x, w) : 0.0;
-        int decision = 0;   // 0 accept, 1 reject, 2 keep sol, 3 take x
+        const double res = check ? scene_residual(a, g, v, y) : 0.0;
+        int decision = 0;   // 0 accept, 1 reject, 2 keep x, 3 take y
         bool stop = false, inc = false;
         if (rigid) {        // gauss_seidel_solver.py:439-482
             double gm;
@@ -1765,26 +2120,23 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
             }
         }
         if (hist && g.rank() == 0) hist[it] = shown;
-        if (decision == 1) {
-            for (int i = 4 * R.c0 + g.rank(); i < 4 * R.c1; i += g.size()) {
-                r[i] = a.pr.nu_reduce * r[i];
-                x[i] = sol[i];
-            }
-        } else if (decision == 0) {
-            for (int i = 4 * R.c0 + g.rank(); i < 4 * R.c1; i += g.size()) {
-                sol[i] = x[i];
-                if (inc) r[i] = a.pr.nu_increase * r[i];
-            }
-        } else if (decision == 3) {   // converged by residual: the current iterate is the solution
-            for (int i = 4 * R.c0 + g.rank(); i < 4 * R.c1; i += g.size()) sol[i] = x[i];
+        if (decision == 1 || (decision == 0 && inc)) {
+            const double nu = decision == 1 ? a.pr.nu_reduce : a.pr.nu_increase;
+            for (int i = 4 * R.c0 + g.rank(); i < 4 * R.c1; i += g.size()) r[i] = nu * r[i];
         }
-        // the residual pass computed w = WJT x; unless x was rolled back that is the next sweep's start
+        // accepted, or converged by residual: the new iterate is the solution so far
+        if (decision == 0 || decision == 3) { double* t = x; x = y; y = t; }
+        // the residual pass computed w = WJT y; unless y was rolled back that is the next sweep's start
         w_is_wjt_x = check && decision != 1;
         g.sync();
         if (stop) { iterations = it; break; }
     }
     if (sweeps32 >= 0) iterations = exitcode == 3 ? sweeps32 + iterations : max_it;
-    if (by_residual && exitcode != 3) shown = scene_residual(a, g, R, sol, w);   // residual of what is returned
+    if (x != sol) {
+        for (int i = 4 * R.c0 + g.rank(); i < 4 * R.c1; i += g.size()) sol[i] = x[i];
+        g.sync();
+    }
+    if (by_residual && exitcode != 3) shown = scene_residual(a, g, v, x);   // residual of what is returned
     if (g.rank() == 0) {
         if (!post) {
             st->iterations = iterations; st->exitcode = exitcode; st->merit = shown;
@@ -1913,17 +2265,17 @@ __device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const Sce
         const int i = t >> 4, q = (t >> 2) & 3, part = t & 3;
         const size_t k = (size_t)order[i];
         float* row = f.c + kS32Floats * i + 12 * q;
-        const double* J = a.ws.J + 48 * k + 12 * q;
+        const double* J = a.ws.J + 48 * k;
         if (part == 0) {
-            row[0] = q < 3 ? (float)J[0] : (float)a.ws.mu[k];
-            row[1] = q < 3 ? (float)J[1] : 0.0f;
-            row[2] = q < 3 ? (float)J[2] : 0.0f;
+            row[0] = q < 3 ? (float)J[j_at(q, 0)] : (float)a.ws.mu[k];
+            row[1] = q < 3 ? (float)J[j_at(q, 1)] : 0.0f;
+            row[2] = q < 3 ? (float)J[j_at(q, 2)] : 0.0f;
             row[3] = (float)a.ws.b[4 * k + q];
         } else if (part == 1) {
-            row[4] = (float)J[3]; row[5] = (float)J[4]; row[6] = (float)J[5];
+            row[4] = (float)J[j_at(q, 3)]; row[5] = (float)J[j_at(q, 4)]; row[6] = (float)J[j_at(q, 5)];
             row[7] = (float)(1.0 / a.ws.diag[4 * k + q]);
         } else if (part == 2) {
-            row[8] = (float)J[9]; row[9] = (float)J[10]; row[10] = (float)J[11];
+            row[8] = (float)J[j_at(q, 9)]; row[9] = (float)J[j_at(q, 10)]; row[10] = (float)J[j_at(q, 11)];
             row[11] = (float)a.ws.x[4 * k + q];
         }
     }
@@ -2268,10 +2620,10 @@ __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, con
             for (int e = f.bptr[bl]; e < f.bptr[bl + 1]; ++e) {
                 const uint32_t code = f.blist[e];
                 const int i = (int)(code >> 1), side = (int)(code & 1);
-                const double* Wk = a.ws.WJT + 48 * (size_t)order[i] + 6 * side;
+                const double* Wk = a.ws.WJT + 48 * (size_t)order[i];
                 for (int q = 0; q < 4; ++q) {
                     const double xq = (double)f.c[kS32Floats * i + 12 * q + 11];
-                    for (int d = 0; d < 6; ++d) acc[d] = fma(Wk[12 * q + d], xq, acc[d]);
+                    for (int d = 0; d < 6; ++d) acc[d] = fma(Wk[w_at(q, 6 * side + d)], xq, acc[d]);
                 }
             }
         }
@@ -2289,10 +2641,12 @@ __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, con
         const float* wh32 = f.body + kS32BodyFloats * hi;
         double z[4], x[4];
         for (int q = 0; q < 4; ++q) {
-            const double* J = a.ws.J + 48 * k + 12 * q;
+            const double* J = a.ws.J + 48 * k;
             double v64 = a.ws.b[4 * k + q];
-            for (int c = 0; c < 6; ++c) v64 = fma(J[c], wl[c], v64);
-            for (int c = 0; c < 6; ++c) v64 = fma(J[6 + c], wh[c], v64);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) v64 = fma(J[j_at(q, c)], wl[c], v64);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) v64 = fma(J[j_at(q, 6 + c)], wh[c], v64);
             float* row = f.c + kS32Floats * i + 12 * q;
             if (correct) {
                 const float v32 = s32_jw(row, q, wl32, wh32) + row[3];
@@ -2554,7 +2908,7 @@ __global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve
     }
 }
 
-constexpr int kSolveBlock = 128;   // threads per scene in the block solver (levels rarely hold more contacts)
+constexpr int kSolveBlock = 256;   // threads per scene in the block solver, at most
 constexpr int kWarpSceneMaxContacts = 2048;
 constexpr int kWarpSceneMaxBodies = 384;
 constexpr int kSolveWarpsPerBlock = 4;
@@ -2566,21 +2920,21 @@ __device__ __forceinline__ int scene_contacts(const StepArgs& a, int s) {
 
 // scenes with at most kWarpSceneMaxContacts contacts and warp_bodies bodies: one warp each
 __global__ void __launch_bounds__(32 * kSolveWarpsPerBlock) k_solve_warps(const StepArgs a, int post, int warp_bodies) {
-    extern __shared__ double wsm[];
+    extern __shared__ __align__(16) double wsm[];
     if (a.ws.counters[kAbort]) return;
     const WarpGroup g;
     const int wib = threadIdx.x >> 5;
-    double* w_smem = warp_bodies > 0 ? wsm + (size_t)wib * 6 * warp_bodies : nullptr;
+    double* w_smem = warp_bodies > 0 ? wsm + (size_t)wib * 6 * (warp_bodies + 1) : nullptr;
     for (int s = blockIdx.x * kSolveWarpsPerBlock + wib; s < a.bd.n_scenes; s += gridDim.x * kSolveWarpsPerBlock) {
         const int nb = a.bd.scene_start[s + 1] - a.bd.scene_start[s];
         if (scene_contacts(a, s) > kWarpSceneMaxContacts || nb > warp_bodies) continue;
-        solve_scene(a, g, s, post, w_smem, warp_bodies);
+        solve_scene(a, g, s, post, w_smem, warp_bodies + 1);
     }
 }
 
 // the other scenes: one block each; the body accumulators are on chip up to smem_bodies bodies
 __global__ void __launch_bounds__(kSolveBlock) k_solve_blocks(const StepArgs a, int post, int warp_bodies, int smem_bodies) {
-    extern __shared__ double wsm[];
+    extern __shared__ __align__(16) double wsm[];
     __shared__ double red[33];
     __shared__ int ired[33];
     if (a.ws.counters[kAbort]) return;
@@ -2588,7 +2942,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_solve_blocks(const StepArgs a, 
     for (int s = blockIdx.x; s < a.bd.n_scenes; s += gridDim.x) {
         const int nb = a.bd.scene_start[s + 1] - a.bd.scene_start[s];
         if (scene_contacts(a, s) <= kWarpSceneMaxContacts && nb <= warp_bodies) continue;
-        solve_scene(a, g, s, post, smem_bodies > 0 ? wsm : nullptr, smem_bodies);
+        solve_scene(a, g, s, post, wsm, smem_bodies);
     }
 }
 
@@ -2604,20 +2958,20 @@ __device__ __forceinline__ void position_update(double* xb, const double* ub, do
     quat_unit(qn, xb + 3);
 }
 
+// six lanes per body, one velocity component each (the sums over a body's contacts are chains of 4 additions a
+// contact); the first of them moves the body
 __global__ void k_integrate(const StepArgs a) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= a.bd.n_bodies || a.ws.counters[kAbort]) return;
-    double* ub = a.bd.u + 6 * b;
-    double du[6];
-    for (int d = 0; d < 6; ++d) du[d] = a.ws.du[6 * b + d];
-    if (!a.bd.fixed[b] && a.ws.bc_ptr[b + 1] > a.ws.bc_ptr[b]) {   // delta_u += WJT sol (steppers.py:84-85)
-        double dc[6];
-        body_wjt_dot(a.ws, b, a.out.contact_sol, dc);
-        for (int d = 0; d < 6; ++d) du[d] = du[d] + dc[d];
-    }
-    if (a.bd.n_hinges > 0 && !a.bd.fixed[b] && a.ws.hbody_ptr[b + 1] > a.ws.hbody_ptr[b]) {
-        // then the hinge problem's WJT sol (hinges.py:52), hinges ascending, 5 rows each
-        for (int d = 0; d < 6; ++d) {
+    if (a.ws.counters[kAbort]) return;
+    int d;
+    const int b = body_of_six(a.bd.n_bodies, d);
+    const bool fixed = b < 0 || a.bd.fixed[b];
+    double ud = 0.0;
+    if (b >= 0) {
+        double du = a.ws.du[6 * b + d];
+        const int e0 = a.ws.bc_ptr[b], e1 = a.ws.bc_ptr[b + 1];
+        if (!fixed && e1 > e0) du = du + body_wjt_dot(a.ws, e0, e1, d, a.out.contact_sol);   // steppers.py:84-85
+        if (a.bd.n_hinges > 0 && !fixed && a.ws.hbody_ptr[b + 1] > a.ws.hbody_ptr[b]) {
+            // then the hinge problem's WJT sol (hinges.py:52), hinges ascending, 5 rows each
             double t = 0.0;
             for (int e = a.ws.hbody_ptr[b]; e < a.ws.hbody_ptr[b + 1]; ++e) {
                 const int code = a.ws.hbody_list[e];
@@ -2625,15 +2979,18 @@ __global__ void k_integrate(const StepArgs a) {
                 const double* Wk = a.ws.hWJT + 60 * (size_t)k + 6 * side;
                 for (int row = 0; row < 5; ++row) t += Wk[12 * row + d] * a.ws.hsol[5 * (size_t)k + row];
             }
-            du[d] = du[d] + t;
+            du = du + t;
         }
+        ud = a.bd.u[6 * b + d] + du;
+        a.bd.u[6 * b + d] = ud;
     }
-    for (int d = 0; d < 6; ++d) ub[d] = ub[d] + du[d];
-    if (a.bd.fixed[b]) return;
+    double ub[6];
+    gather_six(ud, ub);
+    if (fixed || d != 0) return;
     position_update(a.bd.x + 7 * b, ub, a.pr.dt);
     bool finite = true;
-    for (int d = 0; d < 7; ++d) finite &= isfinite(a.bd.x[7 * b + d]);
-    for (int d = 0; d < 6; ++d) finite &= isfinite(ub[d]);
+    for (int i = 0; i < 7; ++i) finite &= isfinite(a.bd.x[7 * b + i]);
+    for (int i = 0; i < 6; ++i) finite &= isfinite(ub[i]);
     if (!finite) atomicOr(a.out.status, RB_STATUS_NONFINITE);
 }
 
@@ -2652,14 +3009,16 @@ __global__ void k_post_setup(const StepArgs a) {
     }
 }
 __global__ void k_post_apply(const StepArgs a) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= a.bd.n_bodies || a.ws.counters[kAbort] || a.bd.fixed[b]) return;
-    // every non-fixed body of a corrected scene is updated (and its quaternion renormalised), contacts or not
-    const int s = scene_of(a.bd.scene_start, a.bd.n_scenes, b);
-    if (a.out.stats[s].post_iterations < 0) return;   // this scene had nothing to correct
+    if (a.ws.counters[kAbort]) return;
+    int d;
+    const int b = body_of_six(a.bd.n_bodies, d);
+    // every non-fixed body of a corrected scene is updated (and its quaternion renormalised), contacts or not;
+    // a scene with post_iterations < 0 had nothing to correct
+    const bool moves = b >= 0 && !a.bd.fixed[b] &&
+                       a.out.stats[scene_of(a.bd.scene_start, a.bd.n_scenes, b)].post_iterations >= 0;
     double dr[6];
-    body_wjt_dot(a.ws, b, a.ws.xold, dr);
-    position_update(a.bd.x + 7 * b, dr, 1.0);
+    gather_six(moves ? body_wjt_dot(a.ws, a.ws.bc_ptr[b], a.ws.bc_ptr[b + 1], d, a.ws.xold) : 0.0, dr);
+    if (moves && d == 0) position_update(a.bd.x + 7 * b, dr, 1.0);
 }
 
 // energies and largest penetration (state_storage.py:188, contacts.py:222): thread per scene, body order
@@ -2844,7 +3203,7 @@ int ensure_kernel_attributes() {
     if (e != cudaSuccess || dev < 0 || dev >= 64) return fail(RB_ERR_CUDA, "rb_step: no current device");
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (g_attr_done[dev]) return RB_OK;
-    const int warp_max = kSolveWarpsPerBlock * 6 * (int)sizeof(double) * kWarpSceneMaxBodies;
+    const int warp_max = kSolveWarpsPerBlock * 6 * (int)sizeof(double) * (kWarpSceneMaxBodies + 1);
     const int block_max = 6 * (int)sizeof(double) * kSolveSmemBodies;
     e = cudaFuncSetAttribute(k_solve_warps, cudaFuncAttributeMaxDynamicSharedMemorySize, warp_max);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_solve_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, block_max);
@@ -3013,11 +3372,14 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     // a warp per scene only pays off once the scenes alone fill the GPU (>= 32 per SM); otherwise blocks
     const int warp_bodies = bd->n_scenes < 148 * 32 ? 0
                           : (bd->max_scene_bodies < kWarpSceneMaxBodies ? bd->max_scene_bodies : kWarpSceneMaxBodies);
-    const size_t warp_smem = (size_t)kSolveWarpsPerBlock * 6 * sizeof(double) * (warp_bodies > 0 ? warp_bodies : 1);
+    const size_t warp_smem = (size_t)kSolveWarpsPerBlock * 6 * sizeof(double) * (warp_bodies > 0 ? warp_bodies + 1 : 1);
     const int wg = (bd->n_scenes + kSolveWarpsPerBlock - 1) / kSolveWarpsPerBlock;
-    const int smem_bodies = bd->max_scene_bodies <= kSolveSmemBodies ? bd->max_scene_bodies : 0;
-    const size_t block_smem = (size_t)6 * sizeof(double) * (smem_bodies > 0 ? smem_bodies : 1);
+    const int smem_bodies = std::min(std::max(bd->max_scene_bodies, 0), kSolveSmemBodies - 1) + 1;   // + 1: fixed bodies
+    const size_t block_smem = (size_t)6 * sizeof(double) * smem_bodies;
     const int bg = bd->n_scenes < 148 * 16 ? bd->n_scenes : 148 * 16;
+    // a scene that has an SM to itself takes as many warps as the registers allow (255 a thread), so that wide levels
+    // and the rebuilds of w have them; more scenes than SMs share them, two or four blocks to an SM
+    const int solve_threads = bd->n_scenes <= 148 ? kSolveBlock : bd->n_scenes <= 2 * 148 ? kSolveBlock / 2 : kSolveBlock / 4;
     k_fp32_classes<<<1, 1024, 0, st>>>(a, small_slab, mid_slab); note_launch();
     if (pr->precision != RB_PRECISION_FP64) {
         // FP32 phase, four size classes side by side: warp teams with small slabs (28 KB unless tuned), warp
@@ -3047,14 +3409,14 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
         }
     }
     if (warp_bodies > 0) { k_solve_warps<<<wg, 32 * kSolveWarpsPerBlock, warp_smem, st>>>(a, 0, warp_bodies); note_launch(); }
-    k_solve_blocks<<<bg, kSolveBlock, block_smem, st>>>(a, 0, warp_bodies, smem_bodies); note_launch();
+    k_solve_blocks<<<bg, solve_threads, block_smem, st>>>(a, 0, warp_bodies, smem_bodies); note_launch();
     prof_mark(prof, 5, st);
-    k_integrate<<<blocks_for(N, 128), 128, 0, st>>>(a); note_launch();
+    k_integrate<<<blocks_for(32 * ((N + 4) / (int64_t)5), 128), 128, 0, st>>>(a); note_launch();
     if (pr->use_post_stabilization) {
         k_post_setup<<<G, 128, 0, st>>>(a); note_launch();
         if (warp_bodies > 0) { k_solve_warps<<<wg, 32 * kSolveWarpsPerBlock, warp_smem, st>>>(a, 1, warp_bodies); note_launch(); }
-        k_solve_blocks<<<bg, kSolveBlock, block_smem, st>>>(a, 1, warp_bodies, smem_bodies); note_launch();
-        k_post_apply<<<blocks_for(N, 128), 128, 0, st>>>(a); note_launch();
+        k_solve_blocks<<<bg, solve_threads, block_smem, st>>>(a, 1, warp_bodies, smem_bodies); note_launch();
+        k_post_apply<<<blocks_for(32 * ((N + 4) / (int64_t)5), 128), 128, 0, st>>>(a); note_launch();
     }
     if (prof) { k_body_energy<<<blocks_for(N, 128), 128, 0, st>>>(a); note_launch(); }
     k_scene_summary<<<blocks_for(32 * (int64_t)bd->n_scenes, 128), 128, 0, st>>>(a); note_launch();

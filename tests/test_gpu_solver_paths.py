@@ -1,0 +1,83 @@
+"""The solver's launch and team variants against the oracle, FP64, bit for bit.
+
+The block solver takes 256, 128 or 64 threads a scene by the number of scenes, sweeps with one to eight warps by the
+width of the levels, and numbers the free bodies that have contacts (with and without a fixed body among the rest);
+batches of many scenes go to the warp solver.  Scenes of one body up, and of levels from one contact to wider than
+eight warps' quads, at the edges of those rules."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def pool():
+    """Small piles squeezed together so that their bodies touch from the first step on."""
+    from rainbow_b200 import scenes
+    arrays, params = scenes.batch_arrays(n_scenes=24, seed=11, pool=3, body_range=(1, 40), resolution=16,
+                                         device="cuda:0")
+    for a in arrays:
+        a["body_r"] = np.concatenate([a["body_r"][:1], a["body_r"][1:] * [0.45, 0.3, 0.45]])
+    return arrays, params
+
+
+def _compare(world, ors, picks, rp, steps, **okw):
+    contacts = 0
+    for _ in range(steps):
+        assert world.step(rp) == 0
+        x, u = world.state()
+        c = world.contacts()
+        st = world.stats()
+        for i in picks:
+            o = ors[i].step(**okw)
+            b0, b1 = world.scene_start[i], world.scene_start[i + 1]
+            k0, K = st[i].contact_start, st[i].n_contacts
+            assert K == o["n_contacts"]
+            contacts += K
+            np.testing.assert_array_equal(c["sol"][4 * k0:4 * (k0 + K)], o["sol"])
+            if K:
+                assert (st[i].iterations, st[i].exitcode) == (o["iterations"], o["exitcode"])
+            np.testing.assert_array_equal(x[b0:b1].ravel(), o["x"])
+            np.testing.assert_array_equal(u[b0:b1].ravel(), o["u"])
+    assert contacts > 0
+
+
+@pytest.mark.parametrize("scheme,mode", [("rigid_gauss_seidel", 0), ("rigid_gauss_seidel", 2), ("gauss_seidel", 1),
+                                         ("parallel_jacobi_hybrid", 0)])
+@pytest.mark.parametrize("n_scenes", [1, 148, 149, 297, 4736])
+def test_scene_counts(oracle_lib, pool, n_scenes, scheme, mode):
+    from rainbow_b200 import world as W
+    arrays, params = pool
+    many = [arrays[(7 * i) % len(arrays)] for i in range(n_scenes)]
+    picks = sorted({0, n_scenes // 2, n_scenes - 1})
+    world = W.DeviceWorld(many, device="cuda:0", max_iterations=100)
+    rp = W.make_rb_params(params, scheme=scheme, termination=("merit", "residual", "residual_fixed_r")[mode],
+                          residual_interval=3)
+    rp.max_iterations = 20
+    ors = {i: oracle_lib.OracleScene(many[i]) for i in picks}
+    for o in ors.values():
+        o.set_param("max_iterations", 20)
+    _compare(world, ors, picks, rp, 2, scheme=scheme, tol_mode=mode, tol=1e-6, residual_interval=3)
+
+
+@pytest.mark.parametrize("count,fixed_ground", [(2, True), (40, True), (400, True), (40, False)])
+def test_level_widths(oracle_lib, pool, count, fixed_ground):
+    """Side-by-side pairs of bodies on one ground: levels of up to `count` contacts; without a fixed body every
+    contact's two bodies are free and the ground chains them all."""
+    from rainbow_b200 import world as W
+    arrays, params = pool
+    a = dict(max(arrays, key=lambda s: len(s["body_mass"])))
+    n = len(a["body_mass"]) - 1
+    side = int(np.ceil(np.sqrt(count)))
+    pick = [1 + i % n for i in range(count)]
+    for k in ("body_shape", "body_mass", "body_inertia", "body_material", "body_force_order", "body_q", "body_v",
+              "body_w", "body_fixed", "body_r"):
+        a[k] = np.concatenate([a[k][:1], a[k][pick]])
+    place = np.array([[2.6 * (i % side - side / 2), 0.45, 2.6 * (i // side - side / 2)] for i in range(count)])
+    a["body_r"] = np.concatenate([a["body_r"][:1], place])
+    if not fixed_ground:
+        a["body_fixed"] = np.zeros(count + 1, np.uint8)
+    world = W.DeviceWorld([a], device="cuda:0", max_iterations=100)
+    rp = W.make_rb_params(params)
+    o = oracle_lib.OracleScene(a)
+    _compare(world, {0: o}, [0], rp, 2)
