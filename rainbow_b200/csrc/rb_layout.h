@@ -10,12 +10,10 @@ namespace rb {
 
 constexpr int kMaxClustersPerShape = 512;   // 16384 triangles per shape (mid-phase cluster masks in shared memory)
 constexpr int kScanBlocks = 1024;           // partial sums of the device-wide scans
-// Strides of the compact FP32 records.  A contact record (12 floats per row, 4 rows) is padded to an odd
-// number of float4s (13), so the 128-bit row loads of eight lanes reading eight different contacts fall on
-// eight different groups of four shared-memory banks (with 12 float4s every other contact shared its banks:
-// 4-way conflicts once a level holds several contacts).  Body records (w, m^-1, fixed, I^-1) are read two
-// per contact and often the same body by several lanes; padding them did not pay.
-constexpr int kS32Floats = 52;               // floats per contact record (48 used)
+// Strides of the compact FP32 records: a contact's four rows of three float4s and its impulses (13 float4s: an odd
+// number spreads the same piece of neighbouring contacts over the shared-memory banks), and a body's (w, m^-1, fixed,
+// I^-1).
+constexpr int kS32Floats = 52;               // floats per contact record
 constexpr int kS32BodyFloats = 16;           // floats per body record
 
 struct Workspace {

@@ -1024,8 +1024,8 @@ struct WarpGroup {
         for (int o = 16; o > 0; o >>= 1) v = ::max(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
     }
-    // collect: the members whose flag is set take consecutive places after the n taken so far (every member
-    // calls it the same number of times); n is then the number taken in all
+    // collect: the members whose flag is set take the places after the n taken so far, in order (every member
+    // calls it the same number of times); n is then the number taken
     __device__ __forceinline__ int append_begin() const { return 0; }
     __device__ __forceinline__ int append(bool flag, int& n) const {
         const unsigned bal = __ballot_sync(0xffffffffu, flag);
@@ -1065,23 +1065,21 @@ struct BlockGroup {
         __syncthreads();
         return m;
     }
-    __device__ int append_begin() const {
-        __syncthreads();
-        if (threadIdx.x == 0) ired[32] = 0;
-        __syncthreads();
-        return 0;
-    }
-    __device__ int append(bool flag, int&) const {
+    __device__ int append_begin() const { return 0; }
+    __device__ int append(bool flag, int& n) const {
         const unsigned bal = __ballot_sync(0xffffffffu, flag);
-        int at = 0;
-        if (bal && (threadIdx.x & 31) == 0) at = atomicAdd(ired + 32, __popc(bal));
-        return __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanemask_lt());
-    }
-    __device__ void append_end(int& n) const {
+        const int wid = threadIdx.x >> 5;
+        if ((threadIdx.x & 31) == 0) ired[wid] = __popc(bal);
         __syncthreads();
-        n = ired[32];
+        int at = n + __popc(bal & lanemask_lt());
+        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
+            if (k < wid) at += ired[k];
+            n += ired[k];
+        }
         __syncthreads();
+        return at;
     }
+    __device__ void append_end(int&) const { __syncthreads(); }
 };
 
 // the first `threads` threads of a block (a multiple of 32), with a barrier of their own
@@ -1177,6 +1175,31 @@ __device__ __forceinline__ int sweep_warps(const int* ptr, int L, int max_warps)
     return best;
 }
 
+// The steps of a sweep: a level of up to `narrow` contacts is one step, a wider one is cut into runs of `run`;
+// put(j, first position, contacts, whether the level ends, whether it is a wide one).  Every warp of the group counts,
+// its first one puts.  Returns their number.
+template <class G, class Put>
+__device__ __forceinline__ int sweep_steps(const G& g, const int* ptr, int L, int narrow, int run, Put put) {
+    int n_steps = 0;
+    for (int l0 = 0; l0 < L; l0 += 32) {
+        const int lane = threadIdx.x & 31, l = l0 + lane;
+        const int st = l < L ? ptr[l] : 0, n = l < L ? ptr[l + 1] - st : 0;
+        const int parts = n <= narrow ? min(n, 1) : (n + run - 1) / run;
+        int at = parts;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, at, 31);
+        if (g.rank() < 32)
+            for (int p = 0; p < parts; ++p)
+                put(n_steps + at - parts + p, st + p * run, min(run, n - p * run), p + 1 == parts, n > narrow);
+        n_steps += total;
+    }
+    return n_steps;
+}
+
 // the scene's working set once its contact order is known (L levels; 0: ascending order, no sweeps); w_smem holds
 // smem_bodies accumulators
 template <class G>
@@ -1202,30 +1225,13 @@ __device__ __forceinline__ Solve64 scene_setup64(const StepArgs& a, const G& g, 
                             (fl ? 1 : 0) | (fh ? 2 : 0));
     }
     if (zero == v.n_touched && g.rank() < 6) v.w[6 * zero + g.rank()] = 0.0;
-    // the steps: a level's contacts in runs of as many as the sweeping warps have quads
     int2* steps = reinterpret_cast<int2*>(meta + v.K);
     v.steps = steps;
     const int* ptr = a.ws.lev_ptr + R.c0 + s;
     v.warps = g.size() > 32 ? sweep_warps(ptr, L, g.size() >> 5) : 1;
-    v.n_steps = 0;
-    const int quads = 8 * v.warps;
-    for (int l0 = 0; l0 < L; l0 += 32) {   // every warp of the group counts; the group's first one writes
-        const int lane = threadIdx.x & 31, l = l0 + lane;
-        const int st = l < L ? ptr[l] : 0, n = l < L ? ptr[l + 1] - st : 0;
-        const int parts = (n + quads - 1) / quads;
-        int at = parts;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, at, o);
-            if (lane >= o) at += t;
-        }
-        const int total = __shfl_sync(0xffffffffu, at, 31);
-        if (g.rank() < 32)
-            for (int p = 0; p < parts; ++p)
-                steps[v.n_steps + at - parts + p] =
-                    make_int2(st + p * quads, min(quads, n - p * quads) | (p + 1 == parts ? kStepEnds : 0));
-        v.n_steps += total;
-    }
+    v.n_steps = sweep_steps(g, ptr, L, 8 * v.warps, 8 * v.warps, [&](int at, int start, int count, bool ends, bool) {
+        steps[at] = make_int2(start, count | (ends ? kStepEnds : 0));
+    });
     g.sync();
     return v;
 }
@@ -2157,16 +2163,14 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
 //
 // Compact form.  A contact's Jacobian rows are [lin_lo | ang_lo | lin_hi | ang_hi] with lin_hi = -lin_lo
 // (the frame direction, zero on the torsion row) and W J^T = (m^-1 lin, I_w^-1 ang) per body, so a contact
-// stores per row q: lin_lo (3), ang_lo (3), ang_hi (3), b, 1/diag and x -- 12 floats, 48 per contact (the
-// torsion row's unused lin slot holds mu), in a record of kS32Floats -- and a body stores its accumulator
-// w (6), m^-1, a fixed flag and the world inverse inertia (6, symmetric), in a record of kS32BodyFloats
-// (m^-1 = I^-1 = 0 for a fixed body).  The update of w after a contact changes by dx is m^-1 sum_q lin_q dx_q
-// (negated on the hi side) and I^-1 sum_q ang_q dx_q.
+// stores per row q: lin_lo (3), ang_lo (3), ang_hi (3), b, 1/diag and x -- 12 floats, 48 per contact -- and mu, in a
+// record of kS32Floats, and a body stores its accumulator w (6), m^-1, a fixed flag and the world inverse
+// inertia (6, symmetric), in a record of kS32BodyFloats (all fixed bodies share one with m^-1 = I^-1 = 0).  The update
+// of w after a contact changes by dx is m^-1 sum_q lin_q dx_q (negated on the hi side) and I^-1 sum_q ang_q dx_q.
 //
 // Execution.  A team -- one warp for scenes of up to the mid slab, a 128-thread block above, a 512-thread
-// block for the scenes whose rows stay in L2 -- takes scenes from its size class's queue; the slab scenes are
-// swept one lane per contact (s32_sweep_lane, by warp 0 in a block team), the L2 scenes four lanes per
-// contact (s32_sweep).  The four classes' launches run concurrently on separate streams.
+// block for the scenes whose rows stay in L2 -- takes scenes from its size class's queue and sweeps them four
+// lanes per contact (s32_sweep).  The four classes' launches run concurrently on separate streams.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kQueueFp32 = 5;                        // counters[5..8]: scene queues of the four size classes
 constexpr int kClassEnd32 = 9;                       // counters[9..12]: end of each class's range in list32
@@ -2188,20 +2192,25 @@ constexpr int kS32StallTests = 16;
 constexpr int kS32StallTestsMax = 512;
 constexpr double kS32RoundGain = 0.9;
 
+// A scene's FP32 copy.  Only the free bodies with contacts have records ("slots", in body order), followed by one
+// that stands for every fixed body, so there are at most min(bodies, 2 K) of them.
 struct S32Scene {
-    float* c;          // kS32Floats per contact, in level order; row q at 12 q as three float4 groups
-                       // (lin[3], b | ang_lo[3], 1/diag | ang_hi[3], x); the torsion row's lin is (mu, 0, 0)
-    float* body;       // kS32BodyFloats per body: w[6], m^-1, fixed, I^-1 (xx, xy, xz, yy, yz, zz), padding
-    uint32_t* lohi;    // per contact in level order: scene-local lo | hi << 16
-    uint16_t* pos;     // level-order position of each contact (scene-local contact index -> position)
-    uint16_t* lptr;    // level starts (L + 1)
-    uint16_t* bptr;    // per body: start of its contact list in blist (nb + 1)
-    uint32_t* blist;   // per body, its contacts in ascending order: level-order position << 1 | side (2K)
+    char* c;       // kS32Floats per contact, in level order, as thirteen float4s: (lin, b) of the four rows, then
+                   // (ang_lo, 1/diag), then (ang_hi, mu), then the four impulses; the torsion row's lin is zero
+    char* body;    // kS32BodyFloats per slot: (w_lin, m^-1), (w_ang, fixed), I^-1 (xx, xy, xz, yy, yz, zz), padding
+    char* lohi;    // per contact in level order: slots lo | hi << 16, each with its top bit set for a fixed body
+    char* pos;     // level-order position of each contact (scene-local contact index -> position), while loading
+    char* bptr;    // per slot: start of its contact list in blist (n_free + 1)
+    char* blist;   // per slot, its contacts in ascending order: level-order position << 1 | side (2K)
+    char* steps;   // the sweep's steps: first position | contacts << 16 | flags; over pos, once that is used
+    int K, n_free, n_steps, warps;
 };
+constexpr uint32_t kStep32Ends = 1u << 31, kStep32Wide = 1u << 30;
+constexpr uint32_t kStep32Turns = 1u << 29;   // the next step is of the other width
 __host__ __device__ inline size_t s32_align(size_t v) { return (v + 15) & ~size_t(15); }
-// shared memory of a scene's FP32 copy; with in_l2 the contact rows, the level-order positions and the
-// per-body contact lists live in global memory (L2) and only the bodies, body indices and level and list
-// starts stay on chip
+// shared memory of a scene's FP32 copy with nr body records (and nb bodies); with in_l2 the contact rows, the
+// level-order positions and the per-body contact lists live in global memory (L2) and only the bodies, body indices
+// and level and list starts stay on chip
 __host__ __device__ inline size_t s32_bytes(int K, int nb, bool in_l2 = false, bool bodies_global = false) {
     return (in_l2 ? 0 : s32_align(sizeof(float) * (size_t)K * kS32Floats) + s32_align(sizeof(uint16_t) * (size_t)K) +
                         s32_align(sizeof(uint32_t) * 2 * (size_t)K)) +
@@ -2209,170 +2218,280 @@ __host__ __device__ inline size_t s32_bytes(int K, int nb, bool in_l2 = false, b
            s32_align(sizeof(uint32_t) * (size_t)K) +
            s32_align(sizeof(uint16_t) * (size_t)(K + 1)) + s32_align(sizeof(uint16_t) * (size_t)(nb + 1));
 }
-// with l2, the contact rows, positions and body lists go to the workspace; with bodies_global the body
+// body records a scene can need
+__host__ __device__ inline int s32_records(int K, int nb) { return nb < 2 * K ? nb : 2 * K; }
+// with l2, the contact rows, positions, steps and body lists go to the workspace; with bodies_global the body
 // records too (the scene's team is the only reader and writer, so block barriers keep them consistent)
-__device__ __forceinline__ S32Scene s32_carve(char* base, int K, int nb, const StepArgs* l2 = nullptr, int c0 = 0,
-                                              bool bodies_global = false, int b0 = 0) {
+__device__ __forceinline__ S32Scene s32_carve(char* base, int K, int nr, const StepArgs* l2 = nullptr, int c0 = 0,
+                                              int s = 0, bool bodies_global = false, int b0 = 0) {
     S32Scene f;
     size_t o = 0;
     auto take = [&](size_t bytes) { char* p = base + o; o += s32_align(bytes); return p; };
-    f.c = l2 ? l2->ws.c32 + kS32Floats * (size_t)c0 : (float*)take(sizeof(float) * (size_t)K * kS32Floats);
-    f.body = (l2 && bodies_global) ? l2->ws.body32 + kS32BodyFloats * (size_t)b0
-                                   : (float*)take(sizeof(float) * (size_t)nb * kS32BodyFloats);
-    f.lohi = (uint32_t*)take(sizeof(uint32_t) * (size_t)K);
-    f.pos = l2 ? l2->ws.pos32 + c0 : (uint16_t*)take(sizeof(uint16_t) * (size_t)K);
-    f.lptr = (uint16_t*)take(sizeof(uint16_t) * (size_t)(K + 1));
-    f.bptr = (uint16_t*)take(sizeof(uint16_t) * (size_t)(nb + 1));
-    f.blist = l2 ? l2->ws.blist32 + 2 * (size_t)c0 : (uint32_t*)take(sizeof(uint32_t) * 2 * (size_t)K);
+    f.c = l2 ? reinterpret_cast<char*>(l2->ws.c32 + kS32Floats * (size_t)c0) : take(sizeof(float) * (size_t)K * kS32Floats);
+    f.body = (l2 && bodies_global) ? reinterpret_cast<char*>(l2->ws.body32 + kS32BodyFloats * (size_t)b0)
+                                   : take(sizeof(float) * (size_t)nr * kS32BodyFloats);
+    f.lohi = take(sizeof(uint32_t) * (size_t)K);
+    // positions, then room of their size: together a word per contact for the steps (in L2: the level cursors)
+    f.pos = l2 ? reinterpret_cast<char*>(l2->ws.pos32 + c0) : take(sizeof(uint16_t) * (size_t)K);
+    take(sizeof(uint16_t) * (size_t)(K + 1));
+    f.steps = l2 ? reinterpret_cast<char*>(l2->ws.lev_cur + c0 + s) : f.pos;
+    f.bptr = take(sizeof(uint16_t) * (size_t)(nr + 1));
+    f.blist = l2 ? reinterpret_cast<char*>(l2->ws.blist32 + 2 * (size_t)c0) : take(sizeof(uint32_t) * 2 * (size_t)K);
+    f.K = K;
+    f.n_free = f.n_steps = 0;
+    f.warps = 1;
     return f;
 }
 
-__device__ __forceinline__ void f32_prox(float zs, float zt, float ztau, float mu, float xn, float* o) {
-    if (xn <= 0.0f) { o[0] = 0.0f; o[1] = 0.0f; o[2] = 0.0f; return; }
-    const float radius = mu * xn;
-    const float sqr = fmaf(zs, zs, fmaf(zt, zt, ztau * ztau));
-    if (sqr <= radius * radius) { o[0] = zs; o[1] = zt; o[2] = ztau; return; }
-    const float scale = radius * rsqrtf(sqr);
-    o[0] = zs * scale; o[1] = zt * scale; o[2] = ztau * scale;
-}
+// Addresses of a scene's copy: in shared memory by that space's own loads and stores (kept in program order, which
+// is the order the sweep wants them issued in), in L2 by ordinary ones.
+struct ShPtr {
+    uint32_t p;
+    __device__ __forceinline__ explicit ShPtr(char* q) : p((uint32_t)__cvta_generic_to_shared(q)) {}
+    __device__ __forceinline__ ShPtr(uint32_t q, int) : p(q) {}
+    __device__ __forceinline__ ShPtr operator+(uint32_t o) const { return ShPtr(p + o, 0); }
+    __device__ __forceinline__ float4 f4() const {
+        float4 v;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ float2 f2() const {
+        float2 v;
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ float f1() const {
+        float v;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(p) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ uint32_t u32() const {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ uint32_t u16() const {
+        uint32_t v;
+        asm volatile("{.reg .u16 t; ld.shared.u16 t, [%1]; cvt.u32.u16 %0, t;}" : "=r"(v) : "r"(p) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ void set(float v) const { asm volatile("st.shared.f32 [%0], %1;" ::"r"(p), "f"(v) : "memory"); }
+    __device__ __forceinline__ void set(float4 v) const {
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+    }
+};
+struct GlPtr {
+    char* p;
+    __device__ __forceinline__ explicit GlPtr(char* q) : p(q) {}
+    __device__ __forceinline__ GlPtr operator+(uint32_t o) const { return GlPtr(p + o); }
+    __device__ __forceinline__ float4 f4() const { return *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ float2 f2() const { return *reinterpret_cast<const float2*>(p); }
+    __device__ __forceinline__ float f1() const { return *reinterpret_cast<const float*>(p); }
+    __device__ __forceinline__ uint32_t u32() const { return *reinterpret_cast<const uint32_t*>(p); }
+    __device__ __forceinline__ uint32_t u16() const { return *reinterpret_cast<const uint16_t*>(p); }
+    __device__ __forceinline__ void set(float v) const { *reinterpret_cast<float*>(p) = v; }
+    __device__ __forceinline__ void set(float4 v) const { *reinterpret_cast<float4*>(p) = v; }
+};
+constexpr uint32_t kC32 = sizeof(float) * kS32Floats, kB32 = sizeof(float) * kS32BodyFloats;   // record strides
+// a contact record's offsets: piece j (0..2) of row q, and the impulses
+__device__ __forceinline__ uint32_t c32_at(int piece, int q) { return 64u * piece + 16u * q; }
+constexpr uint32_t kX32 = 192;
 
-// y = I^-1 t with I^-1 stored symmetric (xx, xy, xz, yy, yz, zz)
-__device__ __forceinline__ void s32_sym3(const float* I, const float* t, float* y) {
-    y[0] = fmaf(I[0], t[0], fmaf(I[1], t[1], I[2] * t[2]));
-    y[1] = fmaf(I[1], t[0], fmaf(I[3], t[1], I[4] * t[2]));
-    y[2] = fmaf(I[2], t[0], fmaf(I[4], t[1], I[5] * t[2]));
-}
-
-// J_q . [w_lo; w_hi] of row q (the torsion row has no linear part): three partial sums, then their total
-__device__ __forceinline__ float s32_jw(const float* row, int q, const float* wl, const float* wh) {
-    float lin = 0.0f;
-    if (q < 3) lin = fmaf(row[0], wl[0] - wh[0], fmaf(row[1], wl[1] - wh[1], row[2] * (wl[2] - wh[2])));
-    const float alo = fmaf(row[4], wl[3], fmaf(row[5], wl[4], row[6] * wl[5]));
-    const float ahi = fmaf(row[8], wh[3], fmaf(row[9], wh[4], row[10] * wh[5]));
-    return (lin + alo) + ahi;
+// Warps that sweep a scene of these levels: the number (a power of two) with the least cost.  A level of up to eight
+// contacts a warp is a step of quads and a wider one steps of a lane per contact, or, with the rows in L2 (in_l2),
+// more steps of quads.  The cycles of a step, in tens, are fitted to the solve times of 18 scenes of 240-510 contacts
+// (2 % off on average: quads 418, 411, 557 and lanes 723, 630, 1038 cycles with one, two and four warps; with quads
+// alone 64 scenes of up to 256 bodies took 4922, 4209, 4683 us, with both 4535, 3944, 4696) and, in L2, of one of 1565
+// (27256, 16884, 9525 us).  Every warp of the group counts for itself.
+__device__ __forceinline__ int s32_warps(const int* ptr, int L, int max_warps, bool in_l2) {
+    int cost[4] = {0, 0, 0, 0};
+    const int quads[4] = {in_l2 ? 120 : 42, in_l2 ? 125 : 41, in_l2 ? 112 : 56, in_l2 ? 140 : 100};
+    const int lanes[4] = {70, 63, 100, 140};
+    for (int l = threadIdx.x & 31; l < L; l += 32) {
+        const int n = ptr[l + 1] - ptr[l];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const int q = 8 << w;
+            cost[w] += in_l2 ? (n + q - 1) / q * quads[w] : n <= q ? quads[w] : (n + 4 * q - 1) / (4 * q) * lanes[w];
+        }
+    }
+    int best = 1, least = INT_MAX;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        const int c = __reduce_add_sync(0xffffffffu, cost[w]);
+        if ((1 << w) <= max_warps && c < least) { least = c; best = 1 << w; }
+    }
+    return best;
 }
 
 // copy scene R into the team's slab as FP32, contacts in level order; returns the number of levels
 template <class G>
-__device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const SceneRange& R, int s, const S32Scene& f,
-                                        bool coloured, int16_t* scratch) {
-    const int K = R.c1 - R.c0, nb = R.b1 - R.b0;
+__device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const SceneRange& R, int s, S32Scene& f,
+                                        bool coloured, bool in_l2, int16_t* scratch) {
+    const int K = f.K;
     // levels by relaxation in shared memory when a scratch is given (the rows' room, not yet filled)
     const int L = coloured ? scene_colours(a, g, R, s)
                 : scratch ? scene_levels_smem(a, g, R, s, scratch) : scene_levels(a, g, R, s);
     const int* order = a.ws.lev_order + R.c0;
-    for (int t = g.rank(); t < 16 * K; t += g.size()) {   // (position, row, float4 group; part 3 idle)
-        const int i = t >> 4, q = (t >> 2) & 3, part = t & 3;
+    float* c = reinterpret_cast<float*>(f.c);
+    for (int t = g.rank(); t < 16 * K; t += g.size()) {   // (position, float4 group, row), impulses last
+        const int i = t >> 4, part = (t >> 2) & 3, q = t & 3;
         const size_t k = (size_t)order[i];
-        float* row = f.c + kS32Floats * i + 12 * q;
+        float* o = c + kS32Floats * (size_t)i + 16 * part;
         const double* J = a.ws.J + 48 * k;
+        float4 v;
         if (part == 0) {
-            row[0] = q < 3 ? (float)J[j_at(q, 0)] : (float)a.ws.mu[k];
-            row[1] = q < 3 ? (float)J[j_at(q, 1)] : 0.0f;
-            row[2] = q < 3 ? (float)J[j_at(q, 2)] : 0.0f;
-            row[3] = (float)a.ws.b[4 * k + q];
+            v.x = q < 3 ? (float)J[j_at(q, 0)] : 0.0f;
+            v.y = q < 3 ? (float)J[j_at(q, 1)] : 0.0f;
+            v.z = q < 3 ? (float)J[j_at(q, 2)] : 0.0f;
+            v.w = (float)a.ws.b[4 * k + q];
         } else if (part == 1) {
-            row[4] = (float)J[j_at(q, 3)]; row[5] = (float)J[j_at(q, 4)]; row[6] = (float)J[j_at(q, 5)];
-            row[7] = (float)(1.0 / a.ws.diag[4 * k + q]);
+            v.x = (float)J[j_at(q, 3)]; v.y = (float)J[j_at(q, 4)]; v.z = (float)J[j_at(q, 5)];
+            v.w = (float)(1.0 / a.ws.diag[4 * k + q]);
         } else if (part == 2) {
-            row[8] = (float)J[j_at(q, 9)]; row[9] = (float)J[j_at(q, 10)]; row[10] = (float)J[j_at(q, 11)];
-            row[11] = (float)a.ws.x[4 * k + q];
+            v.x = (float)J[j_at(q, 9)]; v.y = (float)J[j_at(q, 10)]; v.z = (float)J[j_at(q, 11)];
+            v.w = (float)a.ws.mu[k];
+        } else {
+            o[q] = (float)a.ws.x[4 * k + q];
+            continue;
+        }
+        reinterpret_cast<float4*>(o)[q] = v;
+    }
+    // the slots: the free bodies with contacts in body order (their lists in bc_list then follow one another)
+    const int e0 = a.ws.bc_ptr[R.b0];
+    uint16_t* bptr = reinterpret_cast<uint16_t*>(f.bptr);
+    int n = g.append_begin();
+    for (int base = R.b0; base < R.b1; base += g.size()) {
+        const int b = base + g.rank();
+        const int p0 = b < R.b1 ? a.ws.bc_ptr[b] : 0, p1 = b < R.b1 ? a.ws.bc_ptr[b + 1] : 0;
+        const int at = g.append(p1 > p0, n);
+        if (p1 > p0) {
+            a.ws.bc_fill[b] = at;
+            bptr[at] = (uint16_t)(p0 - e0);
+            float* B = reinterpret_cast<float*>(f.body + kB32 * (size_t)at);
+            const double* Wi = a.ws.Winv + 9 * (size_t)b;
+            B[3] = (float)(1.0 / a.bd.mass[b]);
+            B[7] = 0.0f;
+            B[8] = (float)Wi[0]; B[9] = (float)Wi[1]; B[10] = (float)Wi[2];
+            B[11] = (float)Wi[4]; B[12] = (float)Wi[5]; B[13] = (float)Wi[8];
         }
     }
+    g.append_end(n);
+    f.n_free = n;
+    if (g.rank() == 0) bptr[n] = (uint16_t)(a.ws.bc_ptr[R.b1] - e0);
+    if (n < s32_records(K, R.b1 - R.b0) && g.rank() < kS32BodyFloats)   // the fixed bodies' record
+        reinterpret_cast<float*>(f.body + kB32 * (size_t)n)[g.rank()] = g.rank() == 7 ? 1.0f : 0.0f;
+    g.sync();   // slots complete
+    uint16_t* pos = reinterpret_cast<uint16_t*>(f.pos);
+    uint32_t* lohi = reinterpret_cast<uint32_t*>(f.lohi);
     for (int i = g.rank(); i < K; i += g.size()) {
         const int k = order[i];
-        f.pos[k - R.c0] = (uint16_t)i;
-        f.lohi[i] = (uint32_t)(a.ws.lohi[2 * k] - R.b0) | ((uint32_t)(a.ws.lohi[2 * k + 1] - R.b0) << 16);
+        pos[k - R.c0] = (uint16_t)i;
+        const int lo = a.ws.lohi[2 * k], hi = a.ws.lohi[2 * k + 1];
+        lohi[i] = (uint32_t)(a.bd.fixed[lo] ? 0x8000 | n : a.ws.bc_fill[lo]) |
+                  ((uint32_t)(a.bd.fixed[hi] ? 0x8000 | n : a.ws.bc_fill[hi]) << 16);
     }
-    for (int l = g.rank(); l <= L; l += g.size()) f.lptr[l] = (uint16_t)a.ws.lev_ptr[R.c0 + s + l];
     g.sync();   // pos complete
     // per-body contact lists (the residual's w = W J^T x), positions in level order
-    const int e0 = a.ws.bc_ptr[R.b0];
-    for (int bl = g.rank(); bl <= nb; bl += g.size()) f.bptr[bl] = (uint16_t)(a.ws.bc_ptr[R.b0 + bl] - e0);
+    uint32_t* blist = reinterpret_cast<uint32_t*>(f.blist);
     for (int e = g.rank(); e < a.ws.bc_ptr[R.b1] - e0; e += g.size()) {
         const int code = a.ws.bc_list[e0 + e];
-        f.blist[e] = ((uint32_t)f.pos[(code >> 1) - R.c0] << 1) | (uint32_t)(code & 1);
+        blist[e] = ((uint32_t)pos[(code >> 1) - R.c0] << 1) | (uint32_t)(code & 1);
     }
-    for (int bl = g.rank(); bl < nb; bl += g.size()) {
-        const int b = R.b0 + bl;
-        float* B = f.body + kS32BodyFloats * bl;
-        const bool fx = a.bd.fixed[b] != 0;
-        const double* Wi = a.ws.Winv + 9 * (size_t)b;
-        B[6] = fx ? 0.0f : (float)(1.0 / a.bd.mass[b]);
-        B[7] = fx ? 1.0f : 0.0f;
-        // a fixed body's update is zero (m^-1 = I^-1 = 0); the sweeps still only store to free bodies
-        B[8] = fx ? 0.0f : (float)Wi[0]; B[9] = fx ? 0.0f : (float)Wi[1]; B[10] = fx ? 0.0f : (float)Wi[2];
-        B[11] = fx ? 0.0f : (float)Wi[4]; B[12] = fx ? 0.0f : (float)Wi[5]; B[13] = fx ? 0.0f : (float)Wi[8];
-    }
+    g.sync();   // pos used: the steps take its room
+    const int* ptr = a.ws.lev_ptr + R.c0 + s;
+    f.warps = g.size() > 32 ? s32_warps(ptr, L, g.size() >> 5, in_l2) : 1;
+    uint32_t* steps = reinterpret_cast<uint32_t*>(f.steps);
+    f.n_steps = sweep_steps(g, ptr, L, in_l2 ? 0 : 8 * f.warps, in_l2 ? 8 * f.warps : 32 * f.warps, [&](int at, int start, int count, bool ends, bool wide) {
+        steps[at] = (uint32_t)start | ((uint32_t)count << 16) | (ends ? kStep32Ends : 0u) | (wide && !in_l2 ? kStep32Wide : 0u);
+    });
+    g.sync();
+    for (int i = g.rank(); i < f.n_steps; i += g.size())   // (reads only the widths of others, which stay)
+        if (((steps[i] ^ steps[i + 1 < f.n_steps ? i + 1 : 0]) & kStep32Wide) != 0) atomicOr(steps + i, kStep32Turns);
     g.sync();
     return L;
 }
 
-// w = W J^T x (each body sums its contacts in ascending order)
-template <class G>
-__device__ __forceinline__ void s32_rebuild_w(const G& g, const SceneRange& R, const S32Scene& f) {
-    const int nb = R.b1 - R.b0;
-    for (int bl = g.rank(); bl < nb; bl += g.size()) {
-        float* B = f.body + kS32BodyFloats * bl;
-        float P[3] = {0.f, 0.f, 0.f}, T[3] = {0.f, 0.f, 0.f};
-        if (B[7] == 0.0f) {   // rows read as float4 groups (lin, b | ang_lo, 1/diag | ang_hi, x)
-            for (int e = f.bptr[bl]; e < f.bptr[bl + 1]; ++e) {
-                const uint32_t code = f.blist[e];
-                const int side = code & 1;
-                const float4* C4 = reinterpret_cast<const float4*>(f.c + kS32Floats * (code >> 1));
-                for (int q = 0; q < 4; ++q) {
-                    const float4 lin = C4[3 * q], alo = C4[3 * q + 1], ahi = C4[3 * q + 2];
-                    const float xq = ahi.w;
-                    if (q < 3) {
-                        const float sx = side ? -xq : xq;
-                        P[0] = fmaf(lin.x, sx, P[0]); P[1] = fmaf(lin.y, sx, P[1]); P[2] = fmaf(lin.z, sx, P[2]);
-                    }
-                    const float4 ang = side ? ahi : alo;
-                    T[0] = fmaf(ang.x, xq, T[0]); T[1] = fmaf(ang.y, xq, T[1]); T[2] = fmaf(ang.z, xq, T[2]);
-                }
-            }
+// w = W J^T x: two lanes per slot, one for the linear and one for the angular components, each body's contacts
+// summed in ascending order
+template <class P, class G>
+__device__ __noinline__ void s32_rebuild_w(const G g, const S32Scene f) {
+    const P c(f.c), body(f.body), bptr(f.bptr), blist(f.blist);
+    const int ang = g.rank() & 1;
+    for (int i = g.rank() >> 1; i < f.n_free; i += g.size() >> 1) {
+        uint32_t e = (bptr + 2u * i).u16();
+        const uint32_t e1 = (bptr + (2u * i + 2u)).u16();
+        const P B = body + kB32 * i;
+        float S[3] = {0.f, 0.f, 0.f};
+        uint32_t code = (blist + 4u * e).u32();
+        for (; e < e1; ++e) {
+            const uint32_t side = code & 1u;
+            const P rec = c + kC32 * (code >> 1);
+            const P col = rec + (ang ? 64u + 64u * side : 0u);
+            const float4 v0 = col.f4(), v1 = (col + 16u).f4(), v2 = (col + 32u).f4(), v3 = (col + 48u).f4();
+            const float4 x = (rec + kX32).f4();
+            code = (blist + 4u * min(e + 1u, e1 - 1u)).u32();
+            const float sg = !ang && side ? -1.0f : 1.0f;   // lin_hi = -lin_lo
+            const float x0 = sg * x.x, x1 = sg * x.y, x2 = sg * x.z, x3 = sg * x.w;
+            S[0] = fmaf(v0.x, x0, S[0]); S[1] = fmaf(v0.y, x0, S[1]); S[2] = fmaf(v0.z, x0, S[2]);
+            S[0] = fmaf(v1.x, x1, S[0]); S[1] = fmaf(v1.y, x1, S[1]); S[2] = fmaf(v1.z, x1, S[2]);
+            S[0] = fmaf(v2.x, x2, S[0]); S[1] = fmaf(v2.y, x2, S[1]); S[2] = fmaf(v2.z, x2, S[2]);
+            S[0] = fmaf(v3.x, x3, S[0]); S[1] = fmaf(v3.y, x3, S[1]); S[2] = fmaf(v3.z, x3, S[2]);
         }
-        float om[3];
-        s32_sym3(B + 8, T, om);
-        B[0] = B[6] * P[0]; B[1] = B[6] * P[1]; B[2] = B[6] * P[2];
-        B[3] = om[0]; B[4] = om[1]; B[5] = om[2];
+        const float4 I0 = (B + 32u).f4();
+        const float2 I1 = (B + 48u).f2();
+        if (ang) {
+            (B + 16u).set(make_float4(fmaf(I0.x, S[0], fmaf(I0.y, S[1], I0.z * S[2])),
+                                      fmaf(I0.y, S[0], fmaf(I0.w, S[1], I1.x * S[2])),
+                                      fmaf(I0.z, S[0], fmaf(I1.x, S[1], I1.y * S[2])), 0.0f));
+        } else {
+            const float m = (B + 12u).f1();
+            B.set(make_float4(m * S[0], m * S[1], m * S[2], m));
+        }
     }
     g.sync();
 }
 
-// w = W J^T x, then the FP32 residual ||x - prox(x - D^-1 (A x + b))||_inf / max(1, ||x||_inf)
-template <class G>
-__device__ __forceinline__ float s32_residual(const StepArgs& a, const G& g, const SceneRange& R, const S32Scene& f) {
-    const int K = R.c1 - R.c0;
-    s32_rebuild_w(g, R, f);
+// J_q . [w_lo; w_hi] of a contact's row q: three partial sums, then their total (the torsion row's lin is zero)
+__device__ __forceinline__ float s32_jw(float4 r0, float4 r1, float4 r2, float4 l0, float4 l1, float4 h0, float4 h1) {
+    const float lin = fmaf(r0.x, l0.x - h0.x, fmaf(r0.y, l0.y - h0.y, r0.z * (l0.z - h0.z)));
+    const float alo = fmaf(r1.x, l1.x, fmaf(r1.y, l1.y, r1.z * l1.z));
+    const float ahi = fmaf(r2.x, h1.x, fmaf(r2.y, h1.y, r2.z * h1.z));
+    return (lin + alo) + ahi;
+}
+__device__ __forceinline__ void quad_gather(float z, float* o) {
+    const int base = (threadIdx.x & 31) & ~3;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = __shfl_sync(0xffffffffu, z, base | i);
+}
+
+// w = W J^T x, then the FP32 residual ||x - prox(x - D^-1 (A x + b))||_inf / max(1, ||x||_inf), a quad per contact
+template <class P, class G>
+__device__ __noinline__ float s32_residual(const G g, const S32Scene f) {
+    s32_rebuild_w<P>(g, f);
+    const P c(f.c), body(f.body), lohi(f.lohi);
+    const int q = g.rank() & 3, nslot = g.size() >> 2;
     float m = 0.0f, xm = 0.0f;
-    for (int i = g.rank(); i < K; i += g.size()) {
-        const float4* C4 = reinterpret_cast<const float4*>(f.c + kS32Floats * i);
-        const uint32_t lh = f.lohi[i];
-        const float* Bl = f.body + kS32BodyFloats * (int)(lh & 0xffffu);
-        const float* Bh = f.body + kS32BodyFloats * (int)(lh >> 16);
-        const float4 l0 = *reinterpret_cast<const float4*>(Bl), l1 = *reinterpret_cast<const float4*>(Bl + 4);
-        const float4 h0 = *reinterpret_cast<const float4*>(Bh), h1 = *reinterpret_cast<const float4*>(Bh + 4);
-        float z[4], x[4];
-        float mu = 0.0f;
-        for (int q = 0; q < 4; ++q) {   // the expressions of s32_jw, on float4 loads
-            const float4 r0 = C4[3 * q], r1 = C4[3 * q + 1], r2 = C4[3 * q + 2];
-            float lin = 0.0f;
-            if (q < 3) lin = fmaf(r0.x, l0.x - h0.x, fmaf(r0.y, l0.y - h0.y, r0.z * (l0.z - h0.z)));
-            else mu = r0.x;
-            const float alo = fmaf(r1.x, l0.w, fmaf(r1.y, l1.x, r1.z * l1.y));
-            const float ahi = fmaf(r2.x, h0.w, fmaf(r2.y, h1.x, r2.z * h1.y));
-            x[q] = r2.w;
-            z[q] = x[q] - r1.w * (((lin + alo) + ahi) + r0.w);
-        }
+    for (int i0 = 0; i0 < f.K; i0 += nslot) {
+        const int at = i0 + (g.rank() >> 2), i = min(at, f.K - 1);
+        const uint32_t lh = (lohi + 4u * i).u32();
+        const P rec = c + kC32 * i, row = rec + 16u * q;
+        const P Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
+        const float4 r0 = row.f4(), r1 = (row + 64u).f4(), r2 = (row + 128u).f4();
+        const float4 l0 = Bl.f4(), l1 = (Bl + 16u).f4(), h0 = Bh.f4(), h1 = (Bh + 16u).f4();
+        const float x = (rec + kX32 + 4u * q).f1();
+        float z[4];
+        const float zq = x - r1.w * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
+        quad_gather(zq, z);
         const float pn = fmaxf(z[0], 0.0f);
-        float fr[3];
-        f32_prox(z[1], z[2], z[3], mu, pn, fr);
-        const float d[4] = {x[0] - pn, x[1] - fr[0], x[2] - fr[1], x[3] - fr[2]};
-        for (int t = 0; t < 4; ++t) {
-            m = fmaxf(m, fabsf(d[t]));
-            if (d[t] != d[t]) m = d[t];
-            xm = fmaxf(xm, fabsf(x[t]));
+        const float radius = r2.w * pn;
+        const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
+        const float fr = pn <= 0.0f ? 0.0f : (sqr <= radius * radius ? zq : zq * (radius * rsqrtf(sqr)));
+        const float d = x - (q == 0 ? pn : fr);
+        if (at < f.K) {
+            m = fmaxf(m, fabsf(d));
+            if (d != d) m = d;
+            xm = fmaxf(xm, fabsf(x));
         }
     }
     const double mres = g.max((double)m);
@@ -2380,226 +2499,227 @@ __device__ __forceinline__ float s32_residual(const StepArgs& a, const G& g, con
     return (float)(mres / (mx > 1.0 ? mx : 1.0));
 }
 
-// One Gauss-Seidel sweep over the levels, four lanes per contact.  Lane q computes row q of J w; the z of
-// the four rows meet by shuffles and every lane applies the prox; lane q then forms one 3-vector of the
-// update from the four rows' float4 group it owns (lin for q = 0, 1; ang_lo for 2; ang_hi for 3) and applies
-// +m^-1, -m^-1, I_lo^-1 or I_hi^-1 to it.  Every lane runs the same instructions (lane-dependent offsets);
-// all shared-memory reads are float4 / float2.
-template <class G, bool kL2>
-__device__ __forceinline__ void s32_sweep(const G& g, const S32Scene& f, int L, float rscale, bool bodies_global) {
-    const int q = g.rank() & 3, slot = g.rank() >> 2, nslot = g.size() >> 2;
-    const int base = (threadIdx.x & 31) & ~3;
-    const unsigned qm = 0xfu << base;
-    const int grp = q < 2 ? 0 : q - 1;          // the float4 group of the update columns this lane sums
-    const bool on_hi = (q & 1) != 0;            // lanes 1 and 3 update the hi body
-    const bool linear = q < 2;
-    int start = f.lptr[0], end = f.lptr[1];
-    for (int l = 1; l <= L; ++l) {
-        const int next_end = l < L ? f.lptr[l + 1] : end;
-        if (kL2) {   // rows in L2: pull the next level's rows (contiguous in level order) into L1 meanwhile
-            const char* p0 = reinterpret_cast<const char*>(f.c + kS32Floats * (size_t)end);
-            const int lines = (int)(((size_t)(next_end - end) * kS32Floats * sizeof(float) + 127) / 128);
-            for (int t = g.rank(); t < lines; t += g.size())
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(p0 + 128 * (size_t)t));
-            if (bodies_global)   // and the body records those rows touch
-                for (int i = end + g.rank(); i < next_end; i += g.size()) {
-                    const uint32_t lh = f.lohi[i];
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(f.body + kS32BodyFloats * (size_t)(lh & 0xffffu)));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(f.body + kS32BodyFloats * (size_t)(lh >> 16)));
-                }
-        }
-        // one contact update; every lane of a quad takes the same contacts, so its shuffles see all four lanes
-        auto update = [&](int i) {
-                const float4* C4 = reinterpret_cast<const float4*>(f.c + kS32Floats * i);
-                const uint32_t lh = f.lohi[i];
-                float* Bl = f.body + kS32BodyFloats * (int)(lh & 0xffffu);
-                float* Bh = f.body + kS32BodyFloats * (int)(lh >> 16);
-                const float4 r0 = C4[3 * q], r1 = C4[3 * q + 1], r2 = C4[3 * q + 2];   // own row
-                float4 v[4];                                                         // update columns
-                for (int j = 0; j < 4; ++j) v[j] = C4[3 * j + grp];
-                float xo[4];
-                for (int j = 0; j < 4; ++j) xo[j] = f.c[kS32Floats * i + 12 * j + 11];
-                const float4 l0 = *reinterpret_cast<const float4*>(Bl);
-                const float4 l1 = *reinterpret_cast<const float4*>(Bl + 4);
-                const float4 h0 = *reinterpret_cast<const float4*>(Bh);
-                const float4 h1 = *reinterpret_cast<const float4*>(Bh + 4);
-                float* B = on_hi ? Bh : Bl;
-                const float4 I0 = *reinterpret_cast<const float4*>(B + 8);
-                const float2 I1 = *reinterpret_cast<const float2*>(B + 12);
-                // J_q w: linear part (rows 0-2), angular parts of both bodies
-                float lin = fmaf(r0.x, l0.x - h0.x, fmaf(r0.y, l0.y - h0.y, r0.z * (l0.z - h0.z)));
-                if (q == 3) lin = 0.0f;
-                const float alo = fmaf(r1.x, l0.w, fmaf(r1.y, l1.x, r1.z * l1.y));
-                const float ahi = fmaf(r2.x, h0.w, fmaf(r2.y, h1.x, r2.z * h1.y));
-                const float z = r2.w - rscale * r1.w * (((lin + alo) + ahi) + r0.w);
-                float zz[4];
-                for (int j = 0; j < 4; ++j) zz[j] = __shfl_sync(qm, z, base | j);
-                const float mu = __shfl_sync(qm, r0.x, base | 3);
-                const float xn = fmaxf(zz[0], 0.0f);
-                // prox onto the friction ball of radius mu xn, without branches
-                const float radius = mu * xn;
-                const float sqr = fmaf(zz[1], zz[1], fmaf(zz[2], zz[2], zz[3] * zz[3]));
+// n_sweeps projected Gauss-Seidel sweeps over the levels, as one sequence of steps.  A narrow step takes a quad of
+// lanes per contact: lane q computes z_q from the current w, the four z meet by shuffles and every lane applies the
+// prox (branch-free); the lane then forms one 3-vector of the update -- lin columns for the lo and the hi body (lanes
+// 0 and 1), ang_lo (2), ang_hi (3) -- applies that part of W to it and stores its float4 of w (the linear lanes apply
+// m^-1 as a diagonal matrix).  A wide step takes one lane per contact, which computes all four rows as independent
+// chains and updates both bodies.  Every expression has the same operands in the same order, so both give the same
+// bits.
+//
+// Bound by one contact's chain (~250 cycles: row product, reciprocal root, update, shared-memory store and load) and by
+// the instructions of a step, which one warp issues every ~2.5 cycles: ~150 with a quad per contact, ~250 with a lane.
+// A step of quads takes ~420 cycles and one of lanes ~700, but the quads of four warps hold one another up in the
+// shared-memory pipe (four 128-byte wavefronts a load: 560 cycles).  (One lane per contact at every level, its rows
+// loaded after the level's barrier: ~570 cycles.)  The values of the next step's
+// contact are loaded as soon as the current ones are used up, its indices a step before that, and the loads and
+// shuffles, which share one queue, are issued in the order of their need.
+template <class P, class G>
+__device__ __noinline__ void s32_sweep(const G g, const S32Scene f, float rscale, int n_sweeps) {
+    const P c(f.c), body(f.body), lohi(f.lohi), steps(f.steps);
+    const int rank = g.rank(), last = f.n_steps - 1;
+    auto step = [&](int j) { return (steps + 4u * j).u32(); };
+    auto after = [&](int j) { return j < last ? j + 1 : 0; };   // the sequence goes on from sweep to sweep
+    int j = 0;
+    uint32_t st0 = step(0);
+#pragma unroll 1
+    for (int left = n_sweeps * f.n_steps; left > 0;) {
+        if (!(st0 & kStep32Wide)) {
+            // a run of narrow steps
+            const int q = rank & 3, slot = rank >> 2;
+            const bool linear = q < 2;
+            const uint32_t hi_shift = (q & 1) ? 16u : 0u;          // lanes 1 and 3 update the hi body
+            const uint32_t fixed_bit = 0x8000u << hi_shift;
+            const uint32_t part = linear ? 0u : 16u;                // their float4 of w
+            const uint32_t col = linear ? 0u : 64u * (uint32_t)(q - 1);   // the piece whose columns the lane sums
+            const float sg = q == 1 ? -1.0f : 1.0f;
+            auto at = [&](uint32_t st) { return min((int)(st & 0x7fffu) + slot, f.K - 1); };
+            int j2 = after(after(j));
+            uint32_t st1 = step(after(j));
+            P rec = c + kC32 * at(st0);
+            uint32_t lh = (lohi + 4u * at(st0)).u32();
+            float4 r0 = (rec + 16u * q).f4(), r1 = (rec + (64u + 16u * q)).f4(), r2 = (rec + (128u + 16u * q)).f4();
+            float4 x = (rec + kX32).f4();
+            float xq = (rec + (kX32 + 4u * q)).f1();
+            int i_next = at(st1);
+            uint32_t lh_next = (lohi + 4u * i_next).u32();
+            bool more;
+#pragma unroll 1
+            do {
+                const P Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
+                const float4 l0 = Bl.f4(), h0 = Bh.f4(), l1 = (Bl + 16u).f4(), h1 = (Bh + 16u).f4();
+                const float zq = xq - rscale * r1.w * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
+                float z[4];
+                quad_gather(zq, z);
+                const P cl = rec + col;
+                const float4 v0 = cl.f4(), v1 = (cl + 16u).f4(), v2 = (cl + 32u).f4(), v3 = (cl + 48u).f4();
+                const P B = body + kB32 * ((lh >> hi_shift) & 0x7fffu);
+                const float4 own = (B + part).f4();
+                const float4 I0 = (B + 32u).f4();
+                const float2 I1 = (B + 48u).f2();
+                const float xn = fmaxf(z[0], 0.0f);
+                // prox onto the friction ball of radius mu xn
+                const float radius = r2.w * xn;
+                const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
                 float scale = sqr > radius * radius ? radius * rsqrtf(sqr) : 1.0f;
                 if (xn <= 0.0f) scale = 0.0f;
-                const float f1 = zz[1] * scale, f2 = zz[2] * scale, f3 = zz[3] * scale;
-                const float d0 = xn - xo[0], d1 = f1 - xo[1], d2 = f2 - xo[2];
-                const float d3 = linear ? 0.0f : f3 - xo[3];   // the torsion row has no linear columns
-                const float xq = q == 0 ? xn : (q == 1 ? f1 : (q == 2 ? f2 : f3));
-                f.c[kS32Floats * i + 12 * q + 11] = xq;
-                const float T0 = fmaf(v[2].x, d2, fmaf(v[1].x, d1, v[0].x * d0));
-                const float T1 = fmaf(v[2].y, d2, fmaf(v[1].y, d1, v[0].y * d0));
-                const float T2 = fmaf(v[2].z, d2, fmaf(v[1].z, d1, v[0].z * d0));
-                // the torsion row has no linear columns: linear lanes sum three rows
-                const float S0 = linear ? T0 : fmaf(v[3].x, d3, T0);
-                const float S1 = linear ? T1 : fmaf(v[3].y, d3, T1);
-                const float S2 = linear ? T2 : fmaf(v[3].z, d3, T2);
-                // the lane's body: w, m^-1 and fixed flag were loaded above
-                const float4 w0 = on_hi ? h0 : l0;
-                const float4 w1 = on_hi ? h1 : l1;
-                const float m = on_hi ? -w1.z : w1.z;
-                const float dw0 = linear ? m * S0 : fmaf(I0.x, S0, fmaf(I0.y, S1, I0.z * S2));
-                const float dw1 = linear ? m * S1 : fmaf(I0.y, S0, fmaf(I0.w, S1, I1.x * S2));
-                const float dw2 = linear ? m * S2 : fmaf(I0.z, S0, fmaf(I1.x, S1, I1.y * S2));
-                // the lane's three components of w: linear (0-2) or angular (3-5), without a branch
-                const int off = linear ? 0 : 3;
-                const float o0 = linear ? w0.x : w0.w, o1 = linear ? w0.y : w1.x, o2 = linear ? w0.z : w1.y;
-                if (w1.w == 0.0f) {   // not a fixed body
-                    B[off] = o0 + dw0; B[off + 1] = o1 + dw1; B[off + 2] = o2 + dw2;
+                const uint32_t st2 = step(j2);
+                j2 = after(j2);
+                const P rec_next = c + kC32 * i_next;
+                r0 = (rec_next + 16u * q).f4(); r1 = (rec_next + (64u + 16u * q)).f4(); r2 = (rec_next + (128u + 16u * q)).f4();
+                const float f1 = z[1] * scale, f2 = z[2] * scale, f3 = z[3] * scale;
+                const float d0 = xn - x.x, d1 = f1 - x.y, d2 = f2 - x.z, d3 = f3 - x.w;
+                const float yq = q == 0 ? xn : zq * scale;
+                // the lane's part of W: m^-1 on the diagonal (negative for the hi body: lin_hi = -lin_lo), or I^-1
+                const float m = sg * own.w;
+                const float wxx = linear ? m : I0.x, wxy = linear ? 0.0f : I0.y, wxz = linear ? 0.0f : I0.z;
+                const float wyy = linear ? m : I0.w, wyz = linear ? 0.0f : I1.x, wzz = linear ? m : I1.y;
+                const float S0 = fmaf(v3.x, d3, fmaf(v2.x, d2, fmaf(v1.x, d1, v0.x * d0)));
+                const float S1 = fmaf(v3.y, d3, fmaf(v2.y, d2, fmaf(v1.y, d1, v0.y * d0)));
+                const float S2 = fmaf(v3.z, d3, fmaf(v2.z, d2, fmaf(v1.z, d1, v0.z * d0)));
+                const float4 n = make_float4(own.x + fmaf(wxx, S0, fmaf(wxy, S1, wxz * S2)),
+                                             own.y + fmaf(wxy, S0, fmaf(wyy, S1, wyz * S2)),
+                                             own.z + fmaf(wxz, S0, fmaf(wyz, S1, wzz * S2)), own.w);
+                // the fixed bodies' record is only read; an idle quad writes nothing
+                const bool mine = slot < (int)((st0 >> 16) & 0x1fffu);
+                if (mine && !(lh & fixed_bit)) (B + part).set(n);
+                if (mine) (rec + (kX32 + 4u * q)).set(yq);
+                // after the stores: a scene of one step sweeps the same contacts again
+                x = (rec_next + kX32).f4();
+                xq = (rec_next + (kX32 + 4u * q)).f1();
+                if (st0 & kStep32Ends) g.sync();
+                more = --left > 0 && !(st0 & kStep32Turns);
+                st0 = st1; st1 = st2;
+                rec = rec_next;
+                lh = lh_next;
+                i_next = at(st2);
+                lh_next = (lohi + 4u * i_next).u32();
+                j = after(j);
+            } while (more);
+        } else {
+            // a run of wide steps
+            auto at = [&](uint32_t st) { return min((int)(st & 0x7fffu) + rank, f.K - 1); };
+            uint32_t st1 = step(after(j));
+            P rec = c + kC32 * at(st0);
+            uint32_t lh = (lohi + 4u * at(st0)).u32();
+            float4 r[12];
+#pragma unroll
+            for (int t = 0; t < 12; ++t) r[t] = (rec + 16u * t).f4();
+            float4 x = (rec + kX32).f4();
+            bool more;
+#pragma unroll 1
+            do {
+                const P Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
+                const float4 l0 = Bl.f4(), h0 = Bh.f4(), l1 = (Bl + 16u).f4(), h1 = (Bh + 16u).f4();
+                const float xs[4] = {x.x, x.y, x.z, x.w};
+                float z[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float4 r0 = r[k], r1 = r[4 + k], r2 = r[8 + k];
+                    float lin = 0.0f;
+                    if (k < 3) lin = fmaf(r0.x, l0.x - h0.x, fmaf(r0.y, l0.y - h0.y, r0.z * (l0.z - h0.z)));
+                    const float alo = fmaf(r1.x, l1.x, fmaf(r1.y, l1.y, r1.z * l1.z));
+                    const float ahi = fmaf(r2.x, h1.x, fmaf(r2.y, h1.y, r2.z * h1.z));
+                    z[k] = xs[k] - rscale * r1.w * (((lin + alo) + ahi) + r0.w);
                 }
-        };
-        // the first pass outside the loop: most levels hold no more contacts than a team has quads
-        int i = start + slot;
-        if (i < end) {
-            update(i);
-            for (i += nslot; i < end; i += nslot) update(i);
+                const float mu = r[8].w;
+                float4 v[12];   // the rows once more, for the update: the next ones take r
+#pragma unroll
+                for (int t = 0; t < 12; ++t) v[t] = (rec + 16u * t).f4();
+                const float4 Il0 = (Bl + 32u).f4(), Ih0 = (Bh + 32u).f4();
+                const float2 Il1 = (Bl + 48u).f2(), Ih1 = (Bh + 48u).f2();
+                const P rec_next = c + kC32 * at(st1);
+                const uint32_t lh_next = (lohi + 4u * at(st1)).u32();
+#pragma unroll
+                for (int t = 0; t < 12; ++t) r[t] = (rec_next + 16u * t).f4();
+                const float xn = fmaxf(z[0], 0.0f);
+                const float radius = mu * xn;
+                const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
+                float scale = sqr > radius * radius ? radius * rsqrtf(sqr) : 1.0f;
+                if (xn <= 0.0f) scale = 0.0f;
+                const float f1 = z[1] * scale, f2 = z[2] * scale, f3 = z[3] * scale;
+                const float d0 = xn - x.x, d1 = f1 - x.y, d2 = f2 - x.z, d3 = f3 - x.w;
+                // the three sums of the update (the torsion row has no linear columns)
+                const float L0 = fmaf(v[2].x, d2, fmaf(v[1].x, d1, v[0].x * d0));
+                const float L1 = fmaf(v[2].y, d2, fmaf(v[1].y, d1, v[0].y * d0));
+                const float L2 = fmaf(v[2].z, d2, fmaf(v[1].z, d1, v[0].z * d0));
+                const float A0 = fmaf(v[7].x, d3, fmaf(v[6].x, d2, fmaf(v[5].x, d1, v[4].x * d0)));
+                const float A1 = fmaf(v[7].y, d3, fmaf(v[6].y, d2, fmaf(v[5].y, d1, v[4].y * d0)));
+                const float A2 = fmaf(v[7].z, d3, fmaf(v[6].z, d2, fmaf(v[5].z, d1, v[4].z * d0)));
+                const float H0 = fmaf(v[11].x, d3, fmaf(v[10].x, d2, fmaf(v[9].x, d1, v[8].x * d0)));
+                const float H1 = fmaf(v[11].y, d3, fmaf(v[10].y, d2, fmaf(v[9].y, d1, v[8].y * d0)));
+                const float H2 = fmaf(v[11].z, d3, fmaf(v[10].z, d2, fmaf(v[9].z, d1, v[8].z * d0)));
+                const float ml = l0.w, mh = -h0.w;
+                const bool mine = rank < (int)((st0 >> 16) & 0x1fffu);
+                if (mine && !(lh & 0x8000u)) {
+                    Bl.set(make_float4(l0.x + ml * L0, l0.y + ml * L1, l0.z + ml * L2, ml));
+                    (Bl + 16u).set(make_float4(l1.x + fmaf(Il0.x, A0, fmaf(Il0.y, A1, Il0.z * A2)),
+                                               l1.y + fmaf(Il0.y, A0, fmaf(Il0.w, A1, Il1.x * A2)),
+                                               l1.z + fmaf(Il0.z, A0, fmaf(Il1.x, A1, Il1.y * A2)), 0.0f));
+                }
+                if (mine && !(lh & 0x80000000u)) {
+                    Bh.set(make_float4(h0.x + mh * L0, h0.y + mh * L1, h0.z + mh * L2, h0.w));
+                    (Bh + 16u).set(make_float4(h1.x + fmaf(Ih0.x, H0, fmaf(Ih0.y, H1, Ih0.z * H2)),
+                                               h1.y + fmaf(Ih0.y, H0, fmaf(Ih0.w, H1, Ih1.x * H2)),
+                                               h1.z + fmaf(Ih0.z, H0, fmaf(Ih1.x, H1, Ih1.y * H2)), 0.0f));
+                }
+                if (mine) (rec + kX32).set(make_float4(xn, f1, f2, f3));
+                x = (rec_next + kX32).f4();
+                if (st0 & kStep32Ends) g.sync();
+                more = --left > 0 && !(st0 & kStep32Turns);
+                j = after(j);
+                st0 = st1;
+                st1 = step(after(j));
+                rec = rec_next;
+                lh = lh_next;
+            } while (more);
         }
-        g.sync();
-        start = end;
-        end = next_end;
     }
 }
 
-// The same Gauss-Seidel sweep with one lane per contact: the lane loads the contact's twelve row groups,
-// computes the four rows' J w as independent chains, applies the prox and updates both bodies.  A warp takes
-// 32 contacts of a level per pass instead of 8, and no shuffle lies on the chain.  Every expression is the
-// four-lane sweep's (the same operands, the same fmaf order), so both give the same bits.
-template <class G, bool kL2>
-__device__ __forceinline__ void s32_sweep_lane(const G& g, const S32Scene& f, int L, float rscale, bool bodies_global) {
-    int start = f.lptr[0], end = f.lptr[1];
-    for (int l = 1; l <= L; ++l) {
-        const int next_end = l < L ? f.lptr[l + 1] : end;
-        if (kL2) {   // rows in L2: pull the next level's rows (contiguous in level order) into L1 meanwhile
-            const char* p0 = reinterpret_cast<const char*>(f.c + kS32Floats * (size_t)end);
-            const int lines = (int)(((size_t)(next_end - end) * kS32Floats * sizeof(float) + 127) / 128);
-            for (int t = g.rank(); t < lines; t += g.size())
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(p0 + 128 * (size_t)t));
-            if (bodies_global)
-                for (int i = end + g.rank(); i < next_end; i += g.size()) {
-                    const uint32_t lh = f.lohi[i];
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(f.body + kS32BodyFloats * (size_t)(lh & 0xffffu)));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(f.body + kS32BodyFloats * (size_t)(lh >> 16)));
-                }
-        }
-        for (int i = start + g.rank(); i < end; i += g.size()) {
-            const float4* C4 = reinterpret_cast<const float4*>(f.c + kS32Floats * i);
-            const uint32_t lh = f.lohi[i];
-            float* Bl = f.body + kS32BodyFloats * (int)(lh & 0xffffu);
-            float* Bh = f.body + kS32BodyFloats * (int)(lh >> 16);
-            float4 R[12];
-            for (int k = 0; k < 12; ++k) R[k] = C4[k];
-            const float4 l0 = *reinterpret_cast<const float4*>(Bl), l1 = *reinterpret_cast<const float4*>(Bl + 4);
-            const float4 h0 = *reinterpret_cast<const float4*>(Bh), h1 = *reinterpret_cast<const float4*>(Bh + 4);
-            float z[4];
-            for (int q = 0; q < 4; ++q) {
-                const float4 r0 = R[3 * q], r1 = R[3 * q + 1], r2 = R[3 * q + 2];
-                float lin = fmaf(r0.x, l0.x - h0.x, fmaf(r0.y, l0.y - h0.y, r0.z * (l0.z - h0.z)));
-                if (q == 3) lin = 0.0f;
-                const float alo = fmaf(r1.x, l0.w, fmaf(r1.y, l1.x, r1.z * l1.y));
-                const float ahi = fmaf(r2.x, h0.w, fmaf(r2.y, h1.x, r2.z * h1.y));
-                z[q] = r2.w - rscale * r1.w * (((lin + alo) + ahi) + r0.w);
-            }
-            const float mu = R[9].x;
-            const float xn = fmaxf(z[0], 0.0f);
-            const float radius = mu * xn;
-            const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
-            float scale = sqr > radius * radius ? radius * rsqrtf(sqr) : 1.0f;
-            if (xn <= 0.0f) scale = 0.0f;
-            const float f1 = z[1] * scale, f2 = z[2] * scale, f3 = z[3] * scale;
-            const float d0 = xn - R[2].w, d1 = f1 - R[5].w, d2 = f2 - R[8].w, d3 = f3 - R[11].w;
-            f.c[kS32Floats * i + 11] = xn;
-            f.c[kS32Floats * i + 23] = f1;
-            f.c[kS32Floats * i + 35] = f2;
-            f.c[kS32Floats * i + 47] = f3;
-            // the three sums of the update (the torsion row has no linear columns)
-            const float L0 = fmaf(R[6].x, d2, fmaf(R[3].x, d1, R[0].x * d0));
-            const float L1 = fmaf(R[6].y, d2, fmaf(R[3].y, d1, R[0].y * d0));
-            const float L2 = fmaf(R[6].z, d2, fmaf(R[3].z, d1, R[0].z * d0));
-            const float A0 = fmaf(R[10].x, d3, fmaf(R[7].x, d2, fmaf(R[4].x, d1, R[1].x * d0)));
-            const float A1 = fmaf(R[10].y, d3, fmaf(R[7].y, d2, fmaf(R[4].y, d1, R[1].y * d0)));
-            const float A2 = fmaf(R[10].z, d3, fmaf(R[7].z, d2, fmaf(R[4].z, d1, R[1].z * d0)));
-            const float H0 = fmaf(R[11].x, d3, fmaf(R[8].x, d2, fmaf(R[5].x, d1, R[2].x * d0)));
-            const float H1 = fmaf(R[11].y, d3, fmaf(R[8].y, d2, fmaf(R[5].y, d1, R[2].y * d0)));
-            const float H2 = fmaf(R[11].z, d3, fmaf(R[8].z, d2, fmaf(R[5].z, d1, R[2].z * d0)));
-            // lo body: +m^-1 on the linear sums, I_lo^-1 on the angular ones; hi body: -m^-1 and I_hi^-1.
-            // Both are computed without a branch; only free bodies are written (a fixed body's is zero).
-            const float4 Il0 = *reinterpret_cast<const float4*>(Bl + 8);
-            const float2 Il1 = *reinterpret_cast<const float2*>(Bl + 12);
-            const float4 Ih0 = *reinterpret_cast<const float4*>(Bh + 8);
-            const float2 Ih1 = *reinterpret_cast<const float2*>(Bh + 12);
-            const float ml = l1.z, mh = -h1.z;
-            const float nl0 = l0.x + ml * L0, nl1 = l0.y + ml * L1, nl2 = l0.z + ml * L2;
-            const float nl3 = l0.w + fmaf(Il0.x, A0, fmaf(Il0.y, A1, Il0.z * A2));
-            const float nl4 = l1.x + fmaf(Il0.y, A0, fmaf(Il0.w, A1, Il1.x * A2));
-            const float nl5 = l1.y + fmaf(Il0.z, A0, fmaf(Il1.x, A1, Il1.y * A2));
-            const float nh0 = h0.x + mh * L0, nh1 = h0.y + mh * L1, nh2 = h0.z + mh * L2;
-            const float nh3 = h0.w + fmaf(Ih0.x, H0, fmaf(Ih0.y, H1, Ih0.z * H2));
-            const float nh4 = h1.x + fmaf(Ih0.y, H0, fmaf(Ih0.w, H1, Ih1.x * H2));
-            const float nh5 = h1.y + fmaf(Ih0.z, H0, fmaf(Ih1.x, H1, Ih1.y * H2));
-            if (l1.w == 0.0f) { Bl[0] = nl0; Bl[1] = nl1; Bl[2] = nl2; Bl[3] = nl3; Bl[4] = nl4; Bl[5] = nl5; }
-            if (h1.w == 0.0f) { Bh[0] = nh0; Bh[1] = nh1; Bh[2] = nh2; Bh[3] = nh3; Bh[4] = nh4; Bh[5] = nh5; }
+// n_sweeps sweeps by as many of the team's warps as the scene's levels keep busy
+template <class P, class G>
+__device__ __forceinline__ void s32_sweep_team(const G& g, const S32Scene& f, float rscale, int n_sweeps) {
+    if constexpr (std::is_same_v<G, BlockGroup>) {
+        if (f.warps == 1) {
+            if (threadIdx.x < 32) s32_sweep<P>(WarpGroup{}, f, rscale, n_sweeps);
+        } else if ((int)threadIdx.x < 32 * f.warps) {
+            s32_sweep<P>(SubGroup{32 * f.warps}, f, rscale, n_sweeps);
         }
         g.sync();
-        start = end;
-        end = next_end;
+    } else {
+        s32_sweep<P>(g, f, rscale, n_sweeps);
     }
 }
 
 // One proximal Jacobi sweep (proximal_contact/jacobi_solver.py:41-57) on the FP32 copy: every contact's new
-// impulse from the accumulators w = W J^T x of the previous iterate, four lanes per contact as in the
-// Gauss-Seidel sweep (any order: no contact reads another's new impulse), then w rebuilt from the new
-// impulses.  hybrid (jacobi_solver.py:60-79): the friction ball's radius uses the new normal impulse instead
-// of the previous one.
-template <class G>
-__device__ __forceinline__ void s32_sweep_jacobi(const G& g, const SceneRange& R, const S32Scene& f, float rscale,
-                                                 bool hybrid) {
-    const int K = R.c1 - R.c0;
-    const int q = g.rank() & 3, slot = g.rank() >> 2, nslot = g.size() >> 2;
-    const int base = (threadIdx.x & 31) & ~3;
-    const unsigned qm = 0xfu << base;
-    for (int i = slot; i < K; i += nslot) {   // the four lanes of a quad take the same contacts
-        const float4* C4 = reinterpret_cast<const float4*>(f.c + kS32Floats * i);
-        const uint32_t lh = f.lohi[i];
-        const float* Bl = f.body + kS32BodyFloats * (int)(lh & 0xffffu);
-        const float* Bh = f.body + kS32BodyFloats * (int)(lh >> 16);
-        const float4 r0 = C4[3 * q], r1 = C4[3 * q + 1], r2 = C4[3 * q + 2];   // own row
-        const float4 l0 = *reinterpret_cast<const float4*>(Bl), l1 = *reinterpret_cast<const float4*>(Bl + 4);
-        const float4 h0 = *reinterpret_cast<const float4*>(Bh), h1 = *reinterpret_cast<const float4*>(Bh + 4);
-        float lin = fmaf(r0.x, l0.x - h0.x, fmaf(r0.y, l0.y - h0.y, r0.z * (l0.z - h0.z)));
-        if (q == 3) lin = 0.0f;
-        const float alo = fmaf(r1.x, l0.w, fmaf(r1.y, l1.x, r1.z * l1.y));
-        const float ahi = fmaf(r2.x, h0.w, fmaf(r2.y, h1.x, r2.z * h1.y));
-        const float z = r2.w - rscale * r1.w * (((lin + alo) + ahi) + r0.w);
-        float zz[4];
-        for (int j = 0; j < 4; ++j) zz[j] = __shfl_sync(qm, z, base | j);
-        const float mu = __shfl_sync(qm, r0.x, base | 3);
-        const float xn_old = __shfl_sync(qm, r2.w, base);   // every read of the old impulses is done here
-        const float xn = fmaxf(zz[0], 0.0f);
-        float fr[3];
-        f32_prox(zz[1], zz[2], zz[3], mu, hybrid ? xn : xn_old, fr);
-        f.c[kS32Floats * i + 12 * q + 11] = q == 0 ? xn : fr[q - 1];
+// impulse from the accumulators w = W J^T x of the previous iterate, a quad per contact as in the Gauss-Seidel
+// sweep (any order: no contact reads another's new impulse), then w rebuilt from the new impulses.  hybrid
+// (jacobi_solver.py:60-79): the friction ball's radius uses the new normal impulse instead of the previous one.
+template <class P, class G>
+__device__ __noinline__ void s32_sweep_jacobi(const G g, const S32Scene f, float rscale, bool hybrid) {
+    const P c(f.c), body(f.body), lohi(f.lohi);
+    const int q = g.rank() & 3, nslot = g.size() >> 2;
+    for (int i0 = 0; i0 < f.K; i0 += nslot) {
+        const int at = i0 + (g.rank() >> 2), i = min(at, f.K - 1);
+        const uint32_t lh = (lohi + 4u * i).u32();
+        const P rec = c + kC32 * i, row = rec + 16u * q;
+        const P Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
+        const float4 r0 = row.f4(), r1 = (row + 64u).f4(), r2 = (row + 128u).f4();
+        const float4 l0 = Bl.f4(), l1 = (Bl + 16u).f4(), h0 = Bh.f4(), h1 = (Bh + 16u).f4();
+        const float x = (rec + kX32 + 4u * q).f1();
+        float z[4];
+        const float zq = x - rscale * r1.w * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
+        quad_gather(zq, z);
+        const float xn_old = __shfl_sync(0xffffffffu, x, (threadIdx.x & 31) & ~3);
+        const float xn = fmaxf(z[0], 0.0f), bound = hybrid ? xn : xn_old;
+        const float radius = r2.w * bound;
+        const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
+        const float fr = bound <= 0.0f ? 0.0f : (sqr <= radius * radius ? zq : zq * (radius * rsqrtf(sqr)));
+        if (at < f.K) (rec + kX32 + 4u * q).set(q == 0 ? xn : fr);
     }
     g.sync();
-    s32_rebuild_w(g, R, f);
+    s32_rebuild_w<P>(g, f);
 }
 
 // FP64 check of the FP32 iterate and defect correction of the FP32 problem.  With x the current FP32 iterate,
@@ -2608,61 +2728,67 @@ __device__ __forceinline__ void s32_sweep_jacobi(const G& g, const SceneRange& R
 // ||x - prox(x - D^-1 (A x + b))||_inf / max(1, ||x||_inf).  The FP32 sweeps that follow then converge to the
 // FP64 problem's solution: at the current x the corrected FP32 problem has the FP64 problem's residual.  The
 // FP32 w must hold W J^T x for this x (the residual test just before rebuilt it).
-template <class G>
+template <class P, class G>
 __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, const SceneRange& R, const S32Scene& f,
                                               bool correct = true) {
-    const int K = R.c1 - R.c0, nb = R.b1 - R.b0;
+    const P c(f.c), body(f.body), lohi(f.lohi), bptr(f.bptr), blist(f.blist);
+    const int K = f.K;
     const int* order = a.ws.lev_order + R.c0;
-    double* w64 = a.ws.w + 6 * (size_t)R.b0;   // the scene's FP64 accumulators, unused until the FP64 solve
-    for (int bl = g.rank(); bl < nb; bl += g.size()) {
-        double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        if (f.body[kS32BodyFloats * bl + 7] == 0.0f) {
-            for (int e = f.bptr[bl]; e < f.bptr[bl + 1]; ++e) {
-                const uint32_t code = f.blist[e];
-                const int i = (int)(code >> 1), side = (int)(code & 1);
-                const double* Wk = a.ws.WJT + 48 * (size_t)order[i];
-                for (int q = 0; q < 4; ++q) {
-                    const double xq = (double)f.c[kS32Floats * i + 12 * q + 11];
-                    for (int d = 0; d < 6; ++d) acc[d] = fma(Wk[w_at(q, 6 * side + d)], xq, acc[d]);
-                }
-            }
+    double* w64 = a.ws.w + 6 * (size_t)R.b0;   // by slot; the scene's FP64 accumulators, unused until the FP64 solve
+    for (int i = g.rank(); i < 6 * f.n_free; i += g.size()) {   // a thread per component
+        const int bl = i / 6, d = i - 6 * bl;
+        double acc = 0.0;
+        const uint32_t e1 = (bptr + (2u * bl + 2u)).u16();
+        for (uint32_t e = (bptr + 2u * bl).u16(); e < e1; ++e) {
+            const uint32_t code = (blist + 4u * e).u32();
+            double W[4];
+            w_column(a.ws.WJT, order[code >> 1], 6 * (int)(code & 1u) + d, W);
+            const float4 x = (c + kC32 * (code >> 1) + kX32).f4();
+            acc = fma(W[0], (double)x.x, acc);
+            acc = fma(W[1], (double)x.y, acc);
+            acc = fma(W[2], (double)x.z, acc);
+            acc = fma(W[3], (double)x.w, acc);
         }
-        for (int d = 0; d < 6; ++d) w64[6 * bl + d] = acc[d];
+        w64[i] = acc;
     }
+    if (f.n_free < s32_records(K, R.b1 - R.b0) && g.rank() < 6) w64[6 * f.n_free + g.rank()] = 0.0;
     g.sync();
     double m = 0.0, xm = 0.0;
-    for (int i = g.rank(); i < K; i += g.size()) {
+    const int q = g.rank() & 3, nslot = g.size() >> 2;
+    for (int i0 = 0; i0 < K; i0 += nslot) {   // a quad per contact
+        const int at = i0 + (g.rank() >> 2), i = min(at, K - 1);
         const size_t k = (size_t)order[i];
-        const uint32_t lh = f.lohi[i];
-        const int lo = (int)(lh & 0xffffu), hi = (int)(lh >> 16);
-        const double* wl = w64 + 6 * lo;
-        const double* wh = w64 + 6 * hi;
-        const float* wl32 = f.body + kS32BodyFloats * lo;
-        const float* wh32 = f.body + kS32BodyFloats * hi;
-        double z[4], x[4];
-        for (int q = 0; q < 4; ++q) {
-            const double* J = a.ws.J + 48 * k;
-            double v64 = a.ws.b[4 * k + q];
+        const uint32_t lh = (lohi + 4u * i).u32();
+        const double* wl = w64 + 6 * (lh & 0x7fffu);
+        const double* wh = w64 + 6 * ((lh >> 16) & 0x7fffu);
+        const double2* J = reinterpret_cast<const double2*>(a.ws.J + 48 * k + 2 * q);
+        double v64 = a.ws.b[4 * k + q];
 #pragma unroll
-            for (int c = 0; c < 6; ++c) v64 = fma(J[j_at(q, c)], wl[c], v64);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) v64 = fma(J[j_at(q, 6 + c)], wh[c], v64);
-            float* row = f.c + kS32Floats * i + 12 * q;
-            if (correct) {
-                const float v32 = s32_jw(row, q, wl32, wh32) + row[3];
-                row[3] += (float)(v64 - (double)v32);
-            }
-            x[q] = (double)row[11];
-            z[q] = x[q] - v64 / a.ws.diag[4 * k + q];
+        for (int t = 0; t < 6; ++t) {
+            const double2 j2 = J[4 * t];
+            const double* w = t < 3 ? wl + 2 * t : wh + 2 * t - 6;
+            v64 = fma(j2.x, w[0], v64);
+            v64 = fma(j2.y, w[1], v64);
         }
+        const P rec = c + kC32 * i, row = rec + 16u * q;
+        if (correct && at < K) {
+            const P Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
+            const float4 r0 = row.f4();
+            const float v32 = s32_jw(r0, (row + 64u).f4(), (row + 128u).f4(), Bl.f4(), (Bl + 16u).f4(), Bh.f4(), (Bh + 16u).f4()) + r0.w;
+            (row + 12u).set(r0.w + (float)(v64 - (double)v32));
+        }
+        const double x = (double)(rec + kX32 + 4u * q).f1();
+        const double zq = x - v64 / a.ws.diag[4 * k + q];
+        double z[4];
+        quad_gather(zq, z);
         const double pn = z[0] > 0.0 ? z[0] : 0.0;
-        double fr[3];
-        prox_sphere(z[1], z[2], z[3], a.ws.mu[k], pn, fr);
-        const double d[4] = {x[0] - pn, x[1] - fr[0], x[2] - fr[1], x[3] - fr[2]};
-        for (int t = 0; t < 4; ++t) {
-            m = fmax(m, fabs(d[t]));
-            if (d[t] != d[t]) m = d[t];
-            xm = fmax(xm, fabs(x[t]));
+        double scale;
+        const int kind = prox_factor(z, a.ws.mu[k], pn, scale);
+        const double d = x - (q == 0 ? pn : prox_apply(kind, scale, zq));
+        if (at < K) {
+            m = fmax(m, fabs(d));
+            if (d != d) m = d;
+            xm = fmax(xm, fabs(x));
         }
     }
     const double mres = g.max(m);
@@ -2675,7 +2801,8 @@ __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, con
 // large slab, 3 block teams with the contact rows in L2; -1 for a scene the FP32 phase leaves to FP64
 __host__ __device__ inline int s32_class(int K, int nb, size_t small_slab, size_t mid_slab) {
     if (K == 0 || K > 32767 || nb > 32767) return -1;   // 16-bit positions and list offsets
-    const size_t bytes = s32_bytes(K, nb);
+    const int nr = s32_records(K, nb);
+    const size_t bytes = s32_bytes(K, nr);
     if (bytes <= small_slab) return 0;
     if (bytes <= mid_slab) return 1;
     if (bytes <= (size_t)kFp32LargeSmem) return 2;
@@ -2767,6 +2894,7 @@ __global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve
     __shared__ int next_slot;
     if (a.ws.counters[kAbort]) return;
     G g;
+    using P = std::conditional_t<kL2, GlPtr, ShPtr>;
     constexpr bool block_team = std::is_same_v<G, BlockGroup>;
     if constexpr (block_team) { g.red = red; g.ired = ired; }
     const int team = block_team ? 0 : (int)(threadIdx.x >> 5);
@@ -2796,28 +2924,29 @@ __global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve
         const SceneRange R = scene_range(a, s);
         const int K = R.c1 - R.c0, nb = R.b1 - R.b0;
         if (K == 0 || K > 32767 || nb > 32767) continue;   // 16-bit positions and list offsets
+        const int nr = s32_records(K, nb);
         bool bodies_global = false;
         if (kL2) {   // the scenes no slab holds whole: contact rows in L2, and the bodies too if they do not fit
-            if (s32_bytes(K, nb) <= lo_bytes) continue;
-            bodies_global = s32_bytes(K, nb, true) > slab;
-            if (s32_bytes(K, nb, true, bodies_global) > slab) continue;
+            if (s32_bytes(K, nr) <= lo_bytes) continue;
+            bodies_global = s32_bytes(K, nr, true) > slab;
+            if (s32_bytes(K, nr, true, bodies_global) > slab) continue;
         } else {
-            const size_t bytes = s32_bytes(K, nb);
+            const size_t bytes = s32_bytes(K, nr);
             if (bytes <= lo_bytes || bytes > slab) continue;
         }
         const double t0 = a.pr.profiling ? device_us() : 0.0;
-        const S32Scene f = s32_carve(my_slab, K, nb, kL2 ? &a : nullptr, R.c0, bodies_global, R.b0);
+        S32Scene f = s32_carve(my_slab, K, nr, kL2 ? &a : nullptr, R.c0, s, bodies_global, R.b0);
         // scratch for the level relaxation: the rows' room of the slab, or with rows in L2 what the slab has left
         int16_t* scratch = nullptr;
         if (!kL2) {   // a contact record's bytes per contact there, more than s32_level_scratch needs
             scratch = reinterpret_cast<int16_t*>(f.c);
         } else {
-            const size_t off = (s32_bytes(K, nb, true, bodies_global) + 15) & ~size_t(15);
+            const size_t off = (s32_bytes(K, nr, true, bodies_global) + 15) & ~size_t(15);
             if (off + s32_level_scratch(K) <= slab) scratch = reinterpret_cast<int16_t*>(my_slab + off);
         }
-        const int L = s32_load(a, g, R, s, f, coloured, scratch);
+        const int L = s32_load(a, g, R, s, f, coloured, kL2, scratch);
         if (g.rank() == 0) a.ws.nlev[s] = L;
-        float res = s32_residual(a, g, R, f);   // the warm-started iterate may already be good enough
+        float res = s32_residual<P>(g, f);   // the warm-started iterate may already be good enough
         float best = res;
         int sweeps = 0, stalls = 0, window = kS32StallTests;
         // far above the tolerance (and the stall floor) the residual is tested half as often: no stop and no
@@ -2829,22 +2958,13 @@ __global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve
         for (;;) {
             const int round_start = sweeps;
             while (res > tol && sweeps < budget) {
-                if (jacobi) {
-                    s32_sweep_jacobi(g, R, f, rscale, hybrid);
-                } else if (!block_team) {
-                    s32_sweep_lane<G, kL2>(g, f, L, rscale, bodies_global);
-                } else if (!kL2) {
-                    // a block team's slab scene: its levels rarely hold more contacts than a warp has lanes,
-                    // so warp 0 sweeps it one lane per contact (the same bits as four lanes per contact) with
-                    // warp barriers between levels, and the block meets once per sweep
-                    if (threadIdx.x < 32) s32_sweep_lane<WarpGroup, false>(WarpGroup{}, f, L, rscale, false);
-                    g.sync();
-                } else {
-                    s32_sweep<G, kL2>(g, f, L, rscale, bodies_global);
-                }
-                ++sweeps;
-                if (--next_test == 0 || sweeps == budget) {
-                    res = s32_residual(a, g, R, f);
+                const int n = jacobi ? 1 : min(next_test, budget - sweeps);   // as far as the next test
+                if (jacobi) s32_sweep_jacobi<P>(g, f, rscale, hybrid);
+                else s32_sweep_team<P>(g, f, rscale, n);
+                sweeps += n;
+                next_test -= n;
+                if (next_test == 0 || sweeps == budget) {
+                    res = s32_residual<P>(g, f);
                     next_test = gap(res);
                     // a round ends once the residual, already small, stops improving for a while (the FP32
                     // problem's own rounding, or slow progress a defect correction may speed up).  Above the
@@ -2857,13 +2977,13 @@ __global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve
             // problem's b by the FP64 defect and sweep on in FP32.  FP64 sweeps take over only when the FP32
             // problem meets the tolerance and the FP64 one does not (the FP32 sweeps can do no more).
             if (a.pr.precision != RB_PRECISION_FP32_REFINE || sweeps >= budget) break;
-            r64 = s32_correct(a, g, R, f);
+            r64 = s32_correct<P>(a, g, R, f);
             if (r64 <= a.pr.residual_tolerance) break;
             if (sweeps == round_start) break;   // r64 stays valid for x
             if (r64 > kS32RoundGain * r64_round) window = min(2 * window, kS32StallTestsMax);
             r64_round = fmin(r64_round, r64);
             r64 = -1.0;   // the sweeps that follow change the iterate
-            res = s32_residual(a, g, R, f);
+            res = s32_residual<P>(g, f);
             next_test = gap(res);
             best = res;
             stalls = 0;
@@ -2871,13 +2991,13 @@ __global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve
         // the FP64 residual of the iterate decides whether FP64 sweeps follow; when none do, this kernel
         // finishes the scene (solution, statistics), and when some do, this team runs them right away, so
         // the FP64 solver launched after the FP32 phase skips the scene either way
-        if (r64 < 0.0) r64 = s32_correct(a, g, R, f, false);
+        if (r64 < 0.0) r64 = s32_correct<P>(a, g, R, f, false);
         const bool finished = r64 <= a.pr.residual_tolerance || sweeps >= max_it ||
                               a.pr.precision == RB_PRECISION_FP32;
         for (int t = g.rank(); t < 4 * K; t += g.size()) {   // back to contact order
             const int i = t >> 2, q = t & 3;
             const size_t k4 = 4 * (size_t)a.ws.lev_order[R.c0 + i] + q;
-            const double xv = (double)f.c[kS32Floats * i + 12 * q + 11];
+            const double xv = (double)(P(f.c) + (kC32 * i + kX32 + 4u * q)).f1();
             a.ws.x[k4] = xv;
             if (finished) a.out.contact_sol[k4] = xv;
         }
