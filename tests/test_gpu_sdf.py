@@ -106,3 +106,54 @@ def test_per_body_scenes_do_not_depend_on_which_others_are_built():
             va = a[k].cpu().numpy() if hasattr(a[k], "cpu") else np.asarray(a[k])
             vb = b[k].cpu().numpy() if hasattr(b[k], "cpu") else np.asarray(b[k])
             np.testing.assert_array_equal(va, vb, err_msg=k)
+
+
+def _plain_grid(V, T, meta):
+    """Distance to the nearest triangle and the winding number of every node, summed arc by arc, in NumPy."""
+    I, J, K = (int(v) for v in meta[9:12])
+    k, j, i = np.meshgrid(np.arange(K), np.arange(J), np.arange(I), indexing="ij")
+    P = np.stack([meta[a] + meta[6 + a] * n.ravel() for a, n in zip(range(3), (i, j, k))], axis=1)
+    dist, wind = np.full(len(P), np.inf), np.zeros(len(P))
+    for tri in V[T]:
+        away = [P - c for c in tri]
+        n = np.cross(tri[1] - tri[0], tri[2] - tri[0])
+        n /= np.linalg.norm(n)
+        inside = np.ones(len(P), bool)
+        for c in range(3):
+            e = tri[(c + 1) % 3] - tri[c]
+            t = np.clip(away[c] @ e / (e @ e), 0.0, 1.0)
+            dist = np.minimum(dist, np.linalg.norm(away[c] - t[:, None] * e, axis=1))
+            inside &= np.cross(e, away[c]) @ n >= 0.0
+        dist = np.where(inside, np.minimum(dist, np.abs(away[0] @ n)), dist)
+        A, B, C = (-a for a in away)
+        la, lb, lc = (np.linalg.norm(a, axis=1) for a in away)
+        dots = [(x * y).sum(1) for x, y in ((A, B), (B, C), (C, A))]
+        wind += 2.0 * np.arctan2((A * np.cross(B, C)).sum(1), la * lb * lc + dots[0] * lc + dots[1] * la + dots[2] * lb)
+    return dist, np.abs(wind) / (4.0 * np.pi)
+
+
+@pytest.mark.parametrize("mesh,triangles,margin,res", [
+    ("box", 12, 0.0, (9, 9, 9)),        # nodes on the corners, edges and faces
+    ("box", 12, 0.125, (11, 11, 11)),
+    ("box", 10, 0.25, (13, 7, 5)),      # an open box
+    ("sphere", 127, 0.1, (7, 32, 3)), ("sphere", 128, 0.1, (33, 4, 4)), ("sphere", 129, 0.1, (5, 5, 31)),
+    ("sphere", 448, 0.3, (32, 8, 2)),
+    ("nested", 24, 0.2, (17, 17, 17)),  # one box inside another: winding numbers 0, 1 and 2
+])
+def test_grid_signs_and_distances(mesh, triangles, margin, res):
+    """Node for node against the plain evaluation: distances to 1e-12, signs wherever the winding number is not
+    within rounding of its threshold; parts of meshes, nodes on the surface and sizes at the edges of the tiles."""
+    from rainbow_b200 import geometry as GEO
+    from rainbow_b200.types import Grid
+    V, T = GEO.create_box(1.0, 1.0, 1.0) if mesh != "sphere" else GEO.create_sphere(0.5, 16, 16)
+    V, T = np.asarray(V, np.float64), np.asarray(T, np.int32)
+    if mesh == "nested":
+        V, T = np.concatenate([V, 0.5 * V]), np.concatenate([T, T + len(V)])
+    T = T[:triangles]
+    meta = Grid(V.min(0) - margin, V.max(0) + margin, *res).meta()
+    got = _grid_on_gpu(V, T, meta)
+    dist, wind = _plain_grid(V, T, meta)
+    np.testing.assert_allclose(np.abs(got), dist, rtol=0.0, atol=1e-12)
+    clear = (np.abs(wind - 0.5) > 1e-9) & (dist > 1e-12)
+    assert clear.any()
+    np.testing.assert_array_equal((got < 0.0)[clear], (wind > 0.5)[clear])
