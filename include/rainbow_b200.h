@@ -79,11 +79,12 @@ typedef struct rb_shapes {
     const int64_t* g_off;       /* n_shapes+1 value offsets */
     const double* grid_meta;    /* 12 doubles per shape: min[3], max[3], spacing[3], I, J, K (grid3.py:16) */
     int32_t max_shape_triangles; /* triangles of the largest shape (at most 16384) */
-    const float* grid32;        /* optional FP32 copy of grid (same offsets), or NULL.  With it, the FP32
-                                   precision modes run the contact search's signed distance lookups (the seed
-                                   and Frank-Wolfe iterations, collision_detection.py:134-165) in FP32; the
-                                   acceptance tests and the contact's point, normal and gap (:172-188) stay
-                                   FP64, evaluated at the point the FP32 search found */
+    const float* grid32;        /* optional FP32 copy of grid (same offsets), or NULL.  With it, a profiled step
+                                   of the FP32 precision modes runs the contact search's signed distance lookups
+                                   (the seed and Frank-Wolfe iterations, collision_detection.py:134-165) in FP32
+                                   and counts them; near-ties, the acceptance tests and the contact's point,
+                                   normal and gap (:172-188) stay FP64, so it finds the contacts that the other
+                                   steps' FP64 search finds */
 } rb_shapes;
 
 /* Bodies of one or more independent scenes; scene s owns bodies scene_start[s] .. scene_start[s+1]-1 in the

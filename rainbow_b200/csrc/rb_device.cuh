@@ -153,22 +153,41 @@ __device__ __forceinline__ double ratio_sqrt(double a, double v) {
 // ---------------------------------------------------------------------------------------------------------
 // Signed distance grid (grid3.py)
 // ---------------------------------------------------------------------------------------------------------
+// A grid as one candidate's lookups read it.  The quotients by the spacing and by the minimum corner are taken with
+// their reciprocals, which a candidate computes once: a lookup's nine FP64 divisions (112 cycles of latency and ~20
+// FP64 instructions each) were what the contact search spent its time on.
 struct GridView {
     const double* values;
-    double mn[3], mx[3], sp[3];
+    const double* meta;            // min[3], max[3], spacing[3], I, J, K
+    double mn[3], sp[3];
+    double inv_mn[3], inv_sp[3];   // rounded reciprocals
     int I, J, K;
 };
 __device__ __forceinline__ GridView load_grid(const double* meta, const double* values) {
     GridView g;
     g.values = values;
+    g.meta = meta;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) { g.mn[a] = meta[a]; g.mx[a] = meta[3 + a]; g.sp[a] = meta[6 + a]; }
+    for (int a = 0; a < 3; ++a) {
+        g.mn[a] = meta[a]; g.sp[a] = meta[6 + a];
+        g.inv_mn[a] = 1.0 / g.mn[a]; g.inv_sp[a] = 1.0 / g.sp[a];
+    }
     g.I = (int)meta[9]; g.J = (int)meta[10]; g.K = (int)meta[11];
     return g;
 }
-// grid3.py:107 get_enclosing_cell_idx (floor, then clip to [0, n-2])
-__device__ __forceinline__ int cell_index(double p, double mn, double sp, int n) {
-    const double f = floor((p - mn) / sp);
+// n / d from d's rounded reciprocal: the product corrected by its exact residual, which rounds as the division does
+// (Markstein, IBM J. Res. Dev. 34, 1990).  A quotient outside 1e+-250, zero and NaN among them, is divided.
+__device__ __forceinline__ double quotient(double n, double d, double inv) {
+    const double q = n * inv;
+    const double c = fma(fma(-q, d, n), inv, q);
+    return fabs(c) > 1e-250 && fabs(c) < 1e250 ? c : n / d;
+}
+// grid3.py:107 get_enclosing_cell_idx (floor, then clip to [0, n-2]); a quotient that the reciprocal leaves within
+// 1e-7 of a whole number is divided
+__device__ __forceinline__ int cell_index(double p, double mn, double sp, double inv_sp, int n) {
+    double q = (p - mn) * inv_sp;
+    double f = floor(q);
+    if (fabs(q - f - 0.5) > 0.5 - 1e-7 || !(fabs(q) < 1e8)) f = floor((p - mn) / sp);
     const int lim = n - 2;
     if (!(f >= 0.0)) return 0;
     if (f > (double)lim) return lim;
@@ -177,9 +196,9 @@ __device__ __forceinline__ int cell_index(double p, double mn, double sp, int n)
 struct Corners { double d000, d001, d010, d011, d100, d101, d110, d111; int i, j, k; };
 __device__ __forceinline__ Corners load_corners(const GridView& g, d3 p) {
     Corners c;
-    c.i = cell_index(p.x, g.mn[0], g.sp[0], g.I);
-    c.j = cell_index(p.y, g.mn[1], g.sp[1], g.J);
-    c.k = cell_index(p.z, g.mn[2], g.sp[2], g.K);
+    c.i = cell_index(p.x, g.mn[0], g.sp[0], g.inv_sp[0], g.I);
+    c.j = cell_index(p.y, g.mn[1], g.sp[1], g.inv_sp[1], g.J);
+    c.k = cell_index(p.z, g.mn[2], g.sp[2], g.inv_sp[2], g.K);
     const int64_t I = g.I, IJ = (int64_t)g.I * g.J;
     const double* v = g.values + c.i + I * c.j + IJ * c.k;
     c.d000 = __ldg(v);
@@ -195,9 +214,9 @@ __device__ __forceinline__ Corners load_corners(const GridView& g, d3 p) {
 // grid3.py:126 get_value
 __device__ __forceinline__ double grid_value(const GridView& g, d3 p) {
     const Corners c = load_corners(g, p);
-    const double s = (p.x - (((double)c.i * g.sp[0]) + g.mn[0])) / g.sp[0];
-    const double t = (p.y - (((double)c.j * g.sp[1]) + g.mn[1])) / g.sp[1];
-    const double u = (p.z - (((double)c.k * g.sp[2]) + g.mn[2])) / g.sp[2];
+    const double s = quotient(p.x - (((double)c.i * g.sp[0]) + g.mn[0]), g.sp[0], g.inv_sp[0]);
+    const double t = quotient(p.y - (((double)c.j * g.sp[1]) + g.mn[1]), g.sp[1], g.inv_sp[1]);
+    const double u = quotient(p.z - (((double)c.k * g.sp[2]) + g.mn[2]), g.sp[2], g.inv_sp[2]);
     const double x00 = (c.d100 - c.d000) * s + c.d000;
     const double x01 = (c.d101 - c.d001) * s + c.d001;
     const double x10 = (c.d110 - c.d010) * s + c.d010;
@@ -209,9 +228,9 @@ __device__ __forceinline__ double grid_value(const GridView& g, d3 p) {
 // grid3.py:180 get_gradient, including the reference's division of s, t, u by min_coord (:209-211)
 __device__ __forceinline__ d3 grid_gradient(const GridView& g, d3 p) {
     const Corners c = load_corners(g, p);
-    const double s = (p.x - ((double)c.i * g.sp[0] + g.mn[0])) / g.mn[0];
-    const double t = (p.y - ((double)c.j * g.sp[1] + g.mn[1])) / g.mn[1];
-    const double u = (p.z - ((double)c.k * g.sp[2] + g.mn[2])) / g.mn[2];
+    const double s = quotient(p.x - ((double)c.i * g.sp[0] + g.mn[0]), g.mn[0], g.inv_mn[0]);
+    const double t = quotient(p.y - ((double)c.j * g.sp[1] + g.mn[1]), g.mn[1], g.inv_mn[1]);
+    const double u = quotient(p.z - ((double)c.k * g.sp[2] + g.mn[2]), g.mn[2], g.inv_mn[2]);
     const double x00 = (c.d100 - c.d000) * s + c.d000;
     const double x01 = (c.d101 - c.d001) * s + c.d001;
     const double x10 = (c.d110 - c.d010) * s + c.d010;
@@ -226,13 +245,13 @@ __device__ __forceinline__ d3 grid_gradient(const GridView& g, d3 p) {
     const double dp_ds = (dy1_ds - dy0_ds) * u + dy0_ds;
     const double dp_dt = (dy1_dt - dy0_dt) * u + dy0_dt;
     const double dp_du = y1 - y0;
-    return d3{dp_ds * (1.0 / g.sp[0]), dp_dt * (1.0 / g.sp[1]), dp_du * (1.0 / g.sp[2])};
+    return d3{dp_ds * g.inv_sp[0], dp_dt * g.inv_sp[1], dp_du * g.inv_sp[2]};
 }
 // grid3.py:275 is_inside
 __device__ __forceinline__ bool grid_is_inside(const GridView& g, d3 p, double boundary) {
-    if (p.x > (g.mx[0] - boundary)) return false;
-    if (p.y > (g.mx[1] - boundary)) return false;
-    if (p.z > (g.mx[2] - boundary)) return false;
+    if (p.x > (g.meta[3] - boundary)) return false;
+    if (p.y > (g.meta[4] - boundary)) return false;
+    if (p.z > (g.meta[5] - boundary)) return false;
     if (p.x < (g.mn[0] + boundary)) return false;
     if (p.y < (g.mn[1] + boundary)) return false;
     if (p.z < (g.mn[2] + boundary)) return false;
@@ -240,22 +259,22 @@ __device__ __forceinline__ bool grid_is_inside(const GridView& g, d3 p, double b
 }
 
 // Gradient from the FP32 copy of a grid (the contact search of the FP32 precision modes): the cell and the
-// fractions s, t, u in FP64 exactly as grid_gradient computes them (so the cell is always the FP64 lookup's,
-// grid3.py:107, and the min_coord divisor of :209-211 is kept), the eight corner values and their trilinear
+// fractions s, t, u in FP64 (the cell is always the FP64 lookup's, grid3.py:107, and the min_coord divisor of
+// :209-211 is kept; the fractions take its reciprocal, 2^-52 off, far inside the bound), the eight corner values and their trilinear
 // combination in FP32.  err bounds the absolute difference of each component from grid_gradient's: the FP32
 // rounding of the values (at most 2^-24 |v|) and of the combination, amplified by the weights (1 - s, s) ...,
 // which the min_coord divisor can take outside [0, 1].
 __device__ __forceinline__ d3 grid_gradient_f32(const GridView& g, const float* values32, d3 p, double& err) {
-    const int i = cell_index(p.x, g.mn[0], g.sp[0], g.I);
-    const int j = cell_index(p.y, g.mn[1], g.sp[1], g.J);
-    const int k = cell_index(p.z, g.mn[2], g.sp[2], g.K);
+    const int i = cell_index(p.x, g.mn[0], g.sp[0], g.inv_sp[0], g.I);
+    const int j = cell_index(p.y, g.mn[1], g.sp[1], g.inv_sp[1], g.J);
+    const int k = cell_index(p.z, g.mn[2], g.sp[2], g.inv_sp[2], g.K);
     const int64_t I = g.I, IJ = (int64_t)g.I * g.J;
     const float* v = values32 + i + I * j + IJ * k;
     const float d000 = __ldg(v), d100 = __ldg(v + 1), d010 = __ldg(v + I), d110 = __ldg(v + I + 1);
     const float d001 = __ldg(v + IJ), d101 = __ldg(v + IJ + 1), d011 = __ldg(v + IJ + I), d111 = __ldg(v + IJ + I + 1);
-    const double sd = (p.x - ((double)i * g.sp[0] + g.mn[0])) / g.mn[0];
-    const double td = (p.y - ((double)j * g.sp[1] + g.mn[1])) / g.mn[1];
-    const double ud = (p.z - ((double)k * g.sp[2] + g.mn[2])) / g.mn[2];
+    const double sd = (p.x - ((double)i * g.sp[0] + g.mn[0])) * g.inv_mn[0];
+    const double td = (p.y - ((double)j * g.sp[1] + g.mn[1])) * g.inv_mn[1];
+    const double ud = (p.z - ((double)k * g.sp[2] + g.mn[2])) * g.inv_mn[2];
     const float s = (float)sd, t = (float)td, u = (float)ud;
     const float x00 = (d100 - d000) * s + d000, x01 = (d101 - d001) * s + d001;
     const float x10 = (d110 - d010) * s + d010, x11 = (d111 - d011) * s + d011;
@@ -269,9 +288,9 @@ __device__ __forceinline__ d3 grid_gradient_f32(const GridView& g, const float* 
     float vmax = fmaxf(fmaxf(fmaxf(fabsf(d000), fabsf(d100)), fmaxf(fabsf(d010), fabsf(d110))),
                        fmaxf(fmaxf(fabsf(d001), fabsf(d101)), fmaxf(fabsf(d011), fabsf(d111))));
     const double amp = (1.0 + 2.0 * fabs(sd)) * (1.0 + 2.0 * fabs(td)) * (1.0 + 2.0 * fabs(ud));
-    const double sp_min = fmin(g.sp[0], fmin(g.sp[1], g.sp[2]));
-    err = 64.0 * 5.9604644775390625e-8 * (double)vmax * amp / sp_min;   // 64 x 2^-24 x ...
-    return d3{(double)dp_ds * (1.0 / g.sp[0]), (double)dp_dt * (1.0 / g.sp[1]), (double)dp_du * (1.0 / g.sp[2])};
+    const double inv_sp = fmax(g.inv_sp[0], fmax(g.inv_sp[1], g.inv_sp[2]));
+    err = 64.0 * 5.9604644775390625e-8 * (double)vmax * amp * inv_sp;   // 64 x 2^-24 x ...
+    return d3{(double)dp_ds * g.inv_sp[0], (double)dp_dt * g.inv_sp[1], (double)dp_du * g.inv_sp[2]};
 }
 
 // NumPy np.add.reduceat over one segment: a[0] + pairwise_sum(a[1:]) (8 interleaved partial sums once the

@@ -503,11 +503,12 @@ __global__ void __launch_bounds__(kBlock) k_mid(const StepArgs a, int max_cluste
 // ---------------------------------------------------------------------------------------------------------
 // narrow phase (collision_detection.py:87 _compute_contacts): one thread per candidate triangle
 // ---------------------------------------------------------------------------------------------------------
+constexpr int kAlphas = 32;   // step lengths 2 / (i + 2) of the search, kept in shared memory
 // seed and Frank-Wolfe search on one triangle (ps: its corners in the SDF owner's frame) in FP64
 // (collision_detection.py:134-165).  Returns the point; n_fw = iterations, trace = the seed (bits 0-1) and
 // each iteration's vertex (2 bits each from bit 2)
-__device__ __forceinline__ d3 fw_search64(const GridView& g, const d3* ps, int max_it, double tol, int& n_fw,
-                                          uint32_t& trace) {
+__device__ __forceinline__ d3 fw_search64(const GridView& g, const double* alphas, const d3* ps, int max_it,
+                                          double tol, int& n_fw, uint32_t& trace) {
     // seed: corner with the smallest gradient norm (:136-140); norm(list, axis=1) sums squares unfused
     double gn[3];
     for (int c = 0; c < 3; ++c) {
@@ -530,7 +531,7 @@ __device__ __forceinline__ d3 fw_search64(const GridView& g, const d3* ps, int m
         if (o1 < ov) { v = 1; ov = o1; }
         if (o2 < ov) { v = 2; ov = o2; }
         if (i < 15) trace |= (uint32_t)v << (2 + 2 * i);
-        const double alpha = 2.0 / (double)(i + 2);
+        const double alpha = i < kAlphas ? alphas[i] : 2.0 / (double)(i + 2);
         const d3 s = v == 0 ? ps[0] : (v == 1 ? ps[1] : ps[2]);
         x = d3{x.x + alpha * (s.x - x.x), x.y + alpha * (s.y - x.y), x.z + alpha * (s.z - x.z)};
         if (ov > tol) break;
@@ -542,8 +543,8 @@ __device__ __forceinline__ d3 fw_search64(const GridView& g, const d3* ps, int m
 // the objectives stay FP64; a decision whose margin lies within the FP32 lookups' error bound (an exact tie of
 // coplanar corners, a near-tie, an objective next to the tolerance) is taken again on FP64 lookups, so every
 // decision, and x, equal fw_search64's.  l64 / l32 count the FP64 and FP32 lookups made.
-__device__ __forceinline__ d3 fw_search_f32(const GridView& g, const float* values32, const d3* ps, int max_it,
-                                            double tol, int& n_fw, uint32_t& trace, int& l64, int& l32) {
+__device__ __forceinline__ d3 fw_search_f32(const GridView& g, const float* values32, const double* alphas,
+                                            const d3* ps, int max_it, double tol, int& n_fw, uint32_t& trace, int& l64, int& l32) {
     double scale = 0.0;   // max over corners of |p|_1: an objective's error is at most err x scale
     for (int c = 0; c < 3; ++c) scale = fmax(scale, fabs(ps[c].x) + fabs(ps[c].y) + fabs(ps[c].z));
     double gn[3], err = 0.0;
@@ -591,7 +592,7 @@ __device__ __forceinline__ d3 fw_search_f32(const GridView& g, const float* valu
         if (o1 < ov) { v = 1; ov = o1; }
         if (o2 < ov) { v = 2; ov = o2; }
         if (i < 15) trace |= (uint32_t)v << (2 + 2 * i);
-        const double alpha = 2.0 / (double)(i + 2);
+        const double alpha = i < kAlphas ? alphas[i] : 2.0 / (double)(i + 2);
         const d3 s = v == 0 ? ps[0] : (v == 1 ? ps[1] : ps[2]);
         x = d3{x.x + alpha * (s.x - x.x), x.y + alpha * (s.y - x.y), x.z + alpha * (s.z - x.z)};
         if (ov > tol) break;
@@ -601,9 +602,9 @@ __device__ __forceinline__ d3 fw_search_f32(const GridView& g, const float* valu
 
 // the plain FP64 search's trace and acceptance for a profiled step's check of the FP32 search (a call of its
 // own, so that it does not raise the registers of the search itself)
-__device__ __noinline__ void fw_check64(const GridView& g, const d3* ps, const double* qB, int max_it, double tol,
+__device__ __noinline__ void fw_check64(const GridView& g, const double* alphas, const d3* ps, const double* qB, int max_it, double tol,
                                         double envelope, int& n64, uint32_t& trace64, int& accept64) {
-    const d3 x64 = fw_search64(g, ps, max_it, tol, n64, trace64);
+    const d3 x64 = fw_search64(g, alphas, ps, max_it, tol, n64, trace64);
     accept64 = 0;
     if (grid_is_inside(g, x64, 0.5) && grid_value(g, x64) <= envelope)
         accept64 = norm3_np(quat_rotate(qB, grid_gradient(g, x64))) > 0.0;
@@ -615,6 +616,9 @@ __device__ __noinline__ void fw_check64(const GridView& g, const d3* ps, const d
 // whose search decisions or acceptance differ (a check of the error bound: zero when it holds).
 template <bool kF32>
 __global__ void __launch_bounds__(256, 2) k_narrow(const StepArgs a) {
+    __shared__ double alphas[kAlphas];
+    if (threadIdx.x < kAlphas) alphas[threadIdx.x] = 2.0 / (double)((int)threadIdx.x + 2);
+    __syncthreads();
     if (a.ws.counters[kAbort]) return;
     const int n_items = a.ws.counters[kNItems];
     const int max_it = a.pr.contact_optimization_max_iterations;
@@ -643,9 +647,9 @@ __global__ void __launch_bounds__(256, 2) k_narrow(const StepArgs a) {
         uint32_t trace = 0u;
         d3 x;
         if (kF32) {
-            x = fw_search_f32(g, a.sh.grid32 + a.sh.g_off[ss], ps, max_it, tol, n_fw, trace, lookups, lookups32);
+            x = fw_search_f32(g, a.sh.grid32 + a.sh.g_off[ss], alphas, ps, max_it, tol, n_fw, trace, lookups, lookups32);
         } else {
-            x = fw_search64(g, ps, max_it, tol, n_fw, trace);
+            x = fw_search64(g, alphas, ps, max_it, tol, n_fw, trace);
             lookups = 3 + n_fw;   // seed gradients + one gradient per Frank-Wolfe iteration
         }
         int flag = 0;
@@ -676,7 +680,7 @@ __global__ void __launch_bounds__(256, 2) k_narrow(const StepArgs a) {
             if (kF32 && (a.pr.profiling & 2)) {   // the check against the plain FP64 search, on request
                 int n64 = 0, accept64 = 0;
                 uint32_t trace64 = 0u;
-                fw_check64(g, ps, qB, max_it, tol, envelope, n64, trace64, accept64);
+                fw_check64(g, alphas, ps, qB, max_it, tol, envelope, n64, trace64, accept64);
                 if (n64 != n_fw || trace64 != trace) atomicAdd(&a.out.stats[s].n_search_flips, 1);
                 if (accept64 != flag) atomicAdd(&a.out.stats[s].n_accept_flips, 1);
             }
@@ -3464,7 +3468,11 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     k_check<<<1, 1, 0, st>>>(a.ws.counters, kNItems, caps->item_capacity, RB_STATUS_ITEM_OVERFLOW, out->status); note_launch();
     prof_mark(prof, 2, st);
     // narrow phase
-    if (pr->precision != RB_PRECISION_FP64 && sh->grid32) {
+    // The search on the FP32 grid copy makes the FP64 search's decisions (near-ties go to FP64 lookups), so it finds the
+    // same contacts; with FP64 lookups rid of their divisions it is the slower one, for its error bounds and second
+    // lookups (512 piles with a grid per body 1284 against 710 us, 4096-body lattice 213 against 137).  It runs where its
+    // own statistics are asked for: the lookups on the copy and the decision flips of a profiled step.
+    if (pr->precision != RB_PRECISION_FP64 && sh->grid32 && prof) {
         k_narrow<true><<<narrow_blocks, narrow_threads, 0, st>>>(a); note_launch();
     } else {
         k_narrow<false><<<narrow_blocks, narrow_threads, 0, st>>>(a); note_launch();
