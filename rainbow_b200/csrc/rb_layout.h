@@ -45,7 +45,6 @@ struct Workspace {
     double* item_g;      // C
     // contacts
     int32_t* lohi;       // 2K
-    int32_t* c_scene;    // K
     int32_t* bc_list;    // 2K
     double* J;           // 48K
     double* WJT;         // 48K
@@ -102,7 +101,7 @@ inline size_t layout(Workspace* ws, char* base, int64_t N, int64_t NV, int64_t N
     take(w->pairs, 2 * P); take(w->pair_items, P + 1); take(w->pair_itemsA, P); take(w->pair_cont, P + 1); take(w->pair_ovl, P);
     take(w->item_pair, C); take(w->item_tri, C); take(w->item_flag, C);
     take(w->item_p, 3 * C); take(w->item_n, 3 * C); take(w->item_g, C);
-    take(w->lohi, 2 * K); take(w->c_scene, K); take(w->bc_list, 2 * K);
+    take(w->lohi, 2 * K); take(w->bc_list, 2 * K);
     take(w->J, 48 * K); take(w->WJT, 48 * K); take(w->c32, (size_t)kS32Floats * K); take(w->blist32, 2 * K); take(w->pos32, K);
     take(w->body32, (size_t)kS32BodyFloats * N);
     take(w->b, 4 * K); take(w->diag, 4 * K); take(w->r, 4 * K); take(w->x, 4 * K); take(w->xold, 4 * K);

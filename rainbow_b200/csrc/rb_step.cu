@@ -46,6 +46,7 @@ void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 constexpr int kWarpsPerBlock = 4;
 constexpr int kBlock = 32 * kWarpsPerBlock;
 constexpr int kAbort = 15;   // counters[kAbort]: nonzero once a capacity was exceeded
+constexpr int kNWide = 13, kWideNext = 14;   // counters: pairs of k_mid_wide, and the next of them
 constexpr int kSolveSmemBodies = 4608;   // 216 KB of body accumulators per solver block
 
 // ---------------------------------------------------------------------------------------------------------
@@ -361,9 +362,40 @@ __device__ __forceinline__ void mid_arrays(int max_clusters, int warp, int16_t*&
     listB = listA + max_clusters;
 }
 
-// single pass: warps take pairs from a shared counter, find the pair's candidate triangles, reserve room
-// with one atomic and write them in ascending (side, triangle) order; pair_items[p] = first candidate of
-// the pair, pair_itemsA[p] = number of candidates
+// writes a pair's candidates, the set bits of both sides' masks, in ascending (side, triangle) order, in room reserved
+// with one atomic: pair_items[p] = first candidate of the pair, pair_itemsA[p] = their number (one warp)
+__device__ __forceinline__ void mid_emit(const StepArgs& a, int p, int nA, int nB, const int16_t* listA, const int16_t* listB,
+                                         const uint32_t* maskA, const uint32_t* maskB, int n_ovl) {
+    const int lane = threadIdx.x & 31;
+    int cnt = 0;
+    for (int k = lane; k < nA; k += 32) cnt += __popc(maskA[k]);
+    for (int k = lane; k < nB; k += 32) cnt += __popc(maskB[k]);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    int pos = 0;
+    if (lane == 0) pos = atomicAdd(a.ws.counters + kNItems, cnt);
+    pos = __shfl_sync(0xffffffffu, pos, 0);
+    if (lane == 0) { a.ws.pair_items[p] = pos; a.ws.pair_itemsA[p] = cnt; a.ws.pair_ovl[p] = n_ovl; }
+    if (pos + cnt > a.caps.item_capacity) return;   // k_check aborts the step
+    for (int side = 0; side < 2; ++side) {
+        const int n = side ? nB : nA;
+        const int16_t* list = side ? listB : listA;
+        const uint32_t* mask = side ? maskB : maskA;
+        for (int k = 0; k < n; ++k) {
+            const uint32_t bits = mask[k];
+            if (bits & (1u << lane)) {
+                const int at = pos + __popc(bits & lanemask_lt());
+                a.ws.item_pair[at] = p;
+                a.ws.item_tri[at] = (side << 31) | (32 * list[k] + lane);
+            }
+            pos += __popc(bits);
+        }
+    }
+}
+
+// Single pass: warps take pairs from a shared counter and find the pair's candidate triangles.  A pair of more than
+// kMidLight cluster pairs (4: 944 us, 16: 540, 64: 595 for both kernels on 55,960 pairs) goes to k_mid_wide's list (in pair_cont, which is written later): one warp took up to a
+// millisecond over two deeply overlapping 448-triangle spheres, whatever the other pairs.
+constexpr int kMidLight = 16;
 __global__ void __launch_bounds__(kBlock) k_mid(const StepArgs a, int max_clusters) {
     int16_t *listA, *listB;
     uint32_t *maskA, *maskB;
@@ -410,6 +442,11 @@ __global__ void __launch_bounds__(kBlock) k_mid(const StepArgs a, int max_cluste
             const unsigned bal = __ballot_sync(0xffffffffu, ok);
             if (ok) listB[nB + __popc(bal & lanemask_lt())] = (int16_t)c;
             nB += __popc(bal);
+        }
+        if (nA * nB > kMidLight) {
+            if (lane == 0) a.ws.pair_cont[atomicAdd(a.ws.counters + kNWide, 1)] = p;
+            __syncwarp();
+            continue;
         }
         for (int k = lane; k < nA; k += 32) maskA[k] = 0u;
         for (int k = lane; k < nB; k += 32) maskB[k] = 0u;
@@ -470,33 +507,114 @@ __global__ void __launch_bounds__(kBlock) k_mid(const StepArgs a, int max_cluste
             if (lane == 0) maskA[ia] = bal;
         }
         __syncwarp();
-        int cntA = 0, cntB = 0;
-        for (int k = lane; k < nA; k += 32) cntA += __popc(maskA[k]);
-        for (int k = lane; k < nB; k += 32) cntB += __popc(maskB[k]);
-        cntA = __reduce_add_sync(0xffffffffu, cntA);
-        cntB = __reduce_add_sync(0xffffffffu, cntB);
-        n_ovl = __reduce_add_sync(0xffffffffu, n_ovl);
-        int pos = 0;
-        if (lane == 0) pos = atomicAdd(a.ws.counters + kNItems, cntA + cntB);
-        pos = __shfl_sync(0xffffffffu, pos, 0);
-        if (lane == 0) { a.ws.pair_items[p] = pos; a.ws.pair_itemsA[p] = cntA + cntB; a.ws.pair_ovl[p] = n_ovl; }
-        if (pos + cntA + cntB <= a.caps.item_capacity) {   // otherwise k_check aborts the step
-            for (int side = 0; side < 2; ++side) {
-                const int n = side ? nB : nA;
-                const int16_t* list = side ? listB : listA;
-                const uint32_t* mask = side ? maskB : maskA;
-                for (int k = 0; k < n; ++k) {
-                    const uint32_t bits = mask[k];
-                    if (bits & (1u << lane)) {
-                        const int at = pos + __popc(bits & lanemask_lt());
-                        a.ws.item_pair[at] = p;
-                        a.ws.item_tri[at] = (side << 31) | (32 * list[k] + lane);
-                    }
-                    pos += __popc(bits);
-                }
-            }
-        }
+        mid_emit(a, p, nA, nB, listA, listB, maskA, maskB, __reduce_add_sync(0xffffffffu, n_ovl));
         __syncwarp();
+    }
+}
+
+// The pairs of many cluster pairs, a block each: the leaf boxes of up to kMidCache of B's clusters are computed once into
+// shared memory, and every warp takes clusters of A, finds B's clusters that overlap one a lane each, and tests its 32
+// leaves against the leaves that overlap it, read by all lanes at once.  (All of k_mid with a warp to every pair: 869 us
+// for 55,960 pairs of boxes and 448-triangle spheres, 397 for the 2231 of one pile and 321 for 39,664 lattice pairs; both
+// kernels 540, 120 and 211.)
+constexpr int kMidCache = 16;
+constexpr int kMidWideWarps = 8;
+__host__ __device__ inline size_t mid_wide_bytes(int max_clusters) {
+    return (size_t)kMidCache * 32 * 6 * sizeof(double) + (size_t)3 * sizeof(uint32_t) * max_clusters;
+}
+__global__ void __launch_bounds__(32 * kMidWideWarps) k_mid_wide(const StepArgs a, int max_clusters) {
+    extern __shared__ __align__(16) char wide_smem[];
+    double* leaves = reinterpret_cast<double*>(wide_smem);   // six per leaf of the cached clusters
+    uint32_t* maskA = reinterpret_cast<uint32_t*>(wide_smem + (size_t)kMidCache * 32 * 6 * sizeof(double));
+    uint32_t* maskB = maskA + max_clusters;
+    int16_t* listA = reinterpret_cast<int16_t*>(maskB + max_clusters);
+    int16_t* listB = listA + max_clusters;
+    __shared__ int next, count[2], overlaps;
+    if (a.ws.counters[kAbort]) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n_wide = a.ws.counters[kNWide];
+    const double env = a.pr.envelope;
+    for (;;) {
+        if (threadIdx.x == 0) { next = atomicAdd(a.ws.counters + kWideNext, 1); overlaps = 0; }
+        __syncthreads();
+        if (next >= n_wide) break;
+        const int p = a.ws.pair_cont[next];
+        const int A = a.ws.pairs[2 * p], B = a.ws.pairs[2 * p + 1];
+        const int cA0 = a.bd.body_c0[A], cB0 = a.bd.body_c0[B];
+        const int ntA = a.bd.body_t0[A + 1] - a.bd.body_t0[A], ntB = a.bd.body_t0[B + 1] - a.bd.body_t0[B];
+        const int32_t* TA = a.sh.T + 3 * (size_t)a.sh.t_off[a.bd.shape[A]];
+        const int32_t* TB = a.sh.T + 3 * (size_t)a.sh.t_off[a.bd.shape[B]];
+        const double* VwA = a.ws.Vw + 3 * (size_t)a.bd.body_v0[A];
+        const double* VwB = a.ws.Vw + 3 * (size_t)a.bd.body_v0[B];
+        if (wid < 2) {   // the clusters of either body that overlap the other's box
+            const int me = wid ? B : A, c1 = wid ? cB0 : cA0, nc = a.bd.body_c0[me + 1] - c1;
+            const double* other = a.ws.root + 6 * (wid ? A : B);
+            int16_t* list = wid ? listB : listA;
+            uint32_t* mask = wid ? maskB : maskA;
+            int n = 0;
+            for (int c0 = 0; c0 < nc; c0 += 32) {
+                const int c = c0 + lane;
+                const bool ok = c < nc && overlap(a.ws.clu + 6 * (size_t)(c1 + c), other);
+                const unsigned bal = __ballot_sync(0xffffffffu, ok);
+                if (ok) { const int at = n + __popc(bal & lanemask_lt()); list[at] = (int16_t)c; mask[at] = 0u; }
+                n += __popc(bal);
+            }
+            if (lane == 0) count[wid] = n;
+        }
+        __syncthreads();
+        const int nA = count[0], nB = count[1];
+        int n_ovl = 0;
+        for (int b0 = 0; b0 < nB; b0 += kMidCache) {
+            const int nb = min(kMidCache, nB - b0);
+            for (int ib = wid; ib < nb; ib += kMidWideWarps) {
+                const int t = 32 * listB[b0 + ib] + lane;
+                double L[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};   // overlaps nothing
+                if (t < ntB) leaf_box(TB, VwB, t, env, L);
+                double2* o = reinterpret_cast<double2*>(leaves + 6 * (32 * ib + lane));
+                o[0] = make_double2(L[0], L[1]); o[1] = make_double2(L[2], L[3]); o[2] = make_double2(L[4], L[5]);
+            }
+            __syncthreads();
+            for (int ia = wid; ia < nA; ia += kMidWideWarps) {
+                const int ca = listA[ia];
+                double CA[6], LA[6];
+                for (int k = 0; k < 6; ++k) CA[k] = a.ws.clu[6 * (size_t)(cA0 + ca) + k];
+                const int ta = 32 * ca + lane;
+                const bool validA = ta < ntA;
+                if (validA) leaf_box(TA, VwA, ta, env, LA);
+                unsigned todo = __ballot_sync(0xffffffffu, lane < nb && overlap(CA, a.ws.clu + 6 * (size_t)(cB0 + listB[b0 + min(lane, nb - 1)])));
+                bool hitA = false;
+                for (; todo; todo &= todo - 1) {
+                    const int ib = __ffs(todo) - 1;
+                    const double* CB = a.ws.clu + 6 * (size_t)(cB0 + listB[b0 + ib]);
+                    // a leaf pair can only overlap if each leaf overlaps the other leaf's cluster box
+                    const bool mine = validA && overlap(LA, CB);
+                    if (!__any_sync(0xffffffffu, mine)) continue;
+                    const int tb = 32 * listB[b0 + ib] + lane;
+                    unsigned bmask = __ballot_sync(0xffffffffu, tb < ntB && overlap(leaves + 6 * (32 * ib + lane), CA));
+                    unsigned hitB = 0u;
+                    for (; bmask; bmask &= bmask - 1) {
+                        const int jb = __ffs(bmask) - 1;
+                        const double2* q = reinterpret_cast<const double2*>(leaves + 6 * (32 * ib + jb));
+                        const double2 q0 = q[0], q1 = q[1], q2 = q[2];
+                        // the six comparisons of overlap(), without branches
+                        const bool ov = mine & !((LA[3] < q0.x) | (q1.y < LA[0]) | (LA[4] < q0.y) | (q2.x < LA[1]) |
+                                                 (LA[5] < q1.x) | (q2.y < LA[2]));
+                        const unsigned bal = __ballot_sync(0xffffffffu, ov);
+                        hitA |= ov;
+                        if (bal) hitB |= 1u << jb;
+                        n_ovl += __popc(bal);
+                    }
+                    if (lane == 0 && hitB) atomicOr(maskB + b0 + ib, hitB);
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, hitA);
+                if (lane == 0) maskA[ia] |= bal;   // the warp's own cluster
+            }
+            __syncthreads();
+        }
+        if (lane == 0) atomicAdd(&overlaps, n_ovl);
+        __syncthreads();
+        if (wid == 0) mid_emit(a, p, nA, nB, listA, listB, maskA, maskB, overlaps);
+        __syncthreads();
     }
 }
 
@@ -691,71 +809,85 @@ __global__ void __launch_bounds__(256, 2) k_narrow(const StepArgs a) {
 // ---------------------------------------------------------------------------------------------------------
 // contact reduction (collision_detection.py:255): a contact is dropped when an earlier contact of the same
 // unordered body pair has the identical position.  Contacts of one body pair are contiguous (one pair list
-// entry), so the test runs per pair.  Pass 1 counts survivors, pass 2 writes them in order.
+// entry), so the test runs per pair.
 // ---------------------------------------------------------------------------------------------------------
-template <bool WRITE>
-__global__ void k_dedup(const StepArgs a) {
+// Few candidates of a pair are accepted (of 4.3 million in 55,960 pairs 94,817 are kept), so a warp collects the
+// accepted ones' positions first, in order, and compares each with the kept ones before it; the kept candidates'
+// indices go to the pair's room in item_pair, which is not read any more, for the write pass to go over alone.
+// (Comparing every chunk of candidates with every earlier chunk, and scanning all of them again in the write pass,
+// took 316 and 119 us; this 72 and 42.)
+constexpr int kDedupRoom = 64;   // accepted candidates a warp holds at a time
+__global__ void __launch_bounds__(kBlock) k_dedup(const StepArgs a) {
+    __shared__ double pos[kWarpsPerBlock][kDedupRoom][3];
+    __shared__ int index[kWarpsPerBlock][kDedupRoom];
     if (a.ws.counters[kAbort]) return;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int n_pairs = a.ws.counters[kNPairs];
     for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n_pairs; p += (gridDim.x * blockDim.x) >> 5) {
         const int i0 = a.ws.pair_items[p], i1 = i0 + a.ws.pair_itemsA[p];
         int kept = 0;
-        int base = WRITE ? a.ws.pair_cont[p] : 0;
-        const int A = a.ws.pairs[2 * p], B = a.ws.pairs[2 * p + 1];
-        for (int c0 = i0; c0 < i1; c0 += 32) {
-            const int i = c0 + lane;
-            bool keep = false;
-            if (!WRITE) {
-                // candidate i is kept if no earlier accepted candidate of the pair has its position: the
-                // earlier accepted ones, 32 at a time, are found by ballot and their positions broadcast
+        for (int c0 = i0; c0 < i1;) {
+            // the next accepted candidates, as many whole chunks of 32 as there is room for
+            int n = 0;
+            for (; c0 < i1 && n <= kDedupRoom - 32; c0 += 32) {
+                const int i = c0 + lane;
                 const bool mine = i < i1 && a.ws.item_flag[i] != 0;
-                double px = 0.0, py = 0.0, pz = 0.0;
-                if (mine) { const double* pi = a.ws.item_p + 3 * (size_t)i; px = pi[0]; py = pi[1]; pz = pi[2]; }
-                keep = mine;
-                for (int e0 = i0; e0 <= c0; e0 += 32) {
-                    const int j = e0 + lane;
-                    const bool fj = j < i1 && (e0 == c0 ? mine : a.ws.item_flag[j] != 0);
-                    double qx = 0.0, qy = 0.0, qz = 0.0;
-                    if (fj) { const double* pj = a.ws.item_p + 3 * (size_t)j; qx = pj[0]; qy = pj[1]; qz = pj[2]; }
-                    unsigned m = __ballot_sync(0xffffffffu, fj);
-                    while (m) {   // in the own chunk only lanes below this one count as earlier
-                        const int b = __ffs(m) - 1;
-                        m &= m - 1;
-                        const double bx = __shfl_sync(0xffffffffu, qx, b);
-                        const double by = __shfl_sync(0xffffffffu, qy, b);
-                        const double bz = __shfl_sync(0xffffffffu, qz, b);
-                        const bool earlier = e0 < c0 || b < lane;
-                        if (keep && earlier && px == bx && py == by && pz == bz) keep = false;
-                    }
+                const unsigned bal = __ballot_sync(0xffffffffu, mine);
+                if (mine) {
+                    const int at = n + __popc(bal & lanemask_lt());
+                    const double* q = a.ws.item_p + 3 * (size_t)i;
+                    pos[wid][at][0] = q[0]; pos[wid][at][1] = q[1]; pos[wid][at][2] = q[2];
+                    index[wid][at] = i;
                 }
-            } else {
-                keep = i < i1 && a.ws.item_flag[i] == 2;
+                n += __popc(bal);
             }
-            const unsigned bal = __ballot_sync(0xffffffffu, keep);
-            if (!WRITE && i < i1 && keep) a.ws.item_flag[i] = 2;   // the write pass reads flag 2 = kept
-            if (WRITE && keep) {
-                const int k = base + kept + __popc(bal & lanemask_lt());
-                if (k < a.caps.contact_capacity) {
-                    const int side = ((unsigned)a.ws.item_tri[i]) >> 31;
-                    const int mesh = side ? B : A, sdf = side ? A : B;
-                    a.out.contact_ids[2 * k] = sdf;     // ContactPoint(bodyB_sdf_owner, bodyA_mesh_owner, ...)
-                    a.out.contact_ids[2 * k + 1] = mesh;
-                    for (int c = 0; c < 3; ++c) {
-                        a.out.contact_p[3 * k + c] = a.ws.item_p[3 * (size_t)i + c];
-                        a.out.contact_n[3 * k + c] = a.ws.item_n[3 * (size_t)i + c];
-                    }
-                    a.out.contact_g[k] = a.ws.item_g[i];
-                    a.ws.c_scene[k] = scene_of(a.bd.scene_start, a.bd.n_scenes, A);
-                    // key of the contact for warm starting: contacts come out in ascending key order
-                    a.ws.ckey[2 * k] = ((int64_t)A << 31) | (int64_t)B;
-                    a.ws.ckey[2 * k + 1] = (int64_t)(((unsigned)a.ws.item_tri[i] >> 31) << 30) |
-                                           (int64_t)(a.ws.item_tri[i] & 0x7fffffff);
+            __syncwarp();
+            for (int j0 = 0; j0 < n; j0 += 32) {
+                const int j = j0 + lane;
+                bool keep = j < n;
+                const double px = pos[wid][keep ? j : 0][0], py = pos[wid][keep ? j : 0][1], pz = pos[wid][keep ? j : 0][2];
+                for (int e = 0; e < kept; ++e) {   // those kept in earlier chunks
+                    const double* q = a.ws.item_p + 3 * (size_t)a.ws.item_pair[i0 + e];
+                    if (q[0] == px && q[1] == py && q[2] == pz) keep = false;
                 }
+                const int own = min(32, n - j0);
+                for (int e = 0; e < own; ++e)      // and the earlier ones of this chunk (a dropped one equals a kept one)
+                    if (e < lane && pos[wid][j0 + e][0] == px && pos[wid][j0 + e][1] == py && pos[wid][j0 + e][2] == pz)
+                        keep = false;
+                const unsigned bal = __ballot_sync(0xffffffffu, keep);
+                if (keep) a.ws.item_pair[i0 + kept + __popc(bal & lanemask_lt())] = index[wid][j];
+                kept += __popc(bal);
+                __syncwarp();
             }
-            kept += __popc(bal);
         }
-        if (!WRITE && lane == 0) a.ws.pair_cont[p] = kept;
+        if (lane == 0) a.ws.pair_cont[p] = kept;
+    }
+}
+
+// the kept candidates become contacts, in order: eight lanes a pair (most have fewer than eight contacts)
+__global__ void k_emit(const StepArgs a) {
+    if (a.ws.counters[kAbort]) return;
+    const int n_pairs = a.ws.counters[kNPairs];
+    for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; p < n_pairs; p += (gridDim.x * blockDim.x) >> 3) {
+        const int base = a.ws.pair_cont[p], end = min(a.ws.pair_cont[p + 1], a.caps.contact_capacity);
+        if (base >= end) continue;
+        const int i0 = a.ws.pair_items[p];
+        const int A = a.ws.pairs[2 * p], B = a.ws.pairs[2 * p + 1];
+        for (int k = base + (threadIdx.x & 7); k < end; k += 8) {
+            const int i = a.ws.item_pair[i0 + k - base];
+            const int tri = a.ws.item_tri[i];
+            const int side = (unsigned)tri >> 31;
+            a.out.contact_ids[2 * k] = side ? A : B;     // ContactPoint(bodyB_sdf_owner, bodyA_mesh_owner, ...)
+            a.out.contact_ids[2 * k + 1] = side ? B : A;
+            for (int c = 0; c < 3; ++c) {
+                a.out.contact_p[3 * (size_t)k + c] = a.ws.item_p[3 * (size_t)i + c];
+                a.out.contact_n[3 * (size_t)k + c] = a.ws.item_n[3 * (size_t)i + c];
+            }
+            a.out.contact_g[k] = a.ws.item_g[i];
+            // key of the contact for warm starting: contacts come out in ascending key order
+            a.ws.ckey[2 * (size_t)k] = ((int64_t)A << 31) | (int64_t)B;
+            a.ws.ckey[2 * (size_t)k + 1] = (int64_t)(side << 30) | (int64_t)(tri & 0x7fffffff);
+        }
     }
 }
 
@@ -900,55 +1032,45 @@ __global__ void k_contacts(const StepArgs a) {
         if (row == 0) {
             a.ws.lohi[2 * k] = lo;
             a.ws.lohi[2 * k + 1] = hi;
+            if (hasw[0]) atomicAdd(a.ws.bc_ptr + lo, 1);
+            if (hasw[1]) atomicAdd(a.ws.bc_ptr + hi, 1);
             a.ws.mu[k] = a.bd.material_mu[3 * entry];
         }
     }
 }
 
-// per-body contact lists, ascending contact index (the column order of the SciPy products)
-__global__ void k_body_contacts_count(const StepArgs a) {
-    if (a.ws.counters[kAbort]) return;
-    const int K = a.ws.counters[kNContacts];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x)
-        for (int side = 0; side < 2; ++side) {
-            const int b = a.ws.lohi[2 * k + side];
-            if (!a.bd.fixed[b]) atomicAdd(a.ws.bc_ptr + b, 1);
-        }
-}
+// per-body contact lists, ascending contact index (the column order of the SciPy products): counted by k_contacts,
+// filled in any order, then sorted.  A fixed body has no list, and its contacts no predecessor on it.
 __global__ void k_body_contacts_fill(const StepArgs a) {
     if (a.ws.counters[kAbort]) return;
     const int K = a.ws.counters[kNContacts];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x)
-        for (int side = 0; side < 2; ++side) {
-            const int b = a.ws.lohi[2 * k + side];
-            if (a.bd.fixed[b]) continue;
-            const int at = a.ws.bc_ptr[b] + atomicAdd(a.ws.bc_fill + b, 1);
-            a.ws.bc_list[at] = (k << 1) | side;
-        }
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < 2 * K; c += gridDim.x * blockDim.x) {   // k << 1 | side
+        const int b = a.ws.lohi[c];
+        if (a.bd.fixed[b]) { a.ws.cpred[c] = -1; continue; }
+        a.ws.blist32[a.ws.bc_ptr[b] + atomicAdd(a.ws.bc_fill + b, 1)] = (uint32_t)c;
+    }
 }
+// a warp per body: an entry's place is the number of smaller ones (one thread's insertion sort took 357 us where the
+// busiest of 37,148 bodies has ~100 contacts, this 16); then the predecessor of each contact along this body, the
+// chain the Gauss-Seidel levels follow
 __global__ void k_body_contacts_sort(const StepArgs a) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (b >= a.bd.n_bodies || a.ws.counters[kAbort]) return;
-    int32_t* l = a.ws.bc_list + a.ws.bc_ptr[b];
-    const int n = a.ws.bc_ptr[b + 1] - a.ws.bc_ptr[b];
-    for (int i = 1; i < n; ++i) {
-        const int32_t v = l[i];
-        int j = i - 1;
-        while (j >= 0 && l[j] > v) { l[j + 1] = l[j]; --j; }
-        l[j + 1] = v;
+    const int e0 = a.ws.bc_ptr[b], n = a.ws.bc_ptr[b + 1] - e0;
+    const uint32_t* in = a.ws.blist32 + e0;
+    int32_t* out = a.ws.bc_list + e0;
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const uint32_t v = c0 + lane < n ? in[c0 + lane] : 0xffffffffu;
+        int rank = 0;
+        for (int d0 = 0; d0 < n; d0 += 32) {
+            const uint32_t u = d0 + lane < n ? in[d0 + lane] : 0xffffffffu;
+            const int m = min(32, n - d0);
+            for (int e = 0; e < m; ++e) rank += __shfl_sync(0xffffffffu, u, e) < v;
+        }
+        if (c0 + lane < n) out[rank] = (int32_t)v;
     }
-    // predecessor of each contact along this body: the chain the Gauss-Seidel levels follow
-    int prev = -1;
-    for (int i = 0; i < n; ++i) {
-        const int code = l[i];
-        a.ws.cpred[code] = prev;   // code = (k << 1) | side
-        prev = code >> 1;
-    }
-}
-__global__ void k_preds_init(const StepArgs a) {
-    if (a.ws.counters[kAbort]) return;
-    const int K = a.ws.counters[kNContacts];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * K; i += gridDim.x * blockDim.x) a.ws.cpred[i] = -1;
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) a.ws.cpred[out[i]] = i > 0 ? out[i - 1] >> 1 : -1;
 }
 
 // component d of (WJT x) of a body, over its contacts bc_list[e0 .. e1): sequential over the contacts (ascending)
@@ -3462,8 +3584,12 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     // mid phase
     {
         const int max_clusters = (sh->max_shape_triangles + 31) / 32;
-        const size_t mid_smem = (size_t)kWarpsPerBlock * 3 * sizeof(uint32_t) * (max_clusters > 0 ? max_clusters : 1);
-        k_mid<<<mid_blocks, kBlock, mid_smem, st>>>(a, max_clusters > 0 ? max_clusters : 1); note_launch();
+        const size_t mid_smem = (size_t)kWarpsPerBlock * 3 * sizeof(uint32_t) * max_clusters;
+        k_mid<<<mid_blocks, kBlock, mid_smem, st>>>(a, max_clusters); note_launch();
+        // no pair of single-cluster shapes (up to 32 triangles) is a wide one
+        if (max_clusters * max_clusters > kMidLight) {
+            k_mid_wide<<<148 * 4, 32 * kMidWideWarps, mid_wide_bytes(max_clusters), st>>>(a, max_clusters); note_launch();
+        }
     }
     k_check<<<1, 1, 0, st>>>(a.ws.counters, kNItems, caps->item_capacity, RB_STATUS_ITEM_OVERFLOW, out->status); note_launch();
     prof_mark(prof, 2, st);
@@ -3479,10 +3605,10 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     }
     prof_mark(prof, 3, st);
     // reduction and compaction
-    k_dedup<false><<<G, kBlock, 0, st>>>(a); note_launch();
+    k_dedup<<<2 * G, kBlock, 0, st>>>(a); note_launch();
     scan(a.ws.pair_cont, a.ws.counters + kNPairs, caps->pair_capacity, a.ws.scan_tmp, a.ws.counters + kNContacts, st);
     k_check<<<1, 1, 0, st>>>(a.ws.counters, kNContacts, caps->contact_capacity, RB_STATUS_CONTACT_OVERFLOW, out->status); note_launch();
-    k_dedup<true><<<G, kBlock, 0, st>>>(a); note_launch();
+    k_emit<<<2 * G, kBlock, 0, st>>>(a); note_launch();
     prof_mark(prof, 4, st);
     // contact problem
     k_contacts<<<2 * G, 128, 0, st>>>(a); note_launch();   // a thread per contact row
@@ -3490,11 +3616,9 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
         k_hinge_lists<<<blocks_for(bd->n_scenes, 64), 64, 0, st>>>(a); note_launch();
         k_hinges<<<blocks_for(bd->n_hinges, 128), 128, 0, st>>>(a); note_launch();
     }
-    k_body_contacts_count<<<G, 256, 0, st>>>(a); note_launch();
     scan(a.ws.bc_ptr, nullptr, N, a.ws.scan_tmp, nullptr, st);
     k_body_contacts_fill<<<G, 256, 0, st>>>(a); note_launch();
-    k_preds_init<<<G, 256, 0, st>>>(a); note_launch();
-    k_body_contacts_sort<<<blocks_for(N, 128), 128, 0, st>>>(a); note_launch();
+    k_body_contacts_sort<<<blocks_for(32 * (int64_t)N, 128), 128, 0, st>>>(a); note_launch();
     // solve, integrate, post-stabilise
     // small scenes: one warp each with its body accumulators in shared memory; large scenes: one block each
     // a warp per scene only pays off once the scenes alone fill the GPU (>= 32 per SM); otherwise blocks

@@ -81,3 +81,38 @@ def test_level_widths(oracle_lib, pool, count, fixed_ground):
     rp = W.make_rb_params(params)
     o = oracle_lib.OracleScene(a)
     _compare(world, {0: o}, [0], rp, 2)
+
+
+@pytest.mark.parametrize("slices,resolution", [(4, 12), (8, 12), (16, 12), (24, 10)])
+def test_deep_overlaps(oracle_lib, slices, resolution):
+    """Spheres of 32 to 1100 triangles deep inside one another and a ground: candidate pairs of one cluster pair up to
+    more than the wide mid phase caches, many accepted candidates and duplicates per pair, long contact lists."""
+    from rainbow_b200 import api as API, engine_io, geometry as GEO, world as W
+    engine = API.create_engine("cuda:0")
+    engine.params.resolution = resolution
+    engine.params.max_iterations = 5
+    API.create_surfaces_interaction(engine, "m", "m", 0.0, np.array([0.4, 0.4, 0.4]))
+    V, T = GEO.create_box(8.0, 1.0, 8.0)
+    API.create_shape(engine, "ground", API.create_mesh(V, T))
+    V, T = GEO.create_sphere(1.5, slices, slices)
+    API.create_shape(engine, "ball", API.create_mesh(V, T))
+    API.create_gravity_force(engine, "gravity", 9.81, np.array([0.0, 1.0, 0.0]))
+    rng = np.random.default_rng(slices)
+    for k in range(7):
+        name = "b%d" % k
+        API.create_rigid_body(engine, name)
+        API.connect_shape(engine, name, "ball" if k else "ground")
+        API.set_position(engine, name, rng.uniform(-0.7, 0.7, 3) + [0.0, 1.2, 0.0] if k else np.array([0.0, -0.5, 0.0]), True)
+        q = rng.normal(size=4)
+        API.set_orientation(engine, name, q / np.linalg.norm(q) if k else np.array([1.0, 0.0, 0.0, 0.0]), True)
+        API.set_mass_properties(engine, name, 1.0)
+        API.set_body_material(engine, name, "m")
+        if k:
+            API.connect_force(engine, name, "gravity")
+        else:
+            API.set_body_type(engine, name, "fixed")
+    arrays = engine_io.scene_arrays(engine)
+    world = W.DeviceWorld([arrays, arrays], device="cuda:0", max_iterations=100)
+    o = oracle_lib.OracleScene(arrays)
+    rp = W.make_rb_params(W.params_from_vector(arrays["params"]))
+    _compare(world, {1: o}, [1], rp, 2, capacity=1 << 15)
