@@ -113,9 +113,9 @@ int rb_build_topology(const rb_shapes* sh, const rb_bodies* bd, void* scratch, s
     const int N = bd->n_bodies;
     k_topology_counts<<<blocks_for(N, 256), 256, 0, st>>>(*sh, *bd, v0, t0, c0);
     rb::note_launch();
-    rb::scan(v0, nullptr, N, partial, nullptr, st);
-    rb::scan(t0, nullptr, N, partial, nullptr, st);
-    rb::scan(c0, nullptr, N, partial, nullptr, st);
+    rb::scan(v0, nullptr, N, partial, st);
+    rb::scan(t0, nullptr, N, partial, st);
+    rb::scan(c0, nullptr, N, partial, st);
     k_topology_owners<<<blocks_for(32 * (int64_t)N, 256), 256, 0, st>>>(*bd, const_cast<int32_t*>(bd->vert_body),
                                                                        const_cast<int32_t*>(bd->tri_body),
                                                                        const_cast<int32_t*>(bd->clu_body));
@@ -158,7 +158,7 @@ int rb_repack(const int32_t* body_map, int32_t n_old_bodies, const double* x_old
         k_cache_keep<<<G, 256, 0, st>>>(body_map, n_old_bodies, cache_key_old, cache_count_old, cache_capacity_old,
                                          keep);
         rb::note_launch();
-        rb::scan(keep, cache_count_old, cache_capacity_old, partial, nullptr, st);
+        rb::scan(keep, cache_count_old, cache_capacity_old, partial, st);
         k_cache_move<<<G, 256, 0, st>>>(body_map, cache_key_old, cache_sol_old, cache_count_old, cache_capacity_old,
                                          keep, cache_key_new, cache_sol_new, cache_count_new, cache_capacity_new);
         rb::note_launch();

@@ -90,7 +90,22 @@ __global__ void k_scan_reduce(const int32_t* __restrict__ data, const int32_t* n
         partial[blockIdx.x] = t;
     }
 }
-__global__ void k_scan_top(int32_t* __restrict__ partial, int nblocks, int32_t* total_out) {
+// what becomes of a scan's total: written to counters[which], and, above the capacity, the status bit that aborts the
+// rest of the step (unless an earlier stage overflowed: the total is not meaningful then)
+struct ScanTotal {
+    int32_t* counters = nullptr;
+    int which = 0, capacity = 0, bit = 0;
+    int32_t* status = nullptr;
+    __device__ __forceinline__ void put(int32_t total) const {
+        if (!counters) return;
+        counters[which] = total;
+        if (!counters[kAbort] && total > capacity) {
+            atomicOr(counters + kAbort, bit);
+            atomicOr(status, bit);
+        }
+    }
+};
+__global__ void k_scan_top(int32_t* __restrict__ partial, int nblocks, const ScanTotal total) {
     // single block of 1024 threads, nblocks <= 1024
     __shared__ int s[1024];
     const int t = threadIdx.x;
@@ -104,7 +119,52 @@ __global__ void k_scan_top(int32_t* __restrict__ partial, int nblocks, int32_t* 
         __syncthreads();
     }
     if (t < nblocks) partial[t] = s[t] - v;
-    if (t == 1023) { partial[nblocks] = s[t]; if (total_out) *total_out = s[t]; }
+    if (t == 1023) { partial[nblocks] = s[t]; total.put(s[t]); }
+}
+// the whole scan by one block: with few elements the launches of the three phases cost more than the elements
+// (11 us against 4 for 4097 bodies)
+constexpr int kScanOne = 16384;
+__global__ void __launch_bounds__(1024) k_scan_one(int32_t* __restrict__ data, const int32_t* n_dev, int n_host,
+                                                   const ScanTotal total) {
+    __shared__ int ws[33];
+    const int n = scan_n(n_dev, n_host);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < n; base += 4096) {   // four elements a thread
+        const int i = base + 4 * threadIdx.x;
+        int v[4], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { v[k] = i + k < n ? data[i + k] : 0; sum += v[k]; }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += a;
+        }
+        if (lane == 31) ws[wid] = incl;
+        __syncthreads();
+        if (wid == 0) {
+            const int w = ws[lane];
+            int wi = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, wi, o);
+                if (lane >= o) wi += a;
+            }
+            ws[lane] = wi - w;
+            if (lane == 31) ws[32] = wi;
+        }
+        __syncthreads();
+        int at = carry + ws[wid] + incl - sum;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (i + k < n) data[i + k] = at;
+            at += v[k];
+        }
+        carry += ws[32];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) { data[n] = carry; total.put(carry); }
 }
 __global__ void k_scan_down(int32_t* __restrict__ data, const int32_t* n_dev, int n_host,
                             const int32_t* __restrict__ partial) {
@@ -144,24 +204,19 @@ __global__ void k_scan_down(int32_t* __restrict__ data, const int32_t* n_dev, in
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) data[n] = partial[gridDim.x];
 }
-void scan(int32_t* data, const int32_t* n_dev, int n_host, int32_t* partial, int32_t* total_out, cudaStream_t st) {
+static void scan_total(int32_t* data, const int32_t* n_dev, int n_host, int32_t* partial, const ScanTotal total,
+                       cudaStream_t st) {
+    if (n_host <= kScanOne) {
+        k_scan_one<<<1, 1024, 0, st>>>(data, n_dev, n_host, total); note_launch();
+        return;
+    }
     const int G = kScanGrid;
     k_scan_reduce<<<G, 256, 0, st>>>(data, n_dev, n_host, partial); note_launch();
-    k_scan_top<<<1, 1024, 0, st>>>(partial, G, total_out); note_launch();
+    k_scan_top<<<1, 1024, 0, st>>>(partial, G, total); note_launch();
     k_scan_down<<<G, 256, 0, st>>>(data, n_dev, n_host, partial); note_launch();
 }
-
-__global__ void k_zero_i32(int32_t* p, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = 0;
-}
-struct StepArgs;
-// capacity check after a scan: a total above the capacity aborts the rest of the step
-__global__ void k_check(int32_t* counters, int which, int cap, int bit, int32_t* status) {
-    if (counters[kAbort]) return;   // an earlier stage overflowed: this stage's total is not meaningful
-    if (counters[which] > cap) {
-        atomicOr(counters + kAbort, bit);
-        atomicOr(status, bit);
-    }
+void scan(int32_t* data, const int32_t* n_dev, int n_host, int32_t* partial, cudaStream_t st) {
+    scan_total(data, n_dev, n_host, partial, ScanTotal{}, st);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -176,9 +231,20 @@ struct StepArgs {
     Workspace ws;
 };
 
+// also starts the step: counters, contact counts and the scenes' statistics at zero, and, with no FP32 phase to do it
+// (it reads the last step's), the scenes' FP32 bookkeeping
 __global__ void k_bodies(const StepArgs a) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < 16) a.ws.counters[b] = 0;
+    if (b <= a.bd.n_bodies) a.ws.bc_ptr[b] = 0;
+    if (b < a.bd.n_scenes) {
+        rb_scene_stats* st = a.out.stats + b;
+        st->n_grid_lookups = 0; st->n_leaf_overlaps = 0;
+        st->n_grid_lookups32 = 0; st->n_search_flips = 0; st->n_accept_flips = 0;
+        if (a.pr.precision == RB_PRECISION_FP64) { a.ws.sweeps32[b] = -1; a.ws.fin32[b] = 0; }
+    }
     if (b >= a.bd.n_bodies) return;
+    a.ws.bc_fill[b] = 0;
     double* d = a.ws.dux + 6 * b;
     double* du = a.ws.du + 6 * b;
     double* Wi = a.ws.Winv + 9 * b;
@@ -225,15 +291,6 @@ __global__ void k_bodies(const StepArgs a) {
         t += Wi[3 * i + 2] * T[2];
         d[i] = s; d[3 + i] = t;
         du[i] = dt * s; du[3 + i] = dt * t;   // steppers.py:64 delta_u = dt * delta_u_ext
-    }
-}
-
-__global__ void k_zero_stats(const StepArgs a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < a.bd.n_scenes) {
-        rb_scene_stats* st = a.out.stats + s;
-        st->n_grid_lookups = 0; st->n_leaf_overlaps = 0;
-        st->n_grid_lookups32 = 0; st->n_search_flips = 0; st->n_accept_flips = 0;
     }
 }
 
@@ -375,7 +432,7 @@ __device__ __forceinline__ void mid_emit(const StepArgs& a, int p, int nA, int n
     if (lane == 0) pos = atomicAdd(a.ws.counters + kNItems, cnt);
     pos = __shfl_sync(0xffffffffu, pos, 0);
     if (lane == 0) { a.ws.pair_items[p] = pos; a.ws.pair_itemsA[p] = cnt; a.ws.pair_ovl[p] = n_ovl; }
-    if (pos + cnt > a.caps.item_capacity) return;   // k_check aborts the step
+    if (pos + cnt > a.caps.item_capacity) return;   // k_narrow aborts the step
     for (int side = 0; side < 2; ++side) {
         const int n = side ? nB : nA;
         const int16_t* list = side ? listB : listA;
@@ -739,6 +796,13 @@ __global__ void __launch_bounds__(256, 2) k_narrow(const StepArgs a) {
     __syncthreads();
     if (a.ws.counters[kAbort]) return;
     const int n_items = a.ws.counters[kNItems];
+    if (n_items > a.caps.item_capacity) {   // the mid phase left the candidates out: the rest of the step is off
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            atomicOr(a.ws.counters + kAbort, RB_STATUS_ITEM_OVERFLOW);
+            atomicOr(a.out.status, RB_STATUS_ITEM_OVERFLOW);
+        }
+        return;
+    }
     const int max_it = a.pr.contact_optimization_max_iterations;
     const double tol = a.pr.contact_optimization_tolerance;
     const double envelope = a.pr.envelope;
@@ -2947,7 +3011,7 @@ __global__ void __launch_bounds__(1024) k_fp32_classes(const StepArgs a, size_t 
     __shared__ int cnt[4 * kClassBuckets];
     const int S = a.bd.n_scenes;
     // no lists after an overflow: the contact ranges are not valid then, and the solvers do not run
-    const bool fp32 = a.pr.precision != RB_PRECISION_FP64 && !a.ws.counters[kAbort];
+    const bool fp32 = !a.ws.counters[kAbort];
     const int max_it = a.pr.max_iterations;
     for (int t = threadIdx.x; t < 4 * kClassBuckets; t += blockDim.x) cnt[t] = 0;
     __syncthreads();
@@ -3270,10 +3334,8 @@ __global__ void k_post_apply(const StepArgs a) {
 // energies and largest penetration (state_storage.py:188, contacts.py:222): thread per scene, body order
 // one warp per scene: the deepest gap and the pair / candidate counts by warp reductions (order-free), the
 // energy sums by lane 0 in body order (their rounding follows state_storage.py:188-237)
-__global__ void k_scene_summary(const StepArgs a) {
-    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void scene_summary(const StepArgs& a, int s) {
     const int lane = threadIdx.x & 31;
-    if (s >= a.bd.n_scenes || a.ws.counters[kAbort]) return;
     rb_scene_stats* st = a.out.stats + s;
     const SceneRange R = scene_range(a, s);
     double gap = 0.0;
@@ -3344,27 +3406,32 @@ __global__ void k_body_energy(const StepArgs a) {
     out[1] = pot;
 }
 
-// keep this step's contact keys and impulses for the next step's warm start
-__global__ void k_cache_store(const StepArgs a) {
-    if (!a.out.cache_key || !a.out.cache_sol || !a.out.cache_count) return;
-    if (a.ws.counters[kAbort]) return;
+// The end of the step: the scenes' summaries by the first blocks, and by the others this step's contact keys and impulses
+// kept for the next step's warm start; one thread writes the totals.
+__global__ void __launch_bounds__(128) k_outputs(const StepArgs a, int summary_blocks) {
+    const int ab = a.ws.counters[kAbort];
+    if ((int)blockIdx.x < summary_blocks) {
+        const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        if (s < a.bd.n_scenes && !ab) scene_summary(a, s);
+        return;
+    }
+    const int at = (blockIdx.x - summary_blocks) * blockDim.x + threadIdx.x;
+    if (at == 0) {
+        if (a.out.n_contacts_total) *a.out.n_contacts_total = a.ws.counters[kNContacts];
+        if (a.out.needed) {   // a stage after an overflow did not run: its total is reported as 0
+            a.out.needed[0] = a.ws.counters[kNPairs];
+            a.out.needed[1] = (ab & RB_STATUS_PAIR_OVERFLOW) ? 0 : a.ws.counters[kNItems];
+            a.out.needed[2] = (ab & (RB_STATUS_PAIR_OVERFLOW | RB_STATUS_ITEM_OVERFLOW)) ? 0 : a.ws.counters[kNContacts];
+        }
+    }
+    if (ab || !a.out.cache_key || !a.out.cache_sol || !a.out.cache_count) return;
     const int K = min(a.ws.counters[kNContacts], a.caps.contact_capacity);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
+    for (int k = at; k < K; k += (gridDim.x - summary_blocks) * blockDim.x) {
         a.out.cache_key[2 * k] = a.ws.ckey[2 * k];
         a.out.cache_key[2 * k + 1] = a.ws.ckey[2 * k + 1];
         for (int row = 0; row < 4; ++row) a.out.cache_sol[4 * k + row] = a.out.contact_sol[4 * k + row];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *a.out.cache_count = K;
-}
-
-__global__ void k_finish(const StepArgs a) {
-    if (a.out.n_contacts_total) *a.out.n_contacts_total = a.ws.counters[kNContacts];
-    if (a.out.needed) {   // a stage after an overflow did not run: its total is reported as 0
-        const int ab = a.ws.counters[kAbort];
-        a.out.needed[0] = a.ws.counters[kNPairs];
-        a.out.needed[1] = (ab & RB_STATUS_PAIR_OVERFLOW) ? 0 : a.ws.counters[kNItems];
-        a.out.needed[2] = (ab & (RB_STATUS_PAIR_OVERFLOW | RB_STATUS_ITEM_OVERFLOW)) ? 0 : a.ws.counters[kNContacts];
-    }
+    if (at == 0) *a.out.cache_count = K;
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -3567,19 +3634,15 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     const int G = 148 * 8;
     const bool prof = pr->profiling != 0;
     prof_mark(prof, 0, st);
-    k_zero_i32<<<1, 32, 0, st>>>(a.ws.counters, 16); note_launch();
-    k_zero_stats<<<blocks_for(bd->n_scenes, 128), 128, 0, st>>>(a); note_launch();
-    k_zero_i32<<<blocks_for(N + 1, 256), 256, 0, st>>>(a.ws.bc_ptr, N + 1); note_launch();
-    k_zero_i32<<<blocks_for(N, 256), 256, 0, st>>>(a.ws.bc_fill, N); note_launch();
-    k_bodies<<<blocks_for(N, 128), 128, 0, st>>>(a); note_launch();
+    k_bodies<<<blocks_for(std::max(N + 1, std::max(bd->n_scenes, 16)), 128), 128, 0, st>>>(a); note_launch();
     k_world_vertices<<<blocks_for(n_body_vertices, 256), 256, 0, st>>>(a, (int)n_body_vertices); note_launch();
     k_clusters<<<blocks_for(32 * n_clusters, kBlock), kBlock, 0, st>>>(a, (int)n_clusters); note_launch();
     k_roots<<<blocks_for(32 * (int64_t)N, kBlock), kBlock, 0, st>>>(a); note_launch();
     prof_mark(prof, 1, st);
     // broad phase
     k_pairs<false><<<blocks_for(32 * (int64_t)N, kBlock), kBlock, 0, st>>>(a); note_launch();
-    scan(a.ws.pair_cnt, nullptr, N, a.ws.scan_tmp, a.ws.counters + kNPairs, st);
-    k_check<<<1, 1, 0, st>>>(a.ws.counters, kNPairs, caps->pair_capacity, RB_STATUS_PAIR_OVERFLOW, out->status); note_launch();
+    scan_total(a.ws.pair_cnt, nullptr, N, a.ws.scan_tmp,
+               ScanTotal{a.ws.counters, kNPairs, caps->pair_capacity, RB_STATUS_PAIR_OVERFLOW, out->status}, st);
     k_pairs<true><<<blocks_for(32 * (int64_t)N, kBlock), kBlock, 0, st>>>(a); note_launch();
     // mid phase
     {
@@ -3591,7 +3654,6 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
             k_mid_wide<<<148 * 4, 32 * kMidWideWarps, mid_wide_bytes(max_clusters), st>>>(a, max_clusters); note_launch();
         }
     }
-    k_check<<<1, 1, 0, st>>>(a.ws.counters, kNItems, caps->item_capacity, RB_STATUS_ITEM_OVERFLOW, out->status); note_launch();
     prof_mark(prof, 2, st);
     // narrow phase
     // The search on the FP32 grid copy makes the FP64 search's decisions (near-ties go to FP64 lookups), so it finds the
@@ -3606,8 +3668,8 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     prof_mark(prof, 3, st);
     // reduction and compaction
     k_dedup<<<2 * G, kBlock, 0, st>>>(a); note_launch();
-    scan(a.ws.pair_cont, a.ws.counters + kNPairs, caps->pair_capacity, a.ws.scan_tmp, a.ws.counters + kNContacts, st);
-    k_check<<<1, 1, 0, st>>>(a.ws.counters, kNContacts, caps->contact_capacity, RB_STATUS_CONTACT_OVERFLOW, out->status); note_launch();
+    scan_total(a.ws.pair_cont, a.ws.counters + kNPairs, caps->pair_capacity, a.ws.scan_tmp,
+               ScanTotal{a.ws.counters, kNContacts, caps->contact_capacity, RB_STATUS_CONTACT_OVERFLOW, out->status}, st);
     k_emit<<<2 * G, kBlock, 0, st>>>(a); note_launch();
     prof_mark(prof, 4, st);
     // contact problem
@@ -3616,7 +3678,7 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
         k_hinge_lists<<<blocks_for(bd->n_scenes, 64), 64, 0, st>>>(a); note_launch();
         k_hinges<<<blocks_for(bd->n_hinges, 128), 128, 0, st>>>(a); note_launch();
     }
-    scan(a.ws.bc_ptr, nullptr, N, a.ws.scan_tmp, nullptr, st);
+    scan(a.ws.bc_ptr, nullptr, N, a.ws.scan_tmp, st);
     k_body_contacts_fill<<<G, 256, 0, st>>>(a); note_launch();
     k_body_contacts_sort<<<blocks_for(32 * (int64_t)N, 128), 128, 0, st>>>(a); note_launch();
     // solve, integrate, post-stabilise
@@ -3632,8 +3694,8 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     // a scene that has an SM to itself takes as many warps as the registers allow (255 a thread), so that wide levels
     // and the rebuilds of w have them; more scenes than SMs share them, two or four blocks to an SM
     const int solve_threads = bd->n_scenes <= 148 ? kSolveBlock : bd->n_scenes <= 2 * 148 ? kSolveBlock / 2 : kSolveBlock / 4;
-    k_fp32_classes<<<1, 1024, 0, st>>>(a, small_slab, mid_slab); note_launch();
     if (pr->precision != RB_PRECISION_FP64) {
+        k_fp32_classes<<<1, 1024, 0, st>>>(a, small_slab, mid_slab); note_launch();
         // FP32 phase, four size classes side by side: warp teams with small slabs (28 KB unless tuned), warp
         // teams with mid slabs (56 KB), block teams with 224 KB (1 per SM), and 512-thread block teams for the
         // scenes beyond that, whose contact rows stay in L2
@@ -3671,9 +3733,8 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
         k_post_apply<<<blocks_for(32 * ((N + 4) / (int64_t)5), 128), 128, 0, st>>>(a); note_launch();
     }
     if (prof) { k_body_energy<<<blocks_for(N, 128), 128, 0, st>>>(a); note_launch(); }
-    k_scene_summary<<<blocks_for(32 * (int64_t)bd->n_scenes, 128), 128, 0, st>>>(a); note_launch();
-    k_cache_store<<<G, 256, 0, st>>>(a); note_launch();
-    k_finish<<<1, 1, 0, st>>>(a); note_launch();
+    const int summary_blocks = blocks_for(32 * (int64_t)bd->n_scenes, 128);
+    k_outputs<<<summary_blocks + G, 128, 0, st>>>(a, summary_blocks); note_launch();
     prof_mark(prof, 6, st);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(RB_ERR_CUDA, std::string("rb_step: ") + cudaGetErrorString(e));

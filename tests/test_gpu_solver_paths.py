@@ -116,3 +116,31 @@ def test_deep_overlaps(oracle_lib, slices, resolution):
     o = oracle_lib.OracleScene(arrays)
     rp = W.make_rb_params(W.params_from_vector(arrays["params"]))
     _compare(world, {1: o}, [1], rp, 2, capacity=1 << 15)
+
+
+@pytest.mark.parametrize("count", [1, 3, 4096, 4097, 16383, 16384, 16385, 40000])
+def test_scan_sizes(count):
+    """Topology prefix sums (device scans) of as many bodies as one block scans in a round, one more, and of both
+    scan variants, against NumPy's."""
+    import ctypes
+    import torch
+    from rainbow_b200 import _native as N
+    rng = np.random.default_rng(count)
+    nv, nt = rng.integers(4, 400, 5), rng.integers(4, 900, 5)
+    shape = rng.integers(0, 5, count).astype(np.int32)
+    off = lambda n: torch.from_numpy(np.concatenate([[0], np.cumsum(n)]).astype(np.int32)).cuda()  # noqa: E731
+    v_off, t_off, t_shape = off(nv), off(nt), torch.from_numpy(shape).cuda()
+    sh, bd = N.RbShapes(), N.RbBodies()
+    sh.n_shapes, sh.v_off, sh.t_off = 5, v_off.data_ptr(), t_off.data_ptr()
+    sums = [np.concatenate([[0], np.cumsum(n[shape])]) for n in (nv, nt, (nt + 31) // 32)]
+    bd.n_bodies, bd.n_scenes, bd.shape = count, 1, t_shape.data_ptr()
+    bd.n_body_vertices, bd.n_body_triangles, bd.n_clusters = (int(s[-1]) for s in sums)
+    out = [torch.empty(count + 1, dtype=torch.int32, device="cuda") for _ in range(3)]
+    owners = [torch.empty(int(s[-1]), dtype=torch.int32, device="cuda") for s in sums]
+    for name, t in zip(("body_v0", "body_t0", "body_c0", "vert_body", "tri_body", "clu_body"), out + owners):
+        setattr(bd, name, t.data_ptr())
+    scratch = torch.empty(N.RB_TOPOLOGY_SCRATCH_BYTES, dtype=torch.uint8, device="cuda")
+    N.check(N.load().rb_build_topology(ctypes.byref(sh), ctypes.byref(bd), scratch.data_ptr(), scratch.numel(),
+                                       torch.cuda.current_stream().cuda_stream), "rb_build_topology")
+    for got, want in zip(out, sums):
+        np.testing.assert_array_equal(got.cpu().numpy(), want)
