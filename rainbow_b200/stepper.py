@@ -125,9 +125,8 @@ class GpuStepper:
         world = self._world_for(engine)
         rp = _step_params(engine.params, dt, self.termination, self.residual_tolerance, profiling_on)
         _check_status(world.step(rp))
-        x, u = world.state()
+        x, u, c = world.state_and_contacts()
         engine_io.write_back(engine, x, u)
-        c = world.contacts()
         bodies = list(engine.bodies.values())
         engine.contact_points = ContactPoints(bodies, c["ids"], c["p"], c["n"], c["g"], _contact_factory(engine))
         if profiling_on:

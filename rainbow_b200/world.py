@@ -391,7 +391,7 @@ class DeviceWorld:
         for _ in range(max_retries):
             self.t_status.zero_()
             self.launch(rb_params)
-            status = int(self.t_status[0].item())
+            status, self.step_contacts = self.t_status[:2].tolist()   # one read-back for the status and the count
             grow = status & (N.STATUS_PAIR_OVERFLOW | N.STATUS_ITEM_OVERFLOW | N.STATUS_CONTACT_OVERFLOW)
             if not grow:
                 if status & N.STATUS_MESH_TOO_LARGE:
@@ -415,10 +415,36 @@ class DeviceWorld:
 
     def contacts(self):
         """Host copies of the contact outputs of the last step (global body indices)."""
-        K = min(self.n_contacts_total(), self.caps.contact_capacity)
-        return dict(ids=self.t_cids[:2 * K].view(K, 2).cpu().numpy(), p=self.t_cp[:3 * K].view(K, 3).cpu().numpy(),
-                    n=self.t_cn[:3 * K].view(K, 3).cpu().numpy(), g=self.t_cg[:K].cpu().numpy(),
-                    sol=self.t_csol[:4 * K].cpu().numpy())
+        return self._read_back([], self.n_contacts_total())[1]
+
+    def state_and_contacts(self):
+        """(x, u, contacts) after a :meth:`step`: what :meth:`state` and :meth:`contacts` return, read back with one wait
+        (the step's own read of its status gave the number of contacts)."""
+        (x, u), contacts = self._read_back([self.t_x, self.t_u], self.step_contacts)
+        return x.reshape(-1, 7), u.reshape(-1, 6), contacts
+
+    def _read_back(self, tensors, n_contacts):
+        """Host copies of `tensors` and of the first n_contacts contacts, through pinned staging that is kept: seven
+        copies and one wait instead of a wait for each (~16 us each, of the ~460 us of a small scene's step)."""
+        K = min(n_contacts, self.caps.contact_capacity)
+        parts = list(tensors) + [self.t_cids[:2 * K], self.t_cp[:3 * K], self.t_cn[:3 * K], self.t_cg[:K],
+                                 self.t_csol[:4 * K]]
+        sizes = [-(-t.numel() * t.element_size() // 64) * 64 for t in parts]
+        total = sum(sizes)
+        stage = getattr(self, "h_stage", None)
+        if stage is None or stage.numel() < total:
+            stage = self.h_stage = torch.empty(total + total // 2 + 4096, dtype=torch.uint8, pin_memory=True)
+        host, at = [], 0
+        for t, size in zip(parts, sizes):
+            h = stage[at:at + t.numel() * t.element_size()].view(t.dtype)
+            if t.numel():
+                h.copy_(t, non_blocking=True)
+            host.append(h)
+            at += size
+        torch.cuda.current_stream(self.device).synchronize()
+        out = [h.numpy().copy() for h in host]
+        ids, p, n, g, sol = out[-5:]
+        return out[:-5], dict(ids=ids.reshape(K, 2), p=p.reshape(K, 3), n=n.reshape(K, 3), g=g, sol=sol)
 
     def _pinned(self):
         if not hasattr(self, "h_x"):
