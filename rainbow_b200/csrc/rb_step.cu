@@ -2393,8 +2393,15 @@ struct S32Scene {
     char* bptr;    // per slot: start of its contact list in blist (n_free + 1)
     char* blist;   // per slot, its contacts in ascending order: level-order position << 1 | side (2K)
     char* steps;   // the sweep's steps: first position | contacts << 16 | flags; over pos, once that is used
+    char* x;       // the impulses: float4s `xs` bytes apart (in the records, or, with the rows in a ring, on their own)
+    char* ring;    // room for kRingSteps steps' records, when the rows come from L2 through it, else null
+    uint32_t xs;
     int K, n_free, n_steps, warps;
 };
+// The rows of a scene too large for a slab stay in L2.  When the slab has room for them beside the bodies, the impulses
+// and the indices, they come through a ring of six steps' records, copied four steps ahead (s32_sweep_ring).
+constexpr int kRingSteps = 6, kRingAhead = 4, kRingWarps = 4;
+constexpr int kRingSlot = 8 * kRingWarps * (int)sizeof(float) * kS32Floats;
 constexpr uint32_t kStep32Ends = 1u << 31, kStep32Wide = 1u << 30;
 constexpr uint32_t kStep32Turns = 1u << 29;   // the next step is of the other width
 __host__ __device__ inline size_t s32_align(size_t v) { return (v + 15) & ~size_t(15); }
@@ -2410,10 +2417,16 @@ __host__ __device__ inline size_t s32_bytes(int K, int nb, bool in_l2 = false, b
 }
 // body records a scene can need
 __host__ __device__ inline int s32_records(int K, int nb) { return nb < 2 * K ? nb : 2 * K; }
+// shared memory of a scene whose rows come through the ring (the other arrays as with in_l2, and the impulses)
+__host__ __device__ inline size_t s32_ring_bytes(int K, int nr) {
+    return s32_align(sizeof(float) * (size_t)nr * kS32BodyFloats) + s32_align(sizeof(uint32_t) * (size_t)K) +
+           s32_align(sizeof(uint16_t) * (size_t)(nr + 1)) + s32_align(4 * sizeof(float) * (size_t)K) +
+           (size_t)kRingSteps * kRingSlot;
+}
 // with l2, the contact rows, positions, steps and body lists go to the workspace; with bodies_global the body
 // records too (the scene's team is the only reader and writer, so block barriers keep them consistent)
 __device__ __forceinline__ S32Scene s32_carve(char* base, int K, int nr, const StepArgs* l2 = nullptr, int c0 = 0,
-                                              int s = 0, bool bodies_global = false, int b0 = 0) {
+                                              int s = 0, bool bodies_global = false, int b0 = 0, bool ring = false) {
     S32Scene f;
     size_t o = 0;
     auto take = [&](size_t bytes) { char* p = base + o; o += s32_align(bytes); return p; };
@@ -2423,10 +2436,13 @@ __device__ __forceinline__ S32Scene s32_carve(char* base, int K, int nr, const S
     f.lohi = take(sizeof(uint32_t) * (size_t)K);
     // positions, then room of their size: together a word per contact for the steps (in L2: the level cursors)
     f.pos = l2 ? reinterpret_cast<char*>(l2->ws.pos32 + c0) : take(sizeof(uint16_t) * (size_t)K);
-    take(sizeof(uint16_t) * (size_t)(K + 1));
+    if (!ring) take(sizeof(uint16_t) * (size_t)(K + 1));
     f.steps = l2 ? reinterpret_cast<char*>(l2->ws.lev_cur + c0 + s) : f.pos;
     f.bptr = take(sizeof(uint16_t) * (size_t)(nr + 1));
     f.blist = l2 ? reinterpret_cast<char*>(l2->ws.blist32 + 2 * (size_t)c0) : take(sizeof(uint32_t) * 2 * (size_t)K);
+    f.x = ring ? take(4 * sizeof(float) * (size_t)K) : f.c + 192;
+    f.xs = ring ? 16u : (uint32_t)sizeof(float) * kS32Floats;
+    f.ring = ring ? take((size_t)kRingSteps * kRingSlot) : nullptr;
     f.K = K;
     f.n_free = f.n_steps = 0;
     f.warps = 1;
@@ -2542,7 +2558,7 @@ __device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const Sce
             v.x = (float)J[j_at(q, 9)]; v.y = (float)J[j_at(q, 10)]; v.z = (float)J[j_at(q, 11)];
             v.w = (float)a.ws.mu[k];
         } else {
-            o[q] = (float)a.ws.x[4 * k + q];
+            reinterpret_cast<float*>(f.x + (size_t)f.xs * i)[q] = (float)a.ws.x[4 * k + q];
             continue;
         }
         reinterpret_cast<float4*>(o)[q] = v;
@@ -2590,7 +2606,7 @@ __device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const Sce
     }
     g.sync();   // pos used: the steps take its room
     const int* ptr = a.ws.lev_ptr + R.c0 + s;
-    f.warps = g.size() > 32 ? s32_warps(ptr, L, g.size() >> 5, in_l2) : 1;
+    f.warps = f.ring ? kRingWarps : g.size() > 32 ? s32_warps(ptr, L, g.size() >> 5, in_l2) : 1;
     uint32_t* steps = reinterpret_cast<uint32_t*>(f.steps);
     f.n_steps = sweep_steps(g, ptr, L, in_l2 ? 0 : 8 * f.warps, in_l2 ? 8 * f.warps : 32 * f.warps, [&](int at, int start, int count, bool ends, bool wide) {
         steps[at] = (uint32_t)start | ((uint32_t)count << 16) | (ends ? kStep32Ends : 0u) | (wide && !in_l2 ? kStep32Wide : 0u);
@@ -2606,28 +2622,42 @@ __device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const Sce
 // summed in ascending order
 template <class P, class G>
 __device__ __noinline__ void s32_rebuild_w(const G g, const S32Scene f) {
-    const P c(f.c), body(f.body), bptr(f.bptr), blist(f.blist);
+    const P c(f.c), body(f.body), bptr(f.bptr), blist(f.blist), xp(f.x);
     const int ang = g.rank() & 1;
     for (int i = g.rank() >> 1; i < f.n_free; i += g.size() >> 1) {
         uint32_t e = (bptr + 2u * i).u16();
         const uint32_t e1 = (bptr + (2u * i + 2u)).u16();
         const P B = body + kB32 * i;
         float S[3] = {0.f, 0.f, 0.f};
-        uint32_t code = (blist + 4u * e).u32();
-        for (; e < e1; ++e) {
+        float4 v[2][4], x[2];   // two contacts at a time: their loads are under way together
+        auto fetch = [&](int t, uint32_t code) {
             const uint32_t side = code & 1u;
-            const P rec = c + kC32 * (code >> 1);
-            const P col = rec + (ang ? 64u + 64u * side : 0u);
-            const float4 v0 = col.f4(), v1 = (col + 16u).f4(), v2 = (col + 32u).f4(), v3 = (col + 48u).f4();
-            const float4 x = (rec + kX32).f4();
-            code = (blist + 4u * min(e + 1u, e1 - 1u)).u32();
+            const P col = c + (kC32 * (code >> 1) + (ang ? 64u + 64u * side : 0u));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[t][k] = (col + 16u * k).f4();
+            x[t] = (xp + f.xs * (code >> 1)).f4();
             const float sg = !ang && side ? -1.0f : 1.0f;   // lin_hi = -lin_lo
-            const float x0 = sg * x.x, x1 = sg * x.y, x2 = sg * x.z, x3 = sg * x.w;
-            S[0] = fmaf(v0.x, x0, S[0]); S[1] = fmaf(v0.y, x0, S[1]); S[2] = fmaf(v0.z, x0, S[2]);
-            S[0] = fmaf(v1.x, x1, S[0]); S[1] = fmaf(v1.y, x1, S[1]); S[2] = fmaf(v1.z, x1, S[2]);
-            S[0] = fmaf(v2.x, x2, S[0]); S[1] = fmaf(v2.y, x2, S[1]); S[2] = fmaf(v2.z, x2, S[2]);
-            S[0] = fmaf(v3.x, x3, S[0]); S[1] = fmaf(v3.y, x3, S[1]); S[2] = fmaf(v3.z, x3, S[2]);
+            x[t] = make_float4(sg * x[t].x, sg * x[t].y, sg * x[t].z, sg * x[t].w);
+        };
+        auto add = [&](int t) {
+            const float xs[4] = {x[t].x, x[t].y, x[t].z, x[t].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                S[0] = fmaf(v[t][k].x, xs[k], S[0]);
+                S[1] = fmaf(v[t][k].y, xs[k], S[1]);
+                S[2] = fmaf(v[t][k].z, xs[k], S[2]);
+            }
+        };
+        uint32_t code0 = (blist + 4u * e).u32(), code1 = (blist + 4u * min(e + 1u, e1 - 1u)).u32();
+        for (; e + 1u < e1; e += 2u) {
+            fetch(0, code0);
+            fetch(1, code1);
+            code0 = (blist + 4u * min(e + 2u, e1 - 1u)).u32();
+            code1 = (blist + 4u * min(e + 3u, e1 - 1u)).u32();
+            add(0);
+            add(1);
         }
+        if (e < e1) { fetch(0, code0); add(0); }
         const float4 I0 = (B + 32u).f4();
         const float2 I1 = (B + 48u).f2();
         if (ang) {
@@ -2659,7 +2689,7 @@ __device__ __forceinline__ void quad_gather(float z, float* o) {
 template <class P, class G>
 __device__ __noinline__ float s32_residual(const G g, const S32Scene f) {
     s32_rebuild_w<P>(g, f);
-    const P c(f.c), body(f.body), lohi(f.lohi);
+    const P c(f.c), body(f.body), lohi(f.lohi), xp(f.x);
     const int q = g.rank() & 3, nslot = g.size() >> 2;
     float m = 0.0f, xm = 0.0f;
     for (int i0 = 0; i0 < f.K; i0 += nslot) {
@@ -2669,7 +2699,7 @@ __device__ __noinline__ float s32_residual(const G g, const S32Scene f) {
         const P Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
         const float4 r0 = row.f4(), r1 = (row + 64u).f4(), r2 = (row + 128u).f4();
         const float4 l0 = Bl.f4(), l1 = (Bl + 16u).f4(), h0 = Bh.f4(), h1 = (Bh + 16u).f4();
-        const float x = (rec + kX32 + 4u * q).f1();
+        const float x = (xp + (f.xs * i + 4u * q)).f1();
         float z[4];
         const float zq = x - r1.w * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
         quad_gather(zq, z);
@@ -2867,11 +2897,119 @@ __device__ __noinline__ void s32_sweep(const G g, const S32Scene f, float rscale
     }
 }
 
+// The narrow steps of s32_sweep for a scene whose rows come through the ring: a step's records, contiguous in level
+// order, are copied into its slot four steps ahead by a warp of their own (asynchronous 16-byte copies, one group a
+// step; at a step's end the copies of the next but one are waited for, and the step's barrier shows them to all).  With the rows read from L2 by the lanes that need them a
+// step is bound by L2's latency and the uncoalesced loads: 200 sweeps and their tests over 1565 contacts took 9228 us,
+// through the ring 6376 (copied by the sweeping warps themselves 8400).
+__device__ __noinline__ void s32_sweep_ring(const S32Scene f, float rscale, int n_sweeps) {
+    const ShPtr body(f.body), lohi(f.lohi), xp(f.x), ring(f.ring);
+    const GlPtr steps(f.steps);
+    const SubGroup g{32 * (kRingWarps + 1)};
+    const int rank = threadIdx.x, q = rank & 3, slot = rank >> 2, last = f.n_steps - 1;
+    const bool linear = q < 2;
+    const uint32_t hi_shift = (q & 1) ? 16u : 0u;
+    const uint32_t fixed_bit = 0x8000u << hi_shift;
+    const uint32_t part = linear ? 0u : 16u;
+    const uint32_t col = linear ? 0u : 64u * (uint32_t)(q - 1);
+    const float sg = q == 1 ? -1.0f : 1.0f;
+    auto step = [&](int j) { return (steps + 4u * j).u32(); };
+    auto after = [&](int j) { return j < last ? j + 1 : 0; };
+    auto at = [&](uint32_t st) { return min((int)(st & 0x7fffu) + slot, f.K - 1); };
+    auto record = [&](int place) { return ring + ((uint32_t)kRingSlot * place + kC32 * slot); };
+    auto copy = [&](uint32_t st, int place) {   // a step's records to its slot, 13 pieces each
+        const char* from = f.c + (size_t)kC32 * (st & 0x7fffu);
+        const int pieces = 13 * (int)((st >> 16) & 0x1fffu);
+        const uint32_t to = (ring + (uint32_t)kRingSlot * place).p;
+        for (int t = threadIdx.x & 31; t < pieces; t += 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16u * t), "l"(from + 16 * (size_t)t) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto next_place = [&](int p) { return p + 1 < kRingSteps ? p + 1 : 0; };
+    const int total = n_sweeps * f.n_steps;
+    if (rank >= 32 * kRingWarps) {   // the copying warp
+        int ja = 0, place = 0;
+        for (int k = 0; k < kRingAhead; ++k) { copy(step(ja), place); ja = after(ja); place = next_place(place); }
+        asm volatile("cp.async.wait_group 2;" ::: "memory");
+        g.sync();
+        for (int left = total; left > 0; --left) {
+            copy(step(ja), place);
+            ja = after(ja);
+            place = next_place(place);
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            g.sync();
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        return;
+    }
+    g.sync();
+    int place1 = 1;   // slot of the next step
+    uint32_t st0 = step(0), st1 = step(after(0));
+    int j2 = after(after(0));
+    int i0 = at(st0), i1 = at(st1);
+    uint32_t lh = (lohi + 4u * i0).u32(), lh_next = (lohi + 4u * i1).u32();
+    ShPtr rec = record(0);
+    float4 r0 = (rec + 16u * q).f4(), r1 = (rec + (64u + 16u * q)).f4(), r2 = (rec + (128u + 16u * q)).f4();
+    float4 x = (xp + 16u * i0).f4();
+    float xq = (xp + (16u * i0 + 4u * q)).f1();
+#pragma unroll 1
+    for (int left = total; left > 0; --left) {
+        const ShPtr Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
+        const float4 l0 = Bl.f4(), h0 = Bh.f4(), l1 = (Bl + 16u).f4(), h1 = (Bh + 16u).f4();
+        const float zq = xq - rscale * r1.w * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
+        float z[4];
+        quad_gather(zq, z);
+        const ShPtr cl = rec + col;
+        const float4 v0 = cl.f4(), v1 = (cl + 16u).f4(), v2 = (cl + 32u).f4(), v3 = (cl + 48u).f4();
+        const ShPtr B = body + kB32 * ((lh >> hi_shift) & 0x7fffu);
+        const float4 own = (B + part).f4();
+        const float4 I0 = (B + 32u).f4();
+        const float2 I1 = (B + 48u).f2();
+        const float xn = fmaxf(z[0], 0.0f);
+        const float radius = r2.w * xn;
+        const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
+        float scale = sqr > radius * radius ? radius * rsqrtf(sqr) : 1.0f;
+        if (xn <= 0.0f) scale = 0.0f;
+        const uint32_t st2 = step(j2);
+        j2 = after(j2);
+        const ShPtr rec_next = record(place1);
+        r0 = (rec_next + 16u * q).f4(); r1 = (rec_next + (64u + 16u * q)).f4(); r2 = (rec_next + (128u + 16u * q)).f4();
+        const float f1 = z[1] * scale, f2 = z[2] * scale, f3 = z[3] * scale;
+        const float d0 = xn - x.x, d1 = f1 - x.y, d2 = f2 - x.z, d3 = f3 - x.w;
+        const float yq = q == 0 ? xn : zq * scale;
+        const float m = sg * own.w;
+        const float wxx = linear ? m : I0.x, wxy = linear ? 0.0f : I0.y, wxz = linear ? 0.0f : I0.z;
+        const float wyy = linear ? m : I0.w, wyz = linear ? 0.0f : I1.x, wzz = linear ? m : I1.y;
+        const float S0 = fmaf(v3.x, d3, fmaf(v2.x, d2, fmaf(v1.x, d1, v0.x * d0)));
+        const float S1 = fmaf(v3.y, d3, fmaf(v2.y, d2, fmaf(v1.y, d1, v0.y * d0)));
+        const float S2 = fmaf(v3.z, d3, fmaf(v2.z, d2, fmaf(v1.z, d1, v0.z * d0)));
+        const float4 n = make_float4(own.x + fmaf(wxx, S0, fmaf(wxy, S1, wxz * S2)),
+                                     own.y + fmaf(wxy, S0, fmaf(wyy, S1, wyz * S2)),
+                                     own.z + fmaf(wxz, S0, fmaf(wyz, S1, wzz * S2)), own.w);
+        const bool mine = slot < (int)((st0 >> 16) & 0x1fffu);
+        if (mine && !(lh & fixed_bit)) (B + part).set(n);
+        if (mine) (xp + (16u * i0 + 4u * q)).set(yq);
+        // after the stores: a scene of one step sweeps the same contacts again
+        x = (xp + 16u * i1).f4();
+        xq = (xp + (16u * i1 + 4u * q)).f1();
+        g.sync();   // and the next but one step's rows are there
+        st0 = st1; st1 = st2;
+        place1 = next_place(place1);
+        rec = rec_next;
+        lh = lh_next;
+        i0 = i1;
+        i1 = at(st1);
+        lh_next = (lohi + 4u * i1).u32();
+    }
+}
+
 // n_sweeps sweeps by as many of the team's warps as the scene's levels keep busy
 template <class P, class G>
 __device__ __forceinline__ void s32_sweep_team(const G& g, const S32Scene& f, float rscale, int n_sweeps) {
     if constexpr (std::is_same_v<G, BlockGroup>) {
-        if (f.warps == 1) {
+        if (std::is_same_v<P, GlPtr> && f.ring) {
+            if (threadIdx.x < 32 * (kRingWarps + 1)) s32_sweep_ring(f, rscale, n_sweeps);
+        } else if (f.warps == 1) {
             if (threadIdx.x < 32) s32_sweep<P>(WarpGroup{}, f, rscale, n_sweeps);
         } else if ((int)threadIdx.x < 32 * f.warps) {
             s32_sweep<P>(SubGroup{32 * f.warps}, f, rscale, n_sweeps);
@@ -2921,7 +3059,7 @@ __device__ __noinline__ void s32_sweep_jacobi(const G g, const S32Scene f, float
 template <class P, class G>
 __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, const SceneRange& R, const S32Scene& f,
                                               bool correct = true) {
-    const P c(f.c), body(f.body), lohi(f.lohi), bptr(f.bptr), blist(f.blist);
+    const P c(f.c), body(f.body), lohi(f.lohi), bptr(f.bptr), blist(f.blist), xp(f.x);
     const int K = f.K;
     const int* order = a.ws.lev_order + R.c0;
     double* w64 = a.ws.w + 6 * (size_t)R.b0;   // by slot; the scene's FP64 accumulators, unused until the FP64 solve
@@ -2933,7 +3071,7 @@ __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, con
             const uint32_t code = (blist + 4u * e).u32();
             double W[4];
             w_column(a.ws.WJT, order[code >> 1], 6 * (int)(code & 1u) + d, W);
-            const float4 x = (c + kC32 * (code >> 1) + kX32).f4();
+            const float4 x = (xp + f.xs * (code >> 1)).f4();
             acc = fma(W[0], (double)x.x, acc);
             acc = fma(W[1], (double)x.y, acc);
             acc = fma(W[2], (double)x.z, acc);
@@ -2967,7 +3105,7 @@ __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, con
             const float v32 = s32_jw(r0, (row + 64u).f4(), (row + 128u).f4(), Bl.f4(), (Bl + 16u).f4(), Bh.f4(), (Bh + 16u).f4()) + r0.w;
             (row + 12u).set(r0.w + (float)(v64 - (double)v32));
         }
-        const double x = (double)(rec + kX32 + 4u * q).f1();
+        const double x = (double)(xp + (f.xs * i + 4u * q)).f1();
         const double zq = x - v64 / a.ws.diag[4 * k + q];
         double z[4];
         quad_gather(zq, z);
@@ -3125,14 +3263,16 @@ __global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve
             if (bytes <= lo_bytes || bytes > slab) continue;
         }
         const double t0 = a.pr.profiling ? device_us() : 0.0;
-        S32Scene f = s32_carve(my_slab, K, nr, kL2 ? &a : nullptr, R.c0, s, bodies_global, R.b0);
+        const bool ring = kL2 && !jacobi && s32_ring_bytes(K, nr) <= slab;
+        S32Scene f = s32_carve(my_slab, K, nr, kL2 ? &a : nullptr, R.c0, s, bodies_global, R.b0, ring);
         // scratch for the level relaxation: the rows' room of the slab, or with rows in L2 what the slab has left
         int16_t* scratch = nullptr;
         if (!kL2) {   // a contact record's bytes per contact there, more than s32_level_scratch needs
             scratch = reinterpret_cast<int16_t*>(f.c);
         } else {
             const size_t off = (s32_bytes(K, nr, true, bodies_global) + 15) & ~size_t(15);
-            if (off + s32_level_scratch(K) <= slab) scratch = reinterpret_cast<int16_t*>(my_slab + off);
+            if (ring && s32_level_scratch(K) <= (size_t)kRingSteps * kRingSlot) scratch = reinterpret_cast<int16_t*>(f.ring);
+            else if (!ring && off + s32_level_scratch(K) <= slab) scratch = reinterpret_cast<int16_t*>(my_slab + off);
         }
         const int L = s32_load(a, g, R, s, f, coloured, kL2, scratch);
         if (g.rank() == 0) a.ws.nlev[s] = L;
@@ -3187,7 +3327,7 @@ __global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve
         for (int t = g.rank(); t < 4 * K; t += g.size()) {   // back to contact order
             const int i = t >> 2, q = t & 3;
             const size_t k4 = 4 * (size_t)a.ws.lev_order[R.c0 + i] + q;
-            const double xv = (double)(P(f.c) + (kC32 * i + kX32 + 4u * q)).f1();
+            const double xv = (double)(P(f.x) + (f.xs * i + 4u * q)).f1();
             a.ws.x[k4] = xv;
             if (finished) a.out.contact_sol[k4] = xv;
         }

@@ -144,3 +144,31 @@ def test_scan_sizes(count):
                                        torch.cuda.current_stream().cuda_stream), "rb_build_topology")
     for got, want in zip(out, sums):
         np.testing.assert_array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("bodies", [700, 1500, 2600])   # rows through the ring, and too many bodies for it
+@pytest.mark.parametrize("scheme", ["rigid_gauss_seidel", "parallel_gauss_seidel"])
+def test_large_fp32_scenes_match_their_fp64_solve(bodies, scheme):
+    """A pile too large for a slab, its rows through the ring or, beyond that, straight from L2: the FP32 solve of a
+    step alone in the batch and beside small scenes is the same to the bit, and its impulses give the FP64 residual
+    the solver reports (FP32 rounding of a problem with impulses up to 1e4: 1e-3 of the largest velocity)."""
+    from rainbow_b200 import scenes, world as W
+    big = scenes.batch_arrays(n_scenes=1, seed=3, pool=4, body_range=(bodies, bodies), resolution=16, device="cuda:0",
+                              ground=60.0)[0][0]
+    small, params = scenes.batch_arrays(n_scenes=3, seed=4, pool=4, body_range=(8, 30), resolution=16, device="cuda:0")
+    for a in [big] + small:
+        a["body_r"] = np.concatenate([a["body_r"][:1], a["body_r"][1:] * [0.62, 0.5, 0.62]])
+    kw = dict(scheme=scheme, termination="residual_fixed_r", residual_interval=4, residual_tolerance=1e-6)
+    worlds = [W.DeviceWorld([big], max_iterations=200), W.DeviceWorld(small[:1] + [big] + small[1:], max_iterations=200),
+              W.DeviceWorld([big], max_iterations=200)]
+    for w, precision in zip(worlds, ("fp32_refine", "fp32_refine", "fp64")):
+        rp = W.make_rb_params(params, precision=precision, **kw)
+        rp.max_iterations = 200
+        assert w.step(rp) == 0
+    st = [worlds[0].stats()[0], worlds[1].stats()[1], worlds[2].stats()[0]]
+    assert st[0].n_contacts == st[1].n_contacts == st[2].n_contacts > 500
+    assert st[0].fp32_sweeps == st[1].fp32_sweeps > 0 and st[0].residual == st[1].residual
+    b0, b1 = worlds[1].scene_start[1], worlds[1].scene_start[2]
+    u = [worlds[0].state()[1], worlds[1].state()[1][b0:b1], worlds[2].state()[1]]
+    np.testing.assert_array_equal(u[0], u[1])
+    assert np.max(np.abs(u[0] - u[2])) <= 1e-3 * max(1.0, np.max(np.abs(u[2])))
