@@ -1297,7 +1297,8 @@ struct Solve64 {
     const int32_t* bc_list;
     const double *J, *WJT, *mu;
     int K, n_touched, n_steps;
-    int warps;       // warps that sweep (a block's; 1 for a warp)
+    int warps;       // warps that sweep a step (a block's; 1 for a warp)
+    bool turns;      // two groups of them by turns
     bool w_shared;   // w lies in shared memory
 };
 constexpr int kMetaIdle = 4;
@@ -1345,11 +1346,12 @@ __device__ __forceinline__ int scene_touched(const StepArgs& a, const G& g, cons
     return n;
 }
 
-// Warps that sweep a scene, eight contacts each: the number with the least cost over the scene's levels (ptr), a step
-// (a run of a level's contacts that the warps take at once) costing 1150 cycles with one warp and 100 more for every
-// further one: their FP64 and load instructions hold one another up even where they have no contact (64-box
-// lattice: 1420 with three; 4096-body lattice: 1870 with eight).  Every warp of the group counts for itself.
-__device__ __forceinline__ int sweep_warps(const int* ptr, int L, int max_warps) {
+// Warps that sweep a scene, eight contacts each, and whether two groups of them do so by turns: the choice with the least
+// cost over the scene's levels (ptr).  A step (a run of a level's contacts that the warps take at once) costs 1150 cycles
+// with one warp, or 750 by turns, and 100 more for every further warp: their FP64 and load instructions hold one another
+// up even where they have no contact (64-box lattice: 1420 with three; 4096-body lattice: 1870 with eight).  Every warp
+// of the block counts for itself.
+__device__ __forceinline__ int sweep_warps(const int* ptr, int L, int max_warps, bool& turns) {
     int steps[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int l = threadIdx.x & 31; l < L; l += 32) {
         const int n = ptr[l + 1] - ptr[l];
@@ -1357,10 +1359,13 @@ __device__ __forceinline__ int sweep_warps(const int* ptr, int L, int max_warps)
         for (int w = 0; w < 8; ++w) steps[w] += (n + 8 * w + 7) / (8 * w + 8);
     }
     int best = 1, cost = INT_MAX;
+    turns = false;
 #pragma unroll
     for (int w = 0; w < 8; ++w) {
-        const int c = __reduce_add_sync(0xffffffffu, steps[w]) * (23 + 2 * w);
-        if (w < max_warps && c < cost) { cost = c; best = w + 1; }
+        const int n = __reduce_add_sync(0xffffffffu, steps[w]);
+        const int together = n * (23 + 2 * w), by_turns = n * (15 + 2 * w);
+        if (w < max_warps && together < cost) { cost = together; best = w + 1; turns = false; }
+        if (2 * w + 1 < max_warps && by_turns < cost) { cost = by_turns; best = w + 1; turns = true; }
     }
     return best;
 }
@@ -1418,9 +1423,11 @@ __device__ __forceinline__ Solve64 scene_setup64(const StepArgs& a, const G& g, 
     int2* steps = reinterpret_cast<int2*>(meta + v.K);
     v.steps = steps;
     const int* ptr = a.ws.lev_ptr + R.c0 + s;
-    v.warps = g.size() > 32 ? sweep_warps(ptr, L, g.size() >> 5) : 1;
+    v.warps = 1;
+    v.turns = false;
+    if (g.size() > 32) v.warps = sweep_warps(ptr, L, g.size() >> 5, v.turns);
     v.n_steps = sweep_steps(g, ptr, L, 8 * v.warps, 8 * v.warps, [&](int at, int start, int count, bool ends, bool) {
-        steps[at] = make_int2(start, count | (ends ? kStepEnds : 0));
+        steps[at] = make_int2(start, count | (ends && !v.turns ? kStepEnds : 0));
     });
     g.sync();
     return v;
@@ -1628,6 +1635,77 @@ __device__ __noinline__ double gs_sweep_quads(const G g, const Solve64 v, int n_
     return m;
 }
 
+// The same sweep by two groups of `warps` warps that take the steps by turns: while one computes a step, the other loads all
+// that its next step's contact does not have from w, so only the chain itself lies between the barriers: the accumulators'
+// loads, the row products, the prox, the update and its stores.  A group that has stored its step's w arrives at that
+// step's barrier and goes on to its loads; the other waits there.  (32-box tower 883 -> 631 us a solve of 100 sweeps,
+// 64-box lattice 1150 -> 719, 64 piles 8616 -> 5297; the 4096-body lattice, of which eight warps took a step at once,
+// 2306 -> 2053 with two groups of four.)
+template <bool kShared>
+__device__ __noinline__ double gs_sweep_turns(const Solve64 v, int n_steps, const double* b, const double* r,
+                                              const double* x, double* y, bool normal_only) {
+    const W64<kShared> w(v.w);
+    const int half = 32 * v.warps, group = (int)threadIdx.x >= half, rank = threadIdx.x - group * half;
+    const int q = rank & 3, slot = rank >> 2;
+    const double* J = v.J + 2 * q;
+    const double* WJT = v.WJT + 2 * q;
+    b += q; r += q; y += q;
+    const double* xs = x + q;
+    double m = 0.0;
+    auto meta = [&](int j) {
+        const int2 st = v.steps[min(j, n_steps - 1)];
+        int4 me = v.meta[min(st.x + slot, v.K - 1)];
+        if (slot >= st.y) me.w = kMetaIdle;
+        return me;
+    };
+    int4 next = meta(group);
+#pragma unroll 1
+    for (int j = group; j < n_steps; j += 2) {
+        const int4 me = next;
+        const size_t k = (size_t)me.x;
+        Contact64 c;
+        c.me = me;
+        double W[12];   // columns 2q, 2q + 1, 8 + q, four rows each
+        const double2* pj = reinterpret_cast<const double2*>(J + 48 * k);
+        const double2* pw = reinterpret_cast<const double2*>(WJT + 48 * k);
+        const double2* px = reinterpret_cast<const double2*>(x + 4 * k);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) { const double2 t = pj[4 * i]; c.J[2 * i] = t.x; c.J[2 * i + 1] = t.y; }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) { const double2 t = pw[4 * i]; W[2 * i] = t.x; W[2 * i + 1] = t.y; }
+        const double2 x01 = px[0], x23 = px[1];
+        const double xq = xs[4 * k], bq = b[4 * k], rq = r[4 * k], mu = v.mu[k];
+        next = meta(j + 2);
+        const int ia = q < 3 ? me.y + 2 * q : me.z, ic = me.z + 2 + q;
+        const bool put_a = (me.w & (q < 3 ? 1 : 2)) != 0, put_c = (me.w & 2) != 0;
+        if (j > 0) asm volatile("bar.sync %0, %1;" ::"r"(1 + ((j - 1) & 1)), "r"(2 * half) : "memory");
+        const double zq = xq - rq * (contact64_jw(c, w) + bq);
+        double z[4];
+        quad_gather(zq, z);
+        const double2 wa = w.pair(ia);
+        const double wc = w.one(ic);
+        const double xn = z[0] > 0.0 ? z[0] : 0.0;
+        double scale = 1.0;
+        const int kind = normal_only ? 0 : prox_factor(z, mu, xn, scale);
+        const double d0 = xn - x01.x, d1 = prox_apply(kind, scale, z[1]) - x01.y;
+        const double d2 = prox_apply(kind, scale, z[2]) - x23.x, d3v = prox_apply(kind, scale, z[3]) - x23.y;
+        double ta = 0.0, tb = 0.0, tc = 0.0;
+        ta += W[0] * d0; tb += W[4] * d0; tc += W[8] * d0;
+        ta += W[1] * d1; tb += W[5] * d1; tc += W[9] * d1;
+        ta += W[2] * d2; tb += W[6] * d2; tc += W[10] * d2;
+        ta += W[3] * d3v; tb += W[7] * d3v; tc += W[11] * d3v;
+        if (put_a) w.set(ia, make_double2(wa.x + ta, wa.y + tb));
+        if (put_c) w.set(ic, wc + tc);
+        if (j + 1 < n_steps) asm volatile("bar.arrive %0, %1;" ::"r"(1 + (j & 1)), "r"(2 * half) : "memory");
+        const double yq = q == 0 ? xn : prox_apply(kind, scale, zq);
+        if (!(me.w & kMetaIdle)) {
+            y[4 * k] = yq;
+            m = nanmax(m, fabs(yq - xq));
+        }
+    }
+    return m;
+}
+
 // A block sweeps a scene with the number of its warps that scene_setup64 chose.  One warp has warp barriers between the
 // levels, several a barrier of their own, and the block meets at the end of the sweep.
 template <class G>
@@ -1635,7 +1713,11 @@ __device__ __forceinline__ double gs_sweep_levels(const G& g, const Solve64& v, 
                                                   const double* x, double* y, bool normal_only) {
     if constexpr (std::is_same_v<G, BlockGroup>) {
         double m = 0.0;
-        if (v.warps == 1) {
+        if (v.turns) {
+            if ((int)threadIdx.x < 64 * v.warps)
+                m = v.w_shared ? gs_sweep_turns<true>(v, v.n_steps, b, r, x, y, normal_only)
+                               : gs_sweep_turns<false>(v, v.n_steps, b, r, x, y, normal_only);
+        } else if (v.warps == 1) {
             if (threadIdx.x < 32) m = gs_sweep_levels(WarpGroup{}, v, b, r, x, y, normal_only);
         } else if ((int)threadIdx.x < 32 * v.warps) {
             const SubGroup sub = {32 * v.warps};
