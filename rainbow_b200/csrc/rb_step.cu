@@ -1214,35 +1214,45 @@ struct WarpGroup {
         for (int o = 16; o > 0; o >>= 1) v = ::max(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
     }
-    // collect: the members whose flag is set take the places after the n taken so far, in order (every member
-    // calls it the same number of times); n is then the number taken
-    __device__ __forceinline__ int append_begin() const { return 0; }
-    __device__ __forceinline__ int append(bool flag, int& n) const {
-        const unsigned bal = __ballot_sync(0xffffffffu, flag);
-        const int at = n + __popc(bal & lanemask_lt());
-        n += __popc(bal);
-        return at;
+    __device__ __forceinline__ void max2(double& u, double& v) const { u = max(u); v = max(v); }
+    // exclusive prefix sum of the members' values and their total
+    __device__ __forceinline__ int scan(int v, int& total) const {
+        const int lane = threadIdx.x & 31;
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        total = __shfl_sync(0xffffffffu, incl, 31);
+        return incl - v;
     }
-    __device__ __forceinline__ void append_end(int&) const { __syncwarp(); }
 };
 
 struct BlockGroup {
-    double* red;   // 33 doubles of shared memory
+    double* red;   // 32 doubles of shared memory
     int* ired;     // 33 ints of shared memory
     __device__ __forceinline__ int rank() const { return threadIdx.x; }
     __device__ __forceinline__ int size() const { return blockDim.x; }
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     __device__ __forceinline__ bool any(bool p) const { return __syncthreads_or(p); }
     __device__ double max(double v) const {
-        for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        double w = 0.0;
+        max2(v, w);
+        return v;
+    }
+    // two maxima with one pair of barriers (up to sixteen warps)
+    __device__ void max2(double& u, double& v) const {
+        for (int o = 16; o > 0; o >>= 1) {
+            u = nanmax(u, __shfl_xor_sync(0xffffffffu, u, o));
+            v = nanmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+        }
+        const int wid = threadIdx.x >> 5;
+        if ((threadIdx.x & 31) == 0) { red[2 * wid] = u; red[2 * wid + 1] = v; }
         __syncthreads();
-        if (lane == 0) red[wid] = v;
+        u = red[0]; v = red[1];
+        for (int k = 1; k < (int)(blockDim.x >> 5); ++k) { u = nanmax(u, red[2 * k]); v = nanmax(v, red[2 * k + 1]); }
         __syncthreads();
-        double m = red[0];
-        for (int k = 1; k < (int)(blockDim.x >> 5); ++k) m = nanmax(m, red[k]);
-        __syncthreads();
-        return m;
     }
     __device__ int imax(int v) const {
         for (int o = 16; o > 0; o >>= 1) v = ::max(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -1255,21 +1265,20 @@ struct BlockGroup {
         __syncthreads();
         return m;
     }
-    __device__ int append_begin() const { return 0; }
-    __device__ int append(bool flag, int& n) const {
-        const unsigned bal = __ballot_sync(0xffffffffu, flag);
+    __device__ int scan(int v, int& total) const {
+        int warp_total;
+        int at = WarpGroup{}.scan(v, warp_total);
         const int wid = threadIdx.x >> 5;
-        if ((threadIdx.x & 31) == 0) ired[wid] = __popc(bal);
+        if ((threadIdx.x & 31) == 0) ired[wid] = warp_total;
         __syncthreads();
-        int at = n + __popc(bal & lanemask_lt());
+        total = 0;
         for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
             if (k < wid) at += ired[k];
-            n += ired[k];
+            total += ired[k];
         }
         __syncthreads();
         return at;
     }
-    __device__ void append_end(int&) const { __syncthreads(); }
 };
 
 // the first `threads` threads of a block (a multiple of 32), with a barrier of their own
@@ -1279,6 +1288,17 @@ struct SubGroup {
     __device__ __forceinline__ int size() const { return threads; }
     __device__ __forceinline__ void sync() const { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 };
+
+// two groups of threads by turns: group 0 ends its turn at barrier 1 and waits for the other's end at barrier 2, group 1
+// the other way round (written with their numbers, so that a block keeps three barriers and not all sixteen)
+__device__ __forceinline__ void turn_wait(int group, int threads) {
+    if (group) asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"r"(threads) : "memory");
+}
+__device__ __forceinline__ void turn_done(int group, int threads) {
+    if (group) asm volatile("bar.arrive 2, %0;" ::"r"(threads) : "memory");
+    else asm volatile("bar.arrive 1, %0;" ::"r"(threads) : "memory");
+}
 
 // The working set of one scene's FP64 solve.  Only the free bodies with contacts have accumulators w = WJT x that
 // change; they are numbered ("slots", in any order) and their accumulators lie together, in shared memory when they
@@ -1331,19 +1351,22 @@ struct W64 {
     }
 };
 
-// numbers the scene's touched bodies: their spans, and body -> slot in bc_fill (free once bc_list is filled)
-template <class G>
-__device__ __forceinline__ int scene_touched(const StepArgs& a, const G& g, const SceneRange& R) {
-    int2* span = reinterpret_cast<int2*>(a.ws.w2 + 6 * (size_t)R.b0);
-    int n = g.append_begin();
-    for (int base = R.b0; base < R.b1; base += g.size()) {
-        const int bb = base + g.rank();
-        const int e0 = bb < R.b1 ? a.ws.bc_ptr[bb] : 0, e1 = bb < R.b1 ? a.ws.bc_ptr[bb + 1] : 0;
-        const int at = g.append(e1 > e0, n);   // fixed bodies have no list entries
-        if (e1 > e0) { span[at] = make_int2(e0, e1); a.ws.bc_fill[bb] = at; }
-    }
-    g.append_end(n);
-    return n;
+// numbers the scene's touched bodies in body order: body -> slot in bc_fill (free once bc_list is filled), and
+// put(slot, body, e0, e1) for each.  A member takes a run of bodies, counts and then puts.  Returns their number.
+template <class G, class Put>
+__device__ __forceinline__ int scene_touched(const StepArgs& a, const G& g, const SceneRange& R, Put put) {
+    const int run = (R.b1 - R.b0 + g.size() - 1) / g.size();
+    const int b0 = min(R.b0 + g.rank() * run, R.b1), b1 = min(b0 + run, R.b1);
+    int n = 0, total;
+#pragma unroll 4
+    for (int b = b0; b < b1; ++b) n += a.ws.bc_ptr[b + 1] > a.ws.bc_ptr[b];   // fixed bodies have no list entries
+    int at = g.scan(n, total);
+    if (n > 0)
+        for (int b = b0; b < b1; ++b) {
+            const int e0 = a.ws.bc_ptr[b], e1 = a.ws.bc_ptr[b + 1];
+            if (e1 > e0) { a.ws.bc_fill[b] = at; put(at++, b, e0, e1); }
+        }
+    return total;
 }
 
 // Warps that sweep a scene, eight contacts each, and whether two groups of them do so by turns: the choice with the least
@@ -1403,11 +1426,13 @@ __device__ __forceinline__ Solve64 scene_setup64(const StepArgs& a, const G& g, 
     const int* order = L > 0 ? a.ws.lev_order + R.c0 : nullptr;
     Solve64 v;
     v.K = R.c1 - R.c0;
-    v.n_touched = scene_touched(a, g, R);
+    int2* span = reinterpret_cast<int2*>(a.ws.w2 + 6 * (size_t)R.b0);
+    v.n_touched = scene_touched(a, g, R, [&](int at, int, int e0, int e1) { span[at] = make_int2(e0, e1); });
+    g.sync();
     const int zero = v.n_touched < R.b1 - R.b0 ? v.n_touched : 0;
     v.w_shared = w_smem != nullptr && v.n_touched + 1 <= smem_bodies;
     v.w = v.w_shared ? w_smem : a.ws.w + 6 * (size_t)R.b0;
-    v.span = reinterpret_cast<const int2*>(a.ws.w2 + 6 * (size_t)R.b0);
+    v.span = span;
     int4* meta = reinterpret_cast<int4*>(a.ws.c32 + kS32Floats * (size_t)R.c0);
     v.meta = meta;
     v.bc_list = a.ws.bc_list;
@@ -1678,7 +1703,7 @@ __device__ __noinline__ double gs_sweep_turns(const Solve64 v, int n_steps, cons
         next = meta(j + 2);
         const int ia = q < 3 ? me.y + 2 * q : me.z, ic = me.z + 2 + q;
         const bool put_a = (me.w & (q < 3 ? 1 : 2)) != 0, put_c = (me.w & 2) != 0;
-        if (j > 0) asm volatile("bar.sync %0, %1;" ::"r"(1 + ((j - 1) & 1)), "r"(2 * half) : "memory");
+        if (j > 0) turn_wait(group, 2 * half);
         const double zq = xq - rq * (contact64_jw(c, w) + bq);
         double z[4];
         quad_gather(zq, z);
@@ -1696,7 +1721,7 @@ __device__ __noinline__ double gs_sweep_turns(const Solve64 v, int n_steps, cons
         ta += W[3] * d3v; tb += W[7] * d3v; tc += W[11] * d3v;
         if (put_a) w.set(ia, make_double2(wa.x + ta, wa.y + tb));
         if (put_c) w.set(ic, wc + tc);
-        if (j + 1 < n_steps) asm volatile("bar.arrive %0, %1;" ::"r"(1 + (j & 1)), "r"(2 * half) : "memory");
+        if (j + 1 < n_steps) turn_done(group, 2 * half);
         const double yq = q == 0 ? xn : prox_apply(kind, scale, zq);
         if (!(me.w & kMetaIdle)) {
             y[4 * k] = yq;
@@ -1773,20 +1798,29 @@ __device__ int scene_levels_smem(const StepArgs& a, const G& g, const SceneRange
         const int p0 = a.ws.cpred[2 * (R.c0 + k)], p1 = a.ws.cpred[2 * (R.c0 + k) + 1];
         pred[2 * k] = (int16_t)(p0 >= 0 ? p0 - R.c0 : -1);
         pred[2 * k + 1] = (int16_t)(p1 >= 0 ? p1 - R.c0 : -1);
-        lev[k] = 1;
     }
     g.sync();
-    for (;;) {
-        bool changed = false;
-        for (int k = g.rank(); k < K; k += g.size()) {
-            const int p0 = pred[2 * k], p1 = pred[2 * k + 1];
-            const int l0 = p0 >= 0 ? lev[p0] : 0;
-            const int l1 = p1 >= 0 ? lev[p1] : 0;
-            const int l = 1 + max(l0, l1);
-            if (l != lev[k]) { lev[k] = (int16_t)l; changed = true; }
+    // predecessors come earlier: one warp goes through the contacts 32 at a time, those of the earlier runs final, and
+    // relaxes within the run until nothing changes (relaxing all of them in rounds of the whole team took 60 to 100
+    // thousand cycles for 600 contacts on 50 to 90 levels)
+    if (g.rank() < 32)
+        for (int k0 = 0; k0 < K; k0 += 32) {
+            const int k = k0 + g.rank();
+            const bool mine = k < K;
+            const int p0 = mine ? pred[2 * k] : -1, p1 = mine ? pred[2 * k + 1] : -1;
+            int l = 1;
+            if (mine) lev[k] = 1;
+            __syncwarp();
+            for (;;) {
+                const int l0 = p0 >= 0 ? lev[p0] : 0, l1 = p1 >= 0 ? lev[p1] : 0;
+                const int next = 1 + max(l0, l1);
+                const bool changed = mine && next != l;
+                if (!__any_sync(0xffffffffu, changed)) break;   // (every lane has read before any writes)
+                if (changed) { l = next; lev[k] = (int16_t)l; }
+                __syncwarp();
+            }
         }
-        if (!g.any(changed)) break;
-    }
+    g.sync();
     int L = 0;
     for (int k = g.rank(); k < K; k += g.size()) {
         const int l = lev[k];
@@ -1809,6 +1843,16 @@ __device__ int scene_levels_smem(const StepArgs& a, const G& g, const SceneRange
     for (int k = g.rank(); k < K; k += g.size()) a.ws.lev_order[R.c0 + atomicAdd(cnt + lev[k] - 1, 1)] = R.c0 + k;
     g.sync();
     return L;
+}
+
+// the levels with the accumulators' shared memory as scratch where it suffices (it is not in use yet)
+template <class G>
+__device__ __forceinline__ int scene_levels_any(const StepArgs& a, const G& g, const SceneRange& R, int s, double* w_smem,
+                                                int smem_bodies) {
+    const int K = R.c1 - R.c0;
+    if (w_smem != nullptr && K <= 32767 && s32_level_scratch(K) <= 6 * sizeof(double) * (size_t)smem_bodies)
+        return scene_levels_smem(a, g, R, s, reinterpret_cast<int16_t*>(w_smem));
+    return scene_levels(a, g, R, s);
 }
 
 // Groups the scene's contacts by their class lev_of[k] (1-based level or colour): lev_ptr[c-1] .. lev_ptr[c]
@@ -1935,9 +1979,8 @@ __device__ double scene_residual(const StepArgs& a, const G& g, const Solve64& v
             xm = fmax(xm, fabs(xq));
         }
     }
-    const double mres = g.max(m);
-    const double mx = g.max(xm);
-    return mres / (mx > 1.0 ? mx : 1.0);
+    g.max2(m, xm);
+    return m / (xm > 1.0 ? xm : 1.0);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -2167,7 +2210,7 @@ __device__ void solve_scene_hinges(const StepArgs& a, const G& g, int s, double*
         st->n_levels = 0; st->fp32_sweeps = 0;
     }
     if (hist) for (int i = g.rank(); i < max_it; i += g.size()) hist[i] = INFINITY;
-    const int L = K > 0 ? scene_levels(a, g, R, s) : 0;
+    const int L = K > 0 ? scene_levels_any(a, g, R, s, w_smem, smem_bodies) : 0;
     Solve64 v = {};
     if (K > 0) v = scene_setup64(a, g, R, s, L, w_smem, smem_bodies);
     const int HL = hinge_levels(a, g, R, s, h0, h1);
@@ -2294,7 +2337,7 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
     // FP32 modes: the scene's FP32 phase left its iterate in x and its level order in lev_order / lev_ptr
     const int sweeps32 = (!post && a.pr.precision != RB_PRECISION_FP64) ? a.ws.sweeps32[s] : -1;
     const int L = jacobi ? 0 : sweeps32 >= 0 ? a.ws.nlev[s]
-                : (coloured ? scene_colours(a, g, R, s) : scene_levels(a, g, R, s));
+                : (coloured ? scene_colours(a, g, R, s) : scene_levels_any(a, g, R, s, w_smem, smem_bodies));
     if (!post && g.rank() == 0) st->n_levels = L;
     const Solve64 v = scene_setup64(a, g, R, s, L, w_smem, smem_bodies);
     const bool by_residual = !post && a.pr.termination != RB_TERMINATE_MERIT;
@@ -2446,8 +2489,7 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kQueueFp32 = 5;                        // counters[5..8]: scene queues of the four size classes
 constexpr int kClassEnd32 = 9;                       // counters[9..12]: end of each class's range in list32
-constexpr int kFp32Block = 128;                      // threads per block of the FP32 launches
-constexpr int kFp32BlockMax = 256;                   // ... at most, in the launches for slab scenes
+constexpr int kFp32Block = 128;                      // threads per block of the large slab's launch
 constexpr int kFp32L2Block = 512;                    // threads of the launch for the scenes beyond any slab
 constexpr int kFp32LargeSmem = 224 * 1024;           // slab of a block team (one scene per SM)
 constexpr int kS32SmallSlab = 28 * 1024;             // slab of a warp team, small class (8 scenes per SM)
@@ -2585,16 +2627,16 @@ constexpr uint32_t kC32 = sizeof(float) * kS32Floats, kB32 = sizeof(float) * kS3
 __device__ __forceinline__ uint32_t c32_at(int piece, int q) { return 64u * piece + 16u * q; }
 constexpr uint32_t kX32 = 192;
 
-// Warps that sweep a scene of these levels: the number (a power of two) with the least cost.  A level of up to eight
-// contacts a warp is a step of quads and a wider one steps of a lane per contact, or, with the rows in L2 (in_l2),
-// more steps of quads.  The cycles of a step, in tens, are fitted to the solve times of 18 scenes of 240-510 contacts
-// (2 % off on average: quads 418, 411, 557 and lanes 723, 630, 1038 cycles with one, two and four warps; with quads
-// alone 64 scenes of up to 256 bodies took 4922, 4209, 4683 us, with both 4535, 3944, 4696) and, in L2, of one of 1565
-// (27256, 16884, 9525 us).  Every warp of the group counts for itself.
+// Warps that sweep a step of a scene of these levels: the number (a power of two, up to max_warps) with the least cost.
+// A level of up to eight contacts a warp is a step of quads and a wider one steps of a lane per contact, or, with the
+// rows in L2 (in_l2), more steps of quads.  The cycles of a step, in tens: by turns 400-420 with quads
+// (14 to 600 contacts, one or two warps a step) and 515 with lanes (547 contacts on six levels); in L2 those that fit
+// 200 sweeps over 1565 contacts by one, two and four warps (27256, 16884, 9525 us).
+// Every warp of the block counts for itself.
 __device__ __forceinline__ int s32_warps(const int* ptr, int L, int max_warps, bool in_l2) {
     int cost[4] = {0, 0, 0, 0};
-    const int quads[4] = {in_l2 ? 120 : 42, in_l2 ? 125 : 41, in_l2 ? 112 : 56, in_l2 ? 140 : 100};
-    const int lanes[4] = {70, 63, 100, 140};
+    const int quads[4] = {in_l2 ? 120 : 40, in_l2 ? 125 : 42, in_l2 ? 112 : 60, in_l2 ? 140 : 90};
+    const int lanes[4] = {50, 52, 70, 100};
     for (int l = threadIdx.x & 31; l < L; l += 32) {
         const int n = ptr[l + 1] - ptr[l];
 #pragma unroll
@@ -2622,49 +2664,38 @@ __device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const Sce
                 : scratch ? scene_levels_smem(a, g, R, s, scratch) : scene_levels(a, g, R, s);
     const int* order = a.ws.lev_order + R.c0;
     float* c = reinterpret_cast<float*>(f.c);
-    for (int t = g.rank(); t < 16 * K; t += g.size()) {   // (position, float4 group, row), impulses last
-        const int i = t >> 4, part = (t >> 2) & 3, q = t & 3;
+    // a lane per row (a quad per contact), all of whose values load together: with a lane per float4 group of a row, the
+    // groups' branches each waited for L2 in turn (260 thousand cycles for 600 contacts, a tenth of 100 sweeps)
+#pragma unroll 2
+    for (int t = g.rank(); t < 4 * K; t += g.size()) {
+        const int i = t >> 2, q = t & 3;
         const size_t k = (size_t)order[i];
-        float* o = c + kS32Floats * (size_t)i + 16 * part;
-        const double* J = a.ws.J + 48 * k;
-        float4 v;
-        if (part == 0) {
-            v.x = q < 3 ? (float)J[j_at(q, 0)] : 0.0f;
-            v.y = q < 3 ? (float)J[j_at(q, 1)] : 0.0f;
-            v.z = q < 3 ? (float)J[j_at(q, 2)] : 0.0f;
-            v.w = (float)a.ws.b[4 * k + q];
-        } else if (part == 1) {
-            v.x = (float)J[j_at(q, 3)]; v.y = (float)J[j_at(q, 4)]; v.z = (float)J[j_at(q, 5)];
-            v.w = (float)(1.0 / a.ws.diag[4 * k + q]);
-        } else if (part == 2) {
-            v.x = (float)J[j_at(q, 9)]; v.y = (float)J[j_at(q, 10)]; v.z = (float)J[j_at(q, 11)];
-            v.w = (float)a.ws.mu[k];
-        } else {
-            reinterpret_cast<float*>(f.x + (size_t)f.xs * i)[q] = (float)a.ws.x[4 * k + q];
-            continue;
-        }
-        reinterpret_cast<float4*>(o)[q] = v;
+        const double2* J = reinterpret_cast<const double2*>(a.ws.J + 48 * k + 2 * q);
+        const double2 j0 = J[0], j1 = J[4], j2 = J[8], j4 = J[16], j5 = J[20];   // columns 0..5 and 8..11 of row q
+        const double b = a.ws.b[4 * k + q], diag = a.ws.diag[4 * k + q], x = a.ws.x[4 * k + q], mu = a.ws.mu[k];
+        float4* o = reinterpret_cast<float4*>(c + kS32Floats * (size_t)i) + q;
+        o[0] = q < 3 ? make_float4((float)j0.x, (float)j0.y, (float)j1.x, (float)b) : make_float4(0.0f, 0.0f, 0.0f, (float)b);
+        o[4] = make_float4((float)j1.y, (float)j2.x, (float)j2.y, (float)(1.0 / diag));
+        o[8] = make_float4((float)j4.y, (float)j5.x, (float)j5.y, (float)mu);
+        reinterpret_cast<float*>(f.x + (size_t)f.xs * i)[q] = (float)x;
     }
     // the slots: the free bodies with contacts in body order (their lists in bc_list then follow one another)
     const int e0 = a.ws.bc_ptr[R.b0];
     uint16_t* bptr = reinterpret_cast<uint16_t*>(f.bptr);
-    int n = g.append_begin();
-    for (int base = R.b0; base < R.b1; base += g.size()) {
-        const int b = base + g.rank();
-        const int p0 = b < R.b1 ? a.ws.bc_ptr[b] : 0, p1 = b < R.b1 ? a.ws.bc_ptr[b + 1] : 0;
-        const int at = g.append(p1 > p0, n);
-        if (p1 > p0) {
-            a.ws.bc_fill[b] = at;
-            bptr[at] = (uint16_t)(p0 - e0);
-            float* B = reinterpret_cast<float*>(f.body + kB32 * (size_t)at);
-            const double* Wi = a.ws.Winv + 9 * (size_t)b;
-            B[3] = (float)(1.0 / a.bd.mass[b]);
-            B[7] = 0.0f;
-            B[8] = (float)Wi[0]; B[9] = (float)Wi[1]; B[10] = (float)Wi[2];
-            B[11] = (float)Wi[4]; B[12] = (float)Wi[5]; B[13] = (float)Wi[8];
-        }
+    const int n = scene_touched(a, g, R, [&](int at, int b, int p0, int) {
+        bptr[at] = (uint16_t)(p0 - e0);
+        reinterpret_cast<int*>(f.body + kB32 * (size_t)at)[0] = b;   // whose record it is, until the record is filled
+    });
+    g.sync();
+    for (int i = g.rank(); i < n; i += g.size()) {
+        float* B = reinterpret_cast<float*>(f.body + kB32 * (size_t)i);
+        const int b = reinterpret_cast<const int*>(B)[0];
+        const double* Wi = a.ws.Winv + 9 * (size_t)b;
+        B[3] = (float)(1.0 / a.bd.mass[b]);
+        B[7] = 0.0f;
+        B[8] = (float)Wi[0]; B[9] = (float)Wi[1]; B[10] = (float)Wi[2];
+        B[11] = (float)Wi[4]; B[12] = (float)Wi[5]; B[13] = (float)Wi[8];
     }
-    g.append_end(n);
     f.n_free = n;
     if (g.rank() == 0) bptr[n] = (uint16_t)(a.ws.bc_ptr[R.b1] - e0);
     if (n < s32_records(K, R.b1 - R.b0) && g.rank() < kS32BodyFloats)   // the fixed bodies' record
@@ -2672,6 +2703,7 @@ __device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const Sce
     g.sync();   // slots complete
     uint16_t* pos = reinterpret_cast<uint16_t*>(f.pos);
     uint32_t* lohi = reinterpret_cast<uint32_t*>(f.lohi);
+#pragma unroll 4
     for (int i = g.rank(); i < K; i += g.size()) {
         const int k = order[i];
         pos[k - R.c0] = (uint16_t)i;
@@ -2682,13 +2714,15 @@ __device__ __forceinline__ int s32_load(const StepArgs& a, const G& g, const Sce
     g.sync();   // pos complete
     // per-body contact lists (the residual's w = W J^T x), positions in level order
     uint32_t* blist = reinterpret_cast<uint32_t*>(f.blist);
-    for (int e = g.rank(); e < a.ws.bc_ptr[R.b1] - e0; e += g.size()) {
+    const int entries = a.ws.bc_ptr[R.b1] - e0;
+#pragma unroll 4
+    for (int e = g.rank(); e < entries; e += g.size()) {
         const int code = a.ws.bc_list[e0 + e];
         blist[e] = ((uint32_t)pos[(code >> 1) - R.c0] << 1) | (uint32_t)(code & 1);
     }
     g.sync();   // pos used: the steps take its room
     const int* ptr = a.ws.lev_ptr + R.c0 + s;
-    f.warps = f.ring ? kRingWarps : g.size() > 32 ? s32_warps(ptr, L, g.size() >> 5, in_l2) : 1;
+    f.warps = f.ring ? kRingWarps : s32_warps(ptr, L, in_l2 ? g.size() >> 5 : g.size() >> 6, in_l2);
     uint32_t* steps = reinterpret_cast<uint32_t*>(f.steps);
     f.n_steps = sweep_steps(g, ptr, L, in_l2 ? 0 : 8 * f.warps, in_l2 ? 8 * f.warps : 32 * f.warps, [&](int at, int start, int count, bool ends, bool wide) {
         steps[at] = (uint32_t)start | ((uint32_t)count << 16) | (ends ? kStep32Ends : 0u) | (wide && !in_l2 ? kStep32Wide : 0u);
@@ -2796,8 +2830,8 @@ __device__ __noinline__ float s32_residual(const G g, const S32Scene f) {
             xm = fmaxf(xm, fabsf(x));
         }
     }
-    const double mres = g.max((double)m);
-    const double mx = g.max((double)xm);
+    double mres = (double)m, mx = (double)xm;
+    g.max2(mres, mx);
     return (float)(mres / (mx > 1.0 ? mx : 1.0));
 }
 
@@ -2979,6 +3013,136 @@ __device__ __noinline__ void s32_sweep(const G g, const S32Scene f, float rscale
     }
 }
 
+// n_sweeps sweeps of a slab scene by two groups of f.warps warps that take the steps by turns (as gs_sweep_turns does in
+// FP64): while one computes a step, the other loads all that its next step's contacts do not have from w, so that only
+// the chain itself -- the accumulators' loads, the row products, the prox, the update and its stores -- lies between the
+// barriers.  The steps and their expressions are s32_sweep's: a quad of lanes per contact, or in a wide step a lane.
+// A step's impulses are stored after its barrier, so a sweep has at least five steps (kTurnsSteps): the next one to load
+// them, five or more steps on, has by then passed a barrier that the storing group reached later.
+__device__ __noinline__ void s32_sweep_turns(const S32Scene f, float rscale, int n_sweeps) {
+    const ShPtr c(f.c), body(f.body), lohi(f.lohi), steps(f.steps);
+    const int half = 32 * f.warps, group = (int)threadIdx.x >= half, rank = threadIdx.x - group * half;
+    const int q = rank & 3, quad = rank >> 2;
+    const bool linear = q < 2;
+    const uint32_t hi_shift = (q & 1) ? 16u : 0u;          // lanes 1 and 3 update the hi body
+    const uint32_t fixed_bit = 0x8000u << hi_shift;
+    const uint32_t part = linear ? 0u : 16u;                // their float4 of w
+    const uint32_t col = linear ? 0u : 64u * (uint32_t)(q - 1);   // the piece whose columns the lane sums
+    const float sg = q == 1 ? -1.0f : 1.0f;
+    const int n_steps = f.n_steps, total = n_sweeps * n_steps;
+    auto at = [&](uint32_t st) { return min((int)(st & 0x7fffu) + ((st & kStep32Wide) ? rank : quad), f.K - 1); };
+    int place = group < n_steps ? group : 0;   // the step's place in its sweep
+    uint32_t st_next = (steps + 4u * place).u32();
+    uint32_t lh_next = (lohi + 4u * at(st_next)).u32();
+#pragma unroll 1
+    for (int j = group; j < total; j += 2) {
+        const uint32_t st = st_next, lh = lh_next;
+        const ShPtr rec = c + kC32 * at(st);
+        const ShPtr Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
+        place += 2;
+        while (place >= n_steps) place -= n_steps;
+        st_next = (steps + 4u * place).u32();
+        const int count = (int)((st >> 16) & 0x1fffu);
+        if (!(st & kStep32Wide)) {
+            const float4 r0 = (rec + 16u * q).f4(), r1 = (rec + (64u + 16u * q)).f4(), r2 = (rec + (128u + 16u * q)).f4();
+            const ShPtr cl = rec + col;
+            const float4 v0 = cl.f4(), v1 = (cl + 16u).f4(), v2 = (cl + 32u).f4(), v3 = (cl + 48u).f4();
+            const ShPtr B = body + kB32 * ((lh >> hi_shift) & 0x7fffu);
+            const float4 I0 = (B + 32u).f4();
+            const float2 I1 = (B + 48u).f2();
+            const float wxy = linear ? 0.0f : I0.y, wxz = linear ? 0.0f : I0.z, wyz = linear ? 0.0f : I1.x;
+            const bool mine = quad < count, put = mine && !(lh & fixed_bit);
+            lh_next = (lohi + 4u * at(st_next)).u32();
+            const float rs = rscale * r1.w;
+            const float4 x = (rec + kX32).f4();
+            const float xq = (rec + (kX32 + 4u * q)).f1();
+            if (j > 0) turn_wait(group, 2 * half);
+            const float4 l0 = Bl.f4(), h0 = Bh.f4(), l1 = (Bl + 16u).f4(), h1 = (Bh + 16u).f4();
+            const float4 own = (B + part).f4();
+            const float zq = xq - rs * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
+            float z[4];
+            quad_gather(zq, z);
+            // the lane's part of W: m^-1 on the diagonal (negative for the hi body: lin_hi = -lin_lo), or I^-1
+            const float m = sg * own.w;
+            const float wxx = linear ? m : I0.x, wyy = linear ? m : I0.w, wzz = linear ? m : I1.y;
+            const float xn = fmaxf(z[0], 0.0f);
+            // prox onto the friction ball of radius mu xn
+            const float radius = r2.w * xn;
+            const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
+            float scale = sqr > radius * radius ? radius * rsqrtf(sqr) : 1.0f;
+            if (xn <= 0.0f) scale = 0.0f;
+            const float f1 = z[1] * scale, f2 = z[2] * scale, f3 = z[3] * scale;
+            const float d0 = xn - x.x, d1 = f1 - x.y, d2 = f2 - x.z, d3 = f3 - x.w;
+            const float S0 = fmaf(v3.x, d3, fmaf(v2.x, d2, fmaf(v1.x, d1, v0.x * d0)));
+            const float S1 = fmaf(v3.y, d3, fmaf(v2.y, d2, fmaf(v1.y, d1, v0.y * d0)));
+            const float S2 = fmaf(v3.z, d3, fmaf(v2.z, d2, fmaf(v1.z, d1, v0.z * d0)));
+            const float4 n = make_float4(own.x + fmaf(wxx, S0, fmaf(wxy, S1, wxz * S2)),
+                                         own.y + fmaf(wxy, S0, fmaf(wyy, S1, wyz * S2)),
+                                         own.z + fmaf(wxz, S0, fmaf(wyz, S1, wzz * S2)), own.w);
+            // the fixed bodies' record is only read; an idle quad writes nothing
+            if (put) (B + part).set(n);
+            if (j + 1 < total) turn_done(group, 2 * half);
+            if (mine) (rec + (kX32 + 4u * q)).set(q == 0 ? xn : zq * scale);
+        } else {
+            float4 r[12];
+#pragma unroll
+            for (int t = 0; t < 12; ++t) r[t] = (rec + 16u * t).f4();
+            const float4 Il0 = (Bl + 32u).f4(), Ih0 = (Bh + 32u).f4();
+            const float2 Il1 = (Bl + 48u).f2(), Ih1 = (Bh + 48u).f2();
+            const bool mine = rank < count;
+            lh_next = (lohi + 4u * at(st_next)).u32();
+            const float4 x = (rec + kX32).f4();
+            if (j > 0) turn_wait(group, 2 * half);
+            const float4 l0 = Bl.f4(), h0 = Bh.f4(), l1 = (Bl + 16u).f4(), h1 = (Bh + 16u).f4();
+            const float xs[4] = {x.x, x.y, x.z, x.w};
+            float z[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float4 r0 = r[k], r1 = r[4 + k], r2 = r[8 + k];
+                float lin = 0.0f;
+                if (k < 3) lin = fmaf(r0.x, l0.x - h0.x, fmaf(r0.y, l0.y - h0.y, r0.z * (l0.z - h0.z)));
+                const float alo = fmaf(r1.x, l1.x, fmaf(r1.y, l1.y, r1.z * l1.z));
+                const float ahi = fmaf(r2.x, h1.x, fmaf(r2.y, h1.y, r2.z * h1.z));
+                z[k] = xs[k] - rscale * r1.w * (((lin + alo) + ahi) + r0.w);
+            }
+            const float xn = fmaxf(z[0], 0.0f);
+            const float radius = r[8].w * xn;
+            const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
+            float scale = sqr > radius * radius ? radius * rsqrtf(sqr) : 1.0f;
+            if (xn <= 0.0f) scale = 0.0f;
+            const float f1 = z[1] * scale, f2 = z[2] * scale, f3 = z[3] * scale;
+            const float d0 = xn - x.x, d1 = f1 - x.y, d2 = f2 - x.z, d3 = f3 - x.w;
+            // the three sums of the update (the torsion row has no linear columns)
+            const float L0 = fmaf(r[2].x, d2, fmaf(r[1].x, d1, r[0].x * d0));
+            const float L1 = fmaf(r[2].y, d2, fmaf(r[1].y, d1, r[0].y * d0));
+            const float L2 = fmaf(r[2].z, d2, fmaf(r[1].z, d1, r[0].z * d0));
+            const float A0 = fmaf(r[7].x, d3, fmaf(r[6].x, d2, fmaf(r[5].x, d1, r[4].x * d0)));
+            const float A1 = fmaf(r[7].y, d3, fmaf(r[6].y, d2, fmaf(r[5].y, d1, r[4].y * d0)));
+            const float A2 = fmaf(r[7].z, d3, fmaf(r[6].z, d2, fmaf(r[5].z, d1, r[4].z * d0)));
+            const float H0 = fmaf(r[11].x, d3, fmaf(r[10].x, d2, fmaf(r[9].x, d1, r[8].x * d0)));
+            const float H1 = fmaf(r[11].y, d3, fmaf(r[10].y, d2, fmaf(r[9].y, d1, r[8].y * d0)));
+            const float H2 = fmaf(r[11].z, d3, fmaf(r[10].z, d2, fmaf(r[9].z, d1, r[8].z * d0)));
+            const float ml = l0.w, mh = -h0.w;
+            if (mine && !(lh & 0x8000u)) {
+                Bl.set(make_float4(l0.x + ml * L0, l0.y + ml * L1, l0.z + ml * L2, ml));
+                (Bl + 16u).set(make_float4(l1.x + fmaf(Il0.x, A0, fmaf(Il0.y, A1, Il0.z * A2)),
+                                           l1.y + fmaf(Il0.y, A0, fmaf(Il0.w, A1, Il1.x * A2)),
+                                           l1.z + fmaf(Il0.z, A0, fmaf(Il1.x, A1, Il1.y * A2)), 0.0f));
+            }
+            if (mine && !(lh & 0x80000000u)) {
+                Bh.set(make_float4(h0.x + mh * L0, h0.y + mh * L1, h0.z + mh * L2, h0.w));
+                (Bh + 16u).set(make_float4(h1.x + fmaf(Ih0.x, H0, fmaf(Ih0.y, H1, Ih0.z * H2)),
+                                           h1.y + fmaf(Ih0.y, H0, fmaf(Ih0.w, H1, Ih1.x * H2)),
+                                           h1.z + fmaf(Ih0.z, H0, fmaf(Ih1.x, H1, Ih1.y * H2)), 0.0f));
+            }
+            if (j + 1 < total) turn_done(group, 2 * half);
+            if (mine) (rec + kX32).set(make_float4(xn, f1, f2, f3));
+        }
+        __syncwarp();   // a quad's impulses are stored by its four lanes and loaded by each of them
+    }
+}
+constexpr int kTurnsSteps = 5;
+
 // The narrow steps of s32_sweep for a scene whose rows come through the ring: a step's records, contiguous in level
 // order, are copied into its slot four steps ahead by a warp of their own (asynchronous 16-byte copies, one group a
 // step; at a step's end the copies of the next but one are waited for, and the step's barrier shows them to all).  With the rows read from L2 by the lanes that need them a
@@ -3088,18 +3252,18 @@ __device__ __noinline__ void s32_sweep_ring(const S32Scene f, float rscale, int 
 // n_sweeps sweeps by as many of the team's warps as the scene's levels keep busy
 template <class P, class G>
 __device__ __forceinline__ void s32_sweep_team(const G& g, const S32Scene& f, float rscale, int n_sweeps) {
-    if constexpr (std::is_same_v<G, BlockGroup>) {
-        if (std::is_same_v<P, GlPtr> && f.ring) {
-            if (threadIdx.x < 32 * (kRingWarps + 1)) s32_sweep_ring(f, rscale, n_sweeps);
-        } else if (f.warps == 1) {
-            if (threadIdx.x < 32) s32_sweep<P>(WarpGroup{}, f, rscale, n_sweeps);
-        } else if ((int)threadIdx.x < 32 * f.warps) {
-            s32_sweep<P>(SubGroup{32 * f.warps}, f, rscale, n_sweeps);
-        }
-        g.sync();
-    } else {
-        s32_sweep<P>(g, f, rscale, n_sweeps);
+    if (std::is_same_v<G, WarpGroup>) {
+        s32_sweep<P>(WarpGroup{}, f, rscale, n_sweeps);
+    } else if (std::is_same_v<P, GlPtr> && f.ring) {
+        if (threadIdx.x < 32 * (kRingWarps + 1)) s32_sweep_ring(f, rscale, n_sweeps);
+    } else if (std::is_same_v<P, ShPtr> && f.n_steps >= kTurnsSteps) {
+        if ((int)threadIdx.x < 64 * f.warps) s32_sweep_turns(f, rscale, n_sweeps);
+    } else if (f.warps == 1) {
+        if (threadIdx.x < 32) s32_sweep<P>(WarpGroup{}, f, rscale, n_sweeps);
+    } else if ((int)threadIdx.x < 32 * f.warps) {
+        s32_sweep<P>(SubGroup{32 * f.warps}, f, rscale, n_sweeps);
     }
+    g.sync();
 }
 
 // One proximal Jacobi sweep (proximal_contact/jacobi_solver.py:41-57) on the FP32 copy: every contact's new
@@ -3201,10 +3365,9 @@ __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, con
             xm = fmax(xm, fabs(x));
         }
     }
-    const double mres = g.max(m);
-    const double mx = g.max(xm);
+    g.max2(m, xm);
     g.sync();
-    return mres / (mx > 1.0 ? mx : 1.0);
+    return m / (xm > 1.0 ? xm : 1.0);
 }
 
 // size class of a scene's FP32 copy: 0 and 1 warp teams with small and mid slabs, 2 block teams with the
@@ -3276,14 +3439,17 @@ __global__ void __launch_bounds__(1024) k_fp32_classes(const StepArgs a, size_t 
 
 template <class G>
 __device__ __forceinline__ int team_next(const G& g, int* counter, int* slot) {
-    int s = 0;
-    if (g.rank() == 0) s = atomicAdd(counter, 1);
-    if (g.size() == 32) return __shfl_sync(0xffffffffu, s, 0);
-    if (g.rank() == 0) *slot = s;
-    __syncthreads();
-    s = *slot;
-    __syncthreads();
-    return s;
+    if constexpr (std::is_same_v<G, WarpGroup>) {
+        int s = 0;
+        if (g.rank() == 0) s = atomicAdd(counter, 1);
+        return __shfl_sync(0xffffffffu, s, 0);
+    } else {
+        if (g.rank() == 0) *slot = atomicAdd(counter, 1);
+        __syncthreads();
+        const int s = *slot;
+        __syncthreads();
+        return s;
+    }
 }
 
 // the FP64 solve of a scene as a call of its own, so that it does not raise the FP32 kernel's registers
@@ -3292,23 +3458,22 @@ __device__ __noinline__ void solve_scene_call(const StepArgs& a, const G& g, int
     solve_scene(a, g, s, 0, nullptr, 0);
 }
 
-// FP32 phase for the scenes whose compact copy takes lo_bytes < bytes <= slab bytes; G = WarpGroup gives
-// every warp of the block its own slab and scene, G = BlockGroup one slab and scene per block.  kL2: the
-// scenes too large for any slab, with their contact rows in global memory (L2-resident) and the rest of
-// the copy in the slab.
-template <class G, bool kL2>
-__global__ void __launch_bounds__(kL2 ? kFp32L2Block : kFp32BlockMax, 1) k_solve_fp32(const StepArgs a, int queue, size_t lo_bytes, size_t slab) {
+// FP32 phase for the scenes whose compact copy takes lo_bytes < bytes <= slab bytes, a block per scene.  kL2: the scenes
+// too large for any slab, with their contact rows in global memory (L2-resident) and the rest of the copy in the slab.
+// The small and mid slabs' scenes take one warp each (G = WarpGroup): by turns their steps are a little shorter (396
+// against ~430 cycles), but the team's barriers in every residual test take more than that (32-box tower, 200 sweeps:
+// 530 us with one warp, 638 with two).
+template <class G, bool kL2, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1) k_solve_fp32(const StepArgs a, int queue, size_t lo_bytes, size_t slab) {
     extern __shared__ __align__(16) char f32_smem[];
     __shared__ double red[33];
     __shared__ int ired[33];
     __shared__ int next_slot;
     if (a.ws.counters[kAbort]) return;
     G g;
+    if constexpr (std::is_same_v<G, BlockGroup>) { g.red = red; g.ired = ired; }
     using P = std::conditional_t<kL2, GlPtr, ShPtr>;
-    constexpr bool block_team = std::is_same_v<G, BlockGroup>;
-    if constexpr (block_team) { g.red = red; g.ired = ired; }
-    const int team = block_team ? 0 : (int)(threadIdx.x >> 5);
-    char* my_slab = f32_smem + (size_t)team * slab;
+    char* my_slab = f32_smem;
     const int max_it = a.pr.max_iterations;
     const int interval = a.pr.residual_interval > 1 ? a.pr.residual_interval : 1;
     // the FP32 sweeps aim a little below the tolerance when an FP64 test follows, so that the FP32 problem
@@ -3743,11 +3908,11 @@ int ensure_kernel_attributes() {
     e = cudaFuncSetAttribute(k_solve_warps, cudaFuncAttributeMaxDynamicSharedMemorySize, warp_max);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_solve_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, block_max);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_solve_fp32<WarpGroup, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFp32LargeSmem);
+        e = cudaFuncSetAttribute(k_solve_fp32<WarpGroup, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kS32MidSlab);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_solve_fp32<BlockGroup, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFp32LargeSmem);
+        e = cudaFuncSetAttribute(k_solve_fp32<BlockGroup, false, kFp32Block>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFp32LargeSmem);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_solve_fp32<BlockGroup, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFp32LargeSmem);
+        e = cudaFuncSetAttribute(k_solve_fp32<BlockGroup, true, kFp32L2Block>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFp32LargeSmem);
     if (e != cudaSuccess) return fail(RB_ERR_CUDA, std::string("rb_step: cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     g_attr_done[dev] = true;
     return RB_OK;
@@ -3926,18 +4091,18 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
         if (rc != RB_OK) return rc;
         cudaEventRecord(ss->fork, st);
         for (int c = 0; c < kSideStreams; ++c) cudaStreamWaitEvent(ss->s[c], ss->fork, 0);
-        k_solve_fp32<BlockGroup, true><<<148, kFp32L2Block, (size_t)kFp32LargeSmem, ss->s[3]>>>(
+        k_solve_fp32<BlockGroup, true, kFp32L2Block><<<148, kFp32L2Block, (size_t)kFp32LargeSmem, ss->s[3]>>>(
             a, kQueueFp32 + 3, kFp32LargeSmem, kFp32LargeSmem); note_launch();
-        k_solve_fp32<BlockGroup, false><<<148, kFp32Block, (size_t)kFp32LargeSmem, ss->s[2]>>>(
+        k_solve_fp32<BlockGroup, false, kFp32Block><<<148, kFp32Block, (size_t)kFp32LargeSmem, ss->s[2]>>>(
             a, kQueueFp32 + 2, mid_slab, kFp32LargeSmem); note_launch();
         // warp teams as one-warp blocks: a team's slab is released as soon as the team finds its queue empty
         // (in blocks of four teams the slowest held all four slabs), so the small class fills the room the mid
         // class leaves; as many blocks per SM as the shared memory (227 KB) allows, up to 32
         const int small_per_sm = std::min(32, (227 * 1024) / small_slab);
         const int mid_per_sm = std::max(1, std::min(32, (227 * 1024) / mid_slab));
-        k_solve_fp32<WarpGroup, false><<<148 * mid_per_sm, 32, (size_t)mid_slab, ss->s[1]>>>(
+        k_solve_fp32<WarpGroup, false, 32><<<148 * mid_per_sm, 32, (size_t)mid_slab, ss->s[1]>>>(
             a, kQueueFp32 + 1, small_slab, mid_slab); note_launch();
-        k_solve_fp32<WarpGroup, false><<<148 * small_per_sm, 32, (size_t)small_slab, ss->s[0]>>>(
+        k_solve_fp32<WarpGroup, false, 32><<<148 * small_per_sm, 32, (size_t)small_slab, ss->s[0]>>>(
             a, kQueueFp32, 0, small_slab); note_launch();
         for (int c = 0; c < kSideStreams; ++c) {
             cudaEventRecord(ss->join[c], ss->s[c]);
