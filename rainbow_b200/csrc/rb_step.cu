@@ -2483,9 +2483,9 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
 // inertia (6, symmetric), in a record of kS32BodyFloats (all fixed bodies share one with m^-1 = I^-1 = 0).  The update
 // of w after a contact changes by dx is m^-1 sum_q lin_q dx_q (negated on the hi side) and I^-1 sum_q ang_q dx_q.
 //
-// Execution.  A team -- one warp for scenes of up to the mid slab, a 128-thread block above, a 512-thread
-// block for the scenes whose rows stay in L2 -- takes scenes from its size class's queue and sweeps them four
-// lanes per contact (s32_sweep).  The four classes' launches run concurrently on separate streams.
+// Execution.  A team takes scenes from its size class's queue: one warp for scenes of up to the mid slab (s32_sweep), a
+// 128-thread block above (s32_sweep_turns), a 512-thread block for the scenes whose rows stay in L2 (s32_sweep_ring, or
+// s32_sweep when there are too many bodies for the ring).  The four classes' launches run concurrently on separate streams.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kQueueFp32 = 5;                        // counters[5..8]: scene queues of the four size classes
 constexpr int kClassEnd32 = 9;                       // counters[9..12]: end of each class's range in list32
@@ -2523,9 +2523,11 @@ struct S32Scene {
     int K, n_free, n_steps, warps;
 };
 // The rows of a scene too large for a slab stay in L2.  When the slab has room for them beside the bodies, the impulses
-// and the indices, they come through a ring of six steps' records, copied four steps ahead (s32_sweep_ring).
-constexpr int kRingSteps = 6, kRingAhead = 4, kRingWarps = 4;
-constexpr int kRingSlot = 8 * kRingWarps * (int)sizeof(float) * kS32Floats;
+// and the indices, they come through a ring of six steps' records, three of each group, copied four steps ahead
+// (s32_sweep_ring).
+constexpr int kRingSteps = 6, kRingWarps = 4;
+constexpr int kRingRecord = 192;   // a record without its impulses
+constexpr int kRingSlot = 8 * kRingWarps * kRingRecord;
 constexpr uint32_t kStep32Ends = 1u << 31, kStep32Wide = 1u << 30;
 constexpr uint32_t kStep32Turns = 1u << 29;   // the next step is of the other width
 __host__ __device__ inline size_t s32_align(size_t v) { return (v + 15) & ~size_t(15); }
@@ -3143,109 +3145,138 @@ __device__ __noinline__ void s32_sweep_turns(const S32Scene f, float rscale, int
 }
 constexpr int kTurnsSteps = 5;
 
-// The narrow steps of s32_sweep for a scene whose rows come through the ring: a step's records, contiguous in level
-// order, are copied into its slot four steps ahead by a warp of their own (asynchronous 16-byte copies, one group a
-// step; at a step's end the copies of the next but one are waited for, and the step's barrier shows them to all).  With the rows read from L2 by the lanes that need them a
-// step is bound by L2's latency and the uncoalesced loads: 200 sweeps and their tests over 1565 contacts took 9228 us,
-// through the ring 6376 (copied by the sweeping warps themselves 8400).
+// The float4 of w that lane q updates, of the four that it has.  With two groups of four warps the shared-memory pipe is
+// what a step waits for, and loading it again costs more than the choice (570 against 517 cycles a step); with two groups
+// of one or two warps it is the other way round (424 against 434).
+__device__ __forceinline__ float4 s32_own(int q, float4 l0, float4 l1, float4 h0, float4 h1) {
+    const bool hi = q & 1, linear = q < 2;
+    return make_float4(linear ? (hi ? h0.x : l0.x) : (hi ? h1.x : l1.x), linear ? (hi ? h0.y : l0.y) : (hi ? h1.y : l1.y),
+                       linear ? (hi ? h0.z : l0.z) : (hi ? h1.z : l1.z), linear ? (hi ? h0.w : l0.w) : 0.0f);
+}
+
+// The narrow steps of s32_sweep_turns for a scene whose rows come through the ring.  Each group has three of its slots and
+// a warp that copies its steps' records, contiguous in level order, into them (asynchronous 16-byte copies, one group a
+// step): a step's records are asked for two of the group's own steps ahead, four of the sweep's.  A barrier of the group
+// and its copying warp tells the one that the rows are there and the other that the slot before is free: a group has all
+// of a step's rows in registers before it waits for its turn.  A scene comes here with more than 600 contacts (its copy
+// is too large for a slab), so a sweep has more steps than kTurnsSteps.
+//
+// Bound by the shared-memory pipe of its SM: a warp's step takes about 80 wavefronts of 128 bytes, and eight warps share
+// the pipe with the copies.  1566 contacts in 80 steps: 517 cycles a step; 687 with the records as they lie in L2 (13
+// float4s apart, two of a quad's columns in one bank), and as much with all four warps on every step and one ring.
+//
+// A group of four pieces (lin, ang_lo, ang_hi of the four rows) is kept turned by its number, so that neither the quads'
+// loads of a row each nor those of a column, of two contacts at a time, meet twice in a bank.
+__host__ __device__ constexpr uint32_t ring_piece(int group, int row) { return 64u * group + 16u * ((row + group) & 3); }
+__device__ __forceinline__ void ring_sync(int group) {   // written with their numbers, as in turn_wait
+    if (group) asm volatile("bar.sync 4, %0;" ::"n"(32 * kRingWarps + 32) : "memory");
+    else asm volatile("bar.sync 3, %0;" ::"n"(32 * kRingWarps + 32) : "memory");
+}
 __device__ __noinline__ void s32_sweep_ring(const S32Scene f, float rscale, int n_sweeps) {
-    const ShPtr body(f.body), lohi(f.lohi), xp(f.x), ring(f.ring);
+    constexpr int half = 32 * kRingWarps, kPlaces = kRingSteps / 2;
     const GlPtr steps(f.steps);
-    const SubGroup g{32 * (kRingWarps + 1)};
-    const int rank = threadIdx.x, q = rank & 3, slot = rank >> 2, last = f.n_steps - 1;
-    const bool linear = q < 2;
-    const uint32_t hi_shift = (q & 1) ? 16u : 0u;
-    const uint32_t fixed_bit = 0x8000u << hi_shift;
-    const uint32_t part = linear ? 0u : 16u;
-    const uint32_t col = linear ? 0u : 64u * (uint32_t)(q - 1);
-    const float sg = q == 1 ? -1.0f : 1.0f;
-    auto step = [&](int j) { return (steps + 4u * j).u32(); };
-    auto after = [&](int j) { return j < last ? j + 1 : 0; };
-    auto at = [&](uint32_t st) { return min((int)(st & 0x7fffu) + slot, f.K - 1); };
-    auto record = [&](int place) { return ring + ((uint32_t)kRingSlot * place + kC32 * slot); };
-    auto copy = [&](uint32_t st, int place) {   // a step's records to its slot, 13 pieces each
-        const char* from = f.c + (size_t)kC32 * (st & 0x7fffu);
-        const int pieces = 13 * (int)((st >> 16) & 0x1fffu);
-        const uint32_t to = (ring + (uint32_t)kRingSlot * place).p;
-        for (int t = threadIdx.x & 31; t < pieces; t += 32)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16u * t), "l"(from + 16 * (size_t)t) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    auto next_place = [&](int p) { return p + 1 < kRingSteps ? p + 1 : 0; };
-    const int total = n_sweeps * f.n_steps;
-    if (rank >= 32 * kRingWarps) {   // the copying warp
-        int ja = 0, place = 0;
-        for (int k = 0; k < kRingAhead; ++k) { copy(step(ja), place); ja = after(ja); place = next_place(place); }
-        asm volatile("cp.async.wait_group 2;" ::: "memory");
-        g.sync();
-        for (int left = total; left > 0; --left) {
-            copy(step(ja), place);
-            ja = after(ja);
+    const int n_steps = f.n_steps, total = n_sweeps * n_steps;
+    auto on = [&](int step) { return step + 2 < n_steps ? step + 2 : step + 2 - n_steps; };
+    auto next_place = [&](int p) { return p + 1 < kPlaces ? p + 1 : 0; };
+    if (threadIdx.x >= 2 * half) {   // a group's copying warp
+        const int group = ((int)threadIdx.x - 2 * half) >> 5, lane = threadIdx.x & 31;
+        const ShPtr ring = ShPtr(f.ring) + (uint32_t)kRingSlot * (kPlaces * group);
+        int step = group, place = 0;
+        uint32_t st = (steps + 4u * step).u32();
+        uint32_t src[3], dst[3];   // three times 32 pieces are those of eight records
+        for (int a = 0; a < 3; ++a) {
+            const int t = lane + 32 * a, r = t / 12, p = t % 12;
+            src[a] = kC32 * r + 16u * p;
+            dst[a] = kRingRecord * r + ring_piece(p >> 2, p & 3);
+        }
+        auto copy = [&]() {   // the records of the group's next step
+            const char* from = f.c + (size_t)kC32 * (st & 0x7fffu);
+            const int pieces = 12 * (int)((st >> 16) & 0x1fffu);
+            step = on(step);
+            st = (steps + 4u * step).u32();
+            const uint32_t to = (ring + (uint32_t)kRingSlot * place).p;
+#pragma unroll
+            for (int m = 0; m < 3 * kRingWarps; ++m)
+                if (lane + 32 * m < pieces)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::
+                                 "r"(to + dst[m % 3] + 8 * kRingRecord * (m / 3)), "l"(from + src[m % 3] + 8 * kC32 * (m / 3)) : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
             place = next_place(place);
-            asm volatile("cp.async.wait_group 2;" ::: "memory");
-            g.sync();
+        };
+        copy();
+        copy();
+        for (int j = group; j < total; j += 2) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            ring_sync(group);
+            copy();
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         return;
     }
-    g.sync();
-    int place1 = 1;   // slot of the next step
-    uint32_t st0 = step(0), st1 = step(after(0));
-    int j2 = after(after(0));
-    int i0 = at(st0), i1 = at(st1);
-    uint32_t lh = (lohi + 4u * i0).u32(), lh_next = (lohi + 4u * i1).u32();
-    ShPtr rec = record(0);
-    float4 r0 = (rec + 16u * q).f4(), r1 = (rec + (64u + 16u * q)).f4(), r2 = (rec + (128u + 16u * q)).f4();
-    float4 x = (xp + 16u * i0).f4();
-    float xq = (xp + (16u * i0 + 4u * q)).f1();
+    const ShPtr body(f.body), lohi(f.lohi), xp(f.x);
+    const int group = (int)threadIdx.x >= half, rank = threadIdx.x - group * half;
+    const int q = rank & 3, slot = rank >> 2;
+    const ShPtr ring = ShPtr(f.ring) + (uint32_t)(kRingSlot * (kPlaces * group) + kRingRecord * slot);
+    const bool linear = q < 2;
+    const uint32_t hi_shift = (q & 1) ? 16u : 0u;
+    const uint32_t fixed_bit = 0x8000u << hi_shift;
+    const uint32_t part = linear ? 0u : 16u;
+    const float sg = q == 1 ? -1.0f : 1.0f;
+    const uint32_t row0 = ring_piece(0, q), row1 = ring_piece(1, q), row2 = ring_piece(2, q);
+    const int cg = linear ? 0 : q - 1;   // the group of pieces whose columns the lane sums
+    const uint32_t col0 = ring_piece(cg, 0), col1 = ring_piece(cg, 1), col2 = ring_piece(cg, 2), col3 = ring_piece(cg, 3);
+    auto at = [&](uint32_t st) { return min((int)(st & 0x7fffu) + slot, f.K - 1); };
+    int step = group, place = 0;
+    uint32_t st_next = (steps + 4u * step).u32();
+    int i_next = at(st_next);
+    uint32_t lh_next = (lohi + 4u * i_next).u32();
 #pragma unroll 1
-    for (int left = total; left > 0; --left) {
+    for (int j = group; j < total; j += 2) {
+        const uint32_t st = st_next, lh = lh_next;
+        const int i = i_next;
+        step = on(step);
+        st_next = (steps + 4u * step).u32();
         const ShPtr Bl = body + kB32 * (lh & 0x7fffu), Bh = body + kB32 * ((lh >> 16) & 0x7fffu);
-        const float4 l0 = Bl.f4(), h0 = Bh.f4(), l1 = (Bl + 16u).f4(), h1 = (Bh + 16u).f4();
-        const float zq = xq - rscale * r1.w * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
-        float z[4];
-        quad_gather(zq, z);
-        const ShPtr cl = rec + col;
-        const float4 v0 = cl.f4(), v1 = (cl + 16u).f4(), v2 = (cl + 32u).f4(), v3 = (cl + 48u).f4();
         const ShPtr B = body + kB32 * ((lh >> hi_shift) & 0x7fffu);
-        const float4 own = (B + part).f4();
+        const bool mine = slot < (int)((st >> 16) & 0x1fffu), put = mine && !(lh & fixed_bit);
+        const ShPtr rec = ring + (uint32_t)kRingSlot * place;
+        place = next_place(place);
+        ring_sync(group);
+        const float4 r0 = (rec + row0).f4(), r1 = (rec + row1).f4(), r2 = (rec + row2).f4();
+        const float xq = (xp + (16u * i + 4u * q)).f1();
+        const float4 v0 = (rec + col0).f4(), v1 = (rec + col1).f4(), v2 = (rec + col2).f4(), v3 = (rec + col3).f4();
+        const float4 x = (xp + 16u * i).f4();
         const float4 I0 = (B + 32u).f4();
         const float2 I1 = (B + 48u).f2();
+        const float wxy = linear ? 0.0f : I0.y, wxz = linear ? 0.0f : I0.z, wyz = linear ? 0.0f : I1.x;
+        const float rs = rscale * r1.w;
+        i_next = at(st_next);
+        lh_next = (lohi + 4u * i_next).u32();
+        if (j > 0) turn_wait(group, 2 * half);
+        const float4 l0 = Bl.f4(), h0 = Bh.f4(), l1 = (Bl + 16u).f4(), h1 = (Bh + 16u).f4();
+        const float zq = xq - rs * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
+        float z[4];
+        quad_gather(zq, z);
+        const float4 own = s32_own(q, l0, l1, h0, h1);
+        const float m = sg * own.w;
+        const float wxx = linear ? m : I0.x, wyy = linear ? m : I0.w, wzz = linear ? m : I1.y;
         const float xn = fmaxf(z[0], 0.0f);
         const float radius = r2.w * xn;
         const float sqr = fmaf(z[1], z[1], fmaf(z[2], z[2], z[3] * z[3]));
         float scale = sqr > radius * radius ? radius * rsqrtf(sqr) : 1.0f;
         if (xn <= 0.0f) scale = 0.0f;
-        const uint32_t st2 = step(j2);
-        j2 = after(j2);
-        const ShPtr rec_next = record(place1);
-        r0 = (rec_next + 16u * q).f4(); r1 = (rec_next + (64u + 16u * q)).f4(); r2 = (rec_next + (128u + 16u * q)).f4();
         const float f1 = z[1] * scale, f2 = z[2] * scale, f3 = z[3] * scale;
         const float d0 = xn - x.x, d1 = f1 - x.y, d2 = f2 - x.z, d3 = f3 - x.w;
-        const float yq = q == 0 ? xn : zq * scale;
-        const float m = sg * own.w;
-        const float wxx = linear ? m : I0.x, wxy = linear ? 0.0f : I0.y, wxz = linear ? 0.0f : I0.z;
-        const float wyy = linear ? m : I0.w, wyz = linear ? 0.0f : I1.x, wzz = linear ? m : I1.y;
         const float S0 = fmaf(v3.x, d3, fmaf(v2.x, d2, fmaf(v1.x, d1, v0.x * d0)));
         const float S1 = fmaf(v3.y, d3, fmaf(v2.y, d2, fmaf(v1.y, d1, v0.y * d0)));
         const float S2 = fmaf(v3.z, d3, fmaf(v2.z, d2, fmaf(v1.z, d1, v0.z * d0)));
         const float4 n = make_float4(own.x + fmaf(wxx, S0, fmaf(wxy, S1, wxz * S2)),
                                      own.y + fmaf(wxy, S0, fmaf(wyy, S1, wyz * S2)),
                                      own.z + fmaf(wxz, S0, fmaf(wyz, S1, wzz * S2)), own.w);
-        const bool mine = slot < (int)((st0 >> 16) & 0x1fffu);
-        if (mine && !(lh & fixed_bit)) (B + part).set(n);
-        if (mine) (xp + (16u * i0 + 4u * q)).set(yq);
-        // after the stores: a scene of one step sweeps the same contacts again
-        x = (xp + 16u * i1).f4();
-        xq = (xp + (16u * i1 + 4u * q)).f1();
-        g.sync();   // and the next but one step's rows are there
-        st0 = st1; st1 = st2;
-        place1 = next_place(place1);
-        rec = rec_next;
-        lh = lh_next;
-        i0 = i1;
-        i1 = at(st1);
-        lh_next = (lohi + 4u * i1).u32();
+        if (put) (B + part).set(n);
+        if (j + 1 < total) turn_done(group, 2 * half);
+        if (mine) (xp + (16u * i + 4u * q)).set(q == 0 ? xn : zq * scale);
+        __syncwarp();   // a quad's impulses are stored by its four lanes and loaded by each of them
     }
 }
 
@@ -3255,7 +3286,7 @@ __device__ __forceinline__ void s32_sweep_team(const G& g, const S32Scene& f, fl
     if (std::is_same_v<G, WarpGroup>) {
         s32_sweep<P>(WarpGroup{}, f, rscale, n_sweeps);
     } else if (std::is_same_v<P, GlPtr> && f.ring) {
-        if (threadIdx.x < 32 * (kRingWarps + 1)) s32_sweep_ring(f, rscale, n_sweeps);
+        if (threadIdx.x < 64 * (kRingWarps + 1)) s32_sweep_ring(f, rscale, n_sweeps);
     } else if (std::is_same_v<P, ShPtr> && f.n_steps >= kTurnsSteps) {
         if ((int)threadIdx.x < 64 * f.warps) s32_sweep_turns(f, rscale, n_sweeps);
     } else if (f.warps == 1) {
@@ -3518,8 +3549,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_solve_fp32(const StepArgs a, in
             scratch = reinterpret_cast<int16_t*>(f.c);
         } else {
             const size_t off = (s32_bytes(K, nr, true, bodies_global) + 15) & ~size_t(15);
-            if (ring && s32_level_scratch(K) <= (size_t)kRingSteps * kRingSlot) scratch = reinterpret_cast<int16_t*>(f.ring);
-            else if (!ring && off + s32_level_scratch(K) <= slab) scratch = reinterpret_cast<int16_t*>(my_slab + off);
+            if (ring) scratch = reinterpret_cast<int16_t*>(f.x);   // 16 bytes a contact and the ring after them
+            else if (off + s32_level_scratch(K) <= slab) scratch = reinterpret_cast<int16_t*>(my_slab + off);
         }
         const int L = s32_load(a, g, R, s, f, coloured, kL2, scratch);
         if (g.rank() == 0) a.ws.nlev[s] = L;
