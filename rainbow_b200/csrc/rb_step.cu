@@ -3146,7 +3146,7 @@ __device__ __noinline__ void s32_sweep_turns(const S32Scene f, float rscale, int
 constexpr int kTurnsSteps = 5;
 
 // The float4 of w that lane q updates, of the four that it has.  With two groups of four warps the shared-memory pipe is
-// what a step waits for, and loading it again costs more than the choice (570 against 517 cycles a step); with two groups
+// what a step waits for, and loading it again costs more than the choice (clock-counted 570 against 517 cycles a step); with two groups
 // of one or two warps it is the other way round (424 against 434).
 __device__ __forceinline__ float4 s32_own(int q, float4 l0, float4 l1, float4 h0, float4 h1) {
     const bool hi = q & 1, linear = q < 2;
@@ -3162,8 +3162,9 @@ __device__ __forceinline__ float4 s32_own(int q, float4 l0, float4 l1, float4 h0
 // is too large for a slab), so a sweep has more steps than kTurnsSteps.
 //
 // Bound by the shared-memory pipe of its SM: a warp's step takes about 80 wavefronts of 128 bytes, and eight warps share
-// the pipe with the copies.  1566 contacts in 80 steps: 517 cycles a step; 687 with the records as they lie in L2 (13
-// float4s apart, two of a quad's columns in one bank), and as much with all four warps on every step and one ring.
+// the pipe with the copies.  1566 contacts in 80 steps, 200 sweeps and their tests: 5540 us, 6250 with the records as they
+// lie in L2 (13 float4s apart, two of a quad's columns in one bank), 6310 with all four warps on every step and one ring.
+// (Clock-counted copies of the kernel, whose registers fall otherwise: 517 cycles a step, 687 with records as in L2.)
 //
 // A group of four pieces (lin, ang_lo, ang_hi of the four rows) is kept turned by its number, so that neither the quads'
 // loads of a row each nor those of a column, of two contacts at a time, meet twice in a bank.
@@ -3254,10 +3255,10 @@ __device__ __noinline__ void s32_sweep_ring(const S32Scene f, float rscale, int 
         lh_next = (lohi + 4u * i_next).u32();
         if (j > 0) turn_wait(group, 2 * half);
         const float4 l0 = Bl.f4(), h0 = Bh.f4(), l1 = (Bl + 16u).f4(), h1 = (Bh + 16u).f4();
+        const float4 own = s32_own(q, l0, l1, h0, h1);
         const float zq = xq - rs * (s32_jw(r0, r1, r2, l0, l1, h0, h1) + r0.w);
         float z[4];
         quad_gather(zq, z);
-        const float4 own = s32_own(q, l0, l1, h0, h1);
         const float m = sg * own.w;
         const float wxx = linear ? m : I0.x, wyy = linear ? m : I0.w, wzz = linear ? m : I1.y;
         const float xn = fmaxf(z[0], 0.0f);
