@@ -2922,7 +2922,9 @@ __device__ __noinline__ void s32_sweep(const G g, const S32Scene f, float rscale
                 const bool mine = slot < (int)((st0 >> 16) & 0x1fffu);
                 if (mine && !(lh & fixed_bit)) (B + part).set(n);
                 if (mine) (rec + (kX32 + 4u * q)).set(yq);
-                // after the stores: a scene of one step sweeps the same contacts again
+                // after the stores of all four lanes: a scene of one step sweeps the same contacts again, and each lane
+                // loads what the other three of its quad stored
+                __syncwarp();
                 x = (rec_next + kX32).f4();
                 xq = (rec_next + (kX32 + 4u * q)).f1();
                 if (st0 & kStep32Ends) g.sync();
