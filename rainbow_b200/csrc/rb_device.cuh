@@ -127,11 +127,18 @@ __device__ __forceinline__ void prox_sphere(double zs, double zt, double ztau, d
     o[0] = zs * scale; o[1] = zt * scale; o[2] = ztau * scale;
 }
 
+// whether two positive doubles, given by their high words, both lie in 2^+-500: the sequences below then keep their
+// residuals exact (0x20b: the exponent field of 2^-500; 0x3e8: 1000 binades)
+__device__ __forceinline__ bool mid_range(int hi_a, int hi_v) {
+    return max((unsigned)hi_a - 0x20b00000u, (unsigned)hi_v - 0x20b00000u) <= 0x3e800000u;
+}
 // a / sqrt(v) with both operations rounded to nearest, as one chain without calls: from the hardware's estimate
 // of 1 / sqrt(v), Goldschmidt's coupled iteration for sqrt(v) and 1 / (2 sqrt(v)) with the final correction by the
 // exact residual, then one Newton step to the rounded reciprocal of the root and the quotient corrected by its exact
-// residual (Markstein, IBM J. Res. Dev. 34, 1990; Cornea, Harrison, Tang, 2002).  Operands outside 2^+-500, zeros and
-// NaN among them, take the plain operations.
+// residual (Markstein, IBM J. Res. Dev. 34, 1990; Cornea, Harrison, Tang, 2002).  The reciprocal may come out on the
+// wrong side for a root just below a power of two (Markstein's exception, a mantissa of all ones), and matters to the
+// quotient only there: such roots, and operands outside 2^+-500, negative ones, zeros and NaN among them, take the
+// plain operations.
 __device__ __forceinline__ double ratio_sqrt(double a, double v) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
@@ -145,8 +152,7 @@ __device__ __forceinline__ double ratio_sqrt(double a, double v) {
     y = fma(fma(-root, y, 1.0), y, y);
     double q = a * y;
     q = fma(fma(-root, q, a), y, q);
-    const unsigned ev = (unsigned)__double2hiint(v) - 0x20b00000u, ea = (unsigned)__double2hiint(a) - 0x20b00000u;
-    if (max(ev, ea) > 0x3e800000u) q = a / sqrt(v);   // (exponent field + 500 - 1023) of either beyond 1000
+    if (!mid_range(__double2hiint(a), __double2hiint(v)) || (unsigned)__double2loint(root) >= 0xffffff00u) q = a / sqrt(v);
     return q;
 }
 
@@ -176,11 +182,13 @@ __device__ __forceinline__ GridView load_grid(const double* meta, const double* 
     return g;
 }
 // n / d from d's rounded reciprocal: the product corrected by its exact residual, which rounds as the division does
-// (Markstein, IBM J. Res. Dev. 34, 1990).  A quotient outside 1e+-250, zero and NaN among them, is divided.
+// (Markstein, IBM J. Res. Dev. 34, 1990: the product is one of the two doubles next to a quotient that lies close to
+// halfway between them).  A dividend or quotient outside 2^+-500, zero and NaN among them, is divided: with both inside,
+// the divisor's reciprocal and the residual are normal numbers.
 __device__ __forceinline__ double quotient(double n, double d, double inv) {
     const double q = n * inv;
     const double c = fma(fma(-q, d, n), inv, q);
-    return fabs(c) > 1e-250 && fabs(c) < 1e250 ? c : n / d;
+    return mid_range(__double2hiint(n) & 0x7fffffff, __double2hiint(c) & 0x7fffffff) ? c : n / d;
 }
 // grid3.py:107 get_enclosing_cell_idx (floor, then clip to [0, n-2]); a quotient that the reciprocal leaves within
 // 1e-7 of a whole number is divided
