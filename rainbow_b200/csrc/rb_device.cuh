@@ -156,6 +156,19 @@ __device__ __forceinline__ double ratio_sqrt(double a, double v) {
     return q;
 }
 
+// sqrt(v) of a positive normal v as one chain without calls: one Goldschmidt iteration from the hardware's estimate, then
+// the correction by the residual (Markstein, as above).  The root is right to 2^-39 before the correction and to 2^-76
+// after it, so the result is the rounded root, or its neighbour where the exact one is that near to halfway between two
+// doubles.  NaN for zero and for what the estimate flushes or overflows on.
+__device__ __forceinline__ double sqrt_chain(double v) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+    double g = v * y, h = 0.5 * y;
+    const double r = fma(-g, h, 0.5);
+    g = fma(g, r, g); h = fma(h, r, h);
+    return fma(fma(-g, g, v), h, g);
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // Signed distance grid (grid3.py)
 // ---------------------------------------------------------------------------------------------------------

@@ -60,24 +60,15 @@ __device__ __forceinline__ void solid_angle(d3 A, d3 B, d3 C, double la, double 
     den = la * lb * lc + dot(A, B) * lc + dot(B, C) * la + dot(C, A) * lb;
 }
 
-// the same from lengths to 2^-39, with fused products; |A|^2 and so on come in a2, b2, c2
+// the same from the squares of the lengths, with fused products
 __device__ __forceinline__ double dot_fused(d3 a, d3 b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
-__device__ __forceinline__ double sqrt_near(double v);
-__device__ __forceinline__ void solid_angle_near(d3 A, d3 B, d3 C, double a2, double b2, double c2, double& size,
-                                                 double& num, double& den) {
-    const double la = sqrt_near(a2), lb = sqrt_near(b2), lc = sqrt_near(c2);
+__device__ __forceinline__ void solid_angle_fused(d3 A, d3 B, d3 C, double a2, double b2, double c2, double& size,
+                                                  double& num, double& den) {
+    const double la = rb::sqrt_chain(a2), lb = rb::sqrt_chain(b2), lc = rb::sqrt_chain(c2);
     const d3 n = d3{fma(B.y, C.z, -(B.z * C.y)), fma(B.z, C.x, -(B.x * C.z)), fma(B.x, C.y, -(B.y * C.x))};
     num = dot_fused(A, n);
     size = la * lb * lc;
     den = fma(dot_fused(C, A), lb, fma(dot_fused(B, C), la, fma(dot_fused(A, B), lc, size)));
-}
-
-// sqrt(v) to about 2^-39: the hardware's estimate of 1 / sqrt(v) and one Newton step
-__device__ __forceinline__ double sqrt_near(double v) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
-    const double g = v * y;
-    return fma(g, fma(-g, 0.5 * y, 0.5), g);
 }
 
 // one tile of triangles in shared memory: corners, and a sphere around each (centroid, radius)
@@ -110,12 +101,13 @@ __device__ __forceinline__ void sdf_tile(SdfTile& tile, const double* __restrict
 //
 // Bound by FP64 arithmetic over (node, triangle) pairs.  The sign needs only whether |w| > 1/2, so the solid angles are
 // not summed as arcs: their complex numbers are multiplied, the turns across the negative real axis counted, and one
-// arc taken at the end (exponents are taken out on the way), with lengths to 2^-39.  A node so near an
-// edge of a triangle that its number's modulus is below 1e-4 of its scale, or with a sum within 1e-3 of the threshold,
-// takes the plain sum (a factor's angle is otherwise right to 1e-7, w with 16384 of them to 3e-4).  The distance's
-// minimum is taken over squares, and a triangle is passed over when the sphere around it is farther than the
-// nearest vertex or point so far.  Both give the values of the plain form: an arc, four roots and the closest point
-// for every triangle took 11.5 ms for 96 grids of 32^3 around boxes and 448-triangle spheres, this one 5.5.
+// arc taken at the end (exponents are taken out on the way).  A node so near an edge of a triangle that its number's
+// modulus is below 1e-4 of its scale, or with a sum within 1e-3 of the threshold, takes the plain sum (a factor's angle
+// is otherwise right to 1e-11, w with any number of triangles that memory holds to 1e-3).  The distance's minimum is
+// taken over squares, and a triangle is passed over when the sphere around it is farther than the nearest vertex or
+// point so far.  Both give the values of the plain form: an arc, four roots and the closest point for every triangle
+// took 11.8 ms a pass for 96 grids of 32^3 around boxes and 448-triangle spheres, this one 6.1 (5.8 with lengths to
+// 2^-39 only, which bounded w to 3e-4 for 16384 triangles and not at all for more).
 __device__ __forceinline__ void sdf_node(const double* __restrict__ V, const int32_t* __restrict__ T, int n_tri,
                                          const double* __restrict__ meta, int64_t node, double* __restrict__ values) {
     __shared__ SdfTile tile;
@@ -141,7 +133,7 @@ __device__ __forceinline__ void sdf_node(const double* __restrict__ V, const int
             const double a2 = dot_fused(A, A), b2 = dot_fused(B, B), c2 = dot_fused(C, C);
             near2 = fmin(near2, fmin(a2, fmin(b2, c2)));
             double size, num, den;
-            solid_angle_near(A, B, C, a2, b2, c2, size, num, den);
+            solid_angle_fused(A, B, C, a2, b2, c2, size, num, den);
             // (so put that a NaN is unsure; a zero imaginary part left of zero has no side)
             unsure |= !(fabs(num) + fabs(den) >= 1e-4 * size) || (num == 0.0 && den < 0.0);
             const double r = fma(re, den, -(im * num)), m = fma(re, num, im * den);

@@ -13,6 +13,10 @@ __global__ void k_quotient(const double* a, const double* d, double* out, int n)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = rb::quotient(a[i], d[i], 1.0 / d[i]);
 }
+__global__ void k_sqrt_chain(const double* v, double* out, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = rb::sqrt_chain(v[i]);
+}
 
 }  // namespace
 
@@ -20,7 +24,8 @@ __global__ void k_quotient(const double* a, const double* d, double* out, int n)
 extern "C" int rounding(int what, const double* a, const double* b, double* out, int n) {
     const int blocks = (n + 255) / 256;
     if (what == 0) k_ratio_sqrt<<<blocks, 256>>>(a, b, out, n);
-    else k_quotient<<<blocks, 256>>>(a, b, out, n);
+    else if (what == 1) k_quotient<<<blocks, 256>>>(a, b, out, n);
+    else k_sqrt_chain<<<blocks, 256>>>(a, out, n);
     const cudaError_t e = cudaGetLastError();
     return (int)(e != cudaSuccess ? e : cudaDeviceSynchronize());
 }

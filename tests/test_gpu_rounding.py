@@ -127,3 +127,16 @@ def test_quotient(device_fn):
     d = np.concatenate([d, s[1], _random(rng, m, -1022, 1023), _random(rng, m, -3, 3), small[1], large[1]])
     with np.errstate(all="ignore"):
         _same(device_fn(1, n, d), n / d, n, d)
+
+
+def test_sqrt_chain(device_fn):
+    """Right to half a unit in the last place and the ~2^-23 of one that its last correction leaves: the rounded root on all
+    but a 2^-22 share of operands, and never further off than its neighbour."""
+    rng = np.random.default_rng(2)
+    squares = _hard_squares()
+    v = np.concatenate([squares, 4.0 - 2.0 ** -51 * np.arange(0, 400), rng.uniform(1.0, 4.0, 1 << 20)])
+    v = np.concatenate([v, v * 4.0 ** rng.integers(-500, 500, len(v))])
+    got, want = device_fn(2, v, v), np.sqrt(v)
+    assert np.abs(got.view(np.int64) - want.view(np.int64)).max() <= 1
+    assert (got != want).sum() <= 2 * (len(squares) + 400) + 8
+    assert np.isnan(device_fn(2, np.zeros(1), np.zeros(1))).all()
