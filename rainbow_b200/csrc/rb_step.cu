@@ -3562,17 +3562,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_solve_fp32(const StepArgs a, in
         int sweeps = 0, stalls = 0, window = kS32StallTests;
         // far above the tolerance (and the stall floor) the residual is tested half as often: no stop and no
         // stall can be decided there, and each test rebuilds w
-        auto gap = [&](float r) { return r > kS32FarFactor * tol ? 2 * interval : interval; };
-        int next_test = gap(res);
+        // (unsigned: twice any interval fits)
+        auto gap = [&](float r) { return r > kS32FarFactor * tol ? 2u * (unsigned)interval : (unsigned)interval; };
+        unsigned next_test = gap(res);
+        // sweeps of one call, whose steps are counted in 32 bits
+        const unsigned most = (unsigned)(INT_MAX / f.n_steps);
         double r64 = -1.0;            // FP64 residual of the current iterate, once evaluated
         double r64_round = INFINITY;  // FP64 residual after the previous correction round
         for (;;) {
             const int round_start = sweeps;
             while (res > tol && sweeps < budget) {
-                const int n = jacobi ? 1 : min(next_test, budget - sweeps);   // as far as the next test
+                // as far as the next test
+                const unsigned n = jacobi ? 1u : min(min(next_test, (unsigned)(budget - sweeps)), most);
                 if (jacobi) s32_sweep_jacobi<P>(g, f, rscale, hybrid);
-                else s32_sweep_team<P>(g, f, rscale, n);
-                sweeps += n;
+                else s32_sweep_team<P>(g, f, rscale, (int)n);
+                sweeps += (int)n;
                 next_test -= n;
                 if (next_test == 0 || sweeps == budget) {
                     res = s32_residual<P>(g, f);

@@ -79,3 +79,15 @@ def test_sweeps_of_one_step(count):
     assert np.abs(sol[:, 1:]).max() > 0.0   # friction is at work
     np.testing.assert_allclose(sol, sol64, rtol=0.0, atol=4e-5 * np.abs(sol64).max())
     np.testing.assert_allclose(u, u64, rtol=0.0, atol=4e-5 * np.abs(u64).max())
+
+
+@pytest.mark.parametrize("interval", [1 << 30, (1 << 31) - 1])
+def test_residual_intervals_beyond_the_sweeps(interval):
+    """A residual test spaced further than the sweeps of a step can go, up to the largest number the parameter holds, is
+    made at their end only: the same bits as any interval beyond the cap."""
+    a = chips(20)
+    u, st, sol = step(a, 40, interval=interval)
+    u1, st1, sol1 = step(a, 40, interval=1000)
+    assert st.fp32_sweeps == st1.fp32_sweeps == 40 and st.n_contacts == 20
+    np.testing.assert_array_equal(sol, sol1)
+    np.testing.assert_array_equal(u, u1)
