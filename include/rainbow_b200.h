@@ -79,12 +79,12 @@ typedef struct rb_shapes {
     const int64_t* g_off;       /* n_shapes+1 value offsets */
     const double* grid_meta;    /* 12 doubles per shape: min[3], max[3], spacing[3], I, J, K (grid3.py:16) */
     int32_t max_shape_triangles; /* triangles of the largest shape (at most 16384) */
-    const float* grid32;        /* optional FP32 copy of grid (same offsets), or NULL.  With it, a profiled step
-                                   of the FP32 precision modes runs the contact search's signed distance lookups
-                                   (the seed and Frank-Wolfe iterations, collision_detection.py:134-165) in FP32
-                                   and counts them; near-ties, the acceptance tests and the contact's point,
-                                   normal and gap (:172-188) stay FP64, so it finds the contacts that the other
-                                   steps' FP64 search finds */
+    const float* grid32;        /* optional FP32 copy of grid (same offsets), or NULL.  With it, a step of the FP32
+                                   precision modes with profiling bit 2 runs the contact search's signed distance
+                                   lookups (the seed and Frank-Wolfe iterations, collision_detection.py:134-165)
+                                   in FP32, counts them and checks the decisions; near-ties, the acceptance tests
+                                   and the contact's point, normal and gap (:172-188) stay FP64, so it finds the
+                                   contacts that the other steps' FP64 search finds.  No other step reads it */
 } rb_shapes;
 
 /* Bodies of one or more independent scenes; scene s owns bodies scene_start[s] .. scene_start[s+1]-1 in the
@@ -165,9 +165,10 @@ typedef struct rb_params {
     int32_t scheme;               /* RB_SCHEME_* */
     int32_t termination;          /* RB_TERMINATE_* */
     double residual_tolerance;    /* used by RB_TERMINATE_RESIDUAL */
-    int32_t profiling;            /* nonzero: phase times, energies and residual histories; bit 2 (value 2) also
-                                     checks the FP32 modes' contact search against the plain FP64 search
-                                     (rb_scene_stats.n_search_flips / n_accept_flips) */
+    int32_t profiling;            /* nonzero: phase times, energies and residual histories; bit 2 (value 2), with
+                                     rb_shapes.grid32, runs the FP32 modes' contact search on the FP32 grids and
+                                     checks it against the plain FP64 search (rb_scene_stats.n_search_flips /
+                                     n_accept_flips): its contact search time is the check's */
     double relaxation;            /* RB_TERMINATE_RESIDUAL_FIXED_R: r = relaxation / diag (over-relaxation of the
                                      projected Gauss-Seidel update; values <= 0 mean 1) */
     int32_t residual_interval;    /* RB_TERMINATE_RESIDUAL_FIXED_R: test the residual every this many sweeps
@@ -218,8 +219,8 @@ typedef struct rb_scene_stats {
                                      choices or iteration count differ from the FP64 search's */
     int32_t n_accept_flips;       /* ... candidates the FP32 search accepts as a contact and the FP64 search does
                                      not, or the other way round */
-    int32_t n_grid_lookups32;     /* signed distance lookups of the contact search made on grid32 (profiling only;
-                                     n_grid_lookups counts the FP64 ones) */
+    int32_t n_grid_lookups32;     /* signed distance lookups of the contact search made on grid32 (profiling bit 2
+                                     only; n_grid_lookups counts the FP64 ones) */
 } rb_scene_stats;
 
 /* Outputs: device buffers sized by rb_caps.contact_capacity / n_scenes / max_iterations. */

@@ -279,7 +279,7 @@ __device__ __forceinline__ bool grid_is_inside(const GridView& g, d3 p, double b
     return true;
 }
 
-// Gradient from the FP32 copy of a grid (the contact search of the FP32 precision modes): the cell and the
+// Gradient from the FP32 copy of a grid (the contact search that profiling bit 2 checks): the cell and the
 // fractions s, t, u in FP64 (the cell is always the FP64 lookup's, grid3.py:107, and the min_coord divisor of
 // :209-211 is kept; the fractions take its reciprocal, 2^-52 off, far inside the bound), the eight corner values and their trilinear
 // combination in FP32.  err bounds the absolute difference of each component from grid_gradient's: the FP32

@@ -714,7 +714,7 @@ __device__ __forceinline__ d3 fw_search64(const GridView& g, const double* alpha
     return x;
 }
 
-// the same search with its lookups on the FP32 copy of the grid (the FP32 precision modes).  The point x and
+// the same search with its lookups on the FP32 copy of the grid (profiling bit 2 of the FP32 modes).  The point x and
 // the objectives stay FP64; a decision whose margin lies within the FP32 lookups' error bound (an exact tie of
 // coplanar corners, a near-tie, an objective next to the tolerance) is taken again on FP64 lookups, so every
 // decision, and x, equal fw_search64's.  l64 / l32 count the FP64 and FP32 lookups made.
@@ -775,7 +775,7 @@ __device__ __forceinline__ d3 fw_search_f32(const GridView& g, const float* valu
     return x;
 }
 
-// the plain FP64 search's trace and acceptance for a profiled step's check of the FP32 search (a call of its
+// the plain FP64 search's trace and acceptance for the check of the FP32 search (a call of its
 // own, so that it does not raise the registers of the search itself)
 __device__ __noinline__ void fw_check64(const GridView& g, const double* alphas, const d3* ps, const double* qB, int max_it, double tol,
                                         double envelope, int& n64, uint32_t& trace64, int& accept64) {
@@ -785,10 +785,10 @@ __device__ __noinline__ void fw_check64(const GridView& g, const double* alphas,
         accept64 = norm3_np(quat_rotate(qB, grid_gradient(g, x64))) > 0.0;
 }
 
-// kF32: the seed and Frank-Wolfe lookups on the FP32 grid copy (near-ties decided on FP64 lookups); the
-// acceptance tests (is_inside, phi <= envelope) and the contact's point, normal and gap in FP64 at the point
-// found.  A step profiled with bit 2 set also runs the plain FP64 search and counts, per scene, the candidates
-// whose search decisions or acceptance differ (a check of the error bound: zero when it holds).
+// kF32 (profiling bit 2): the seed and Frank-Wolfe lookups on the FP32 grid copy (near-ties decided on FP64 lookups);
+// the acceptance tests (is_inside, phi <= envelope) and the contact's point, normal and gap in FP64 at the point
+// found.  It also runs the plain FP64 search and counts, per scene, the candidates whose search decisions or
+// acceptance differ (a check of the error bound: zero when it holds).
 template <bool kF32>
 __global__ void __launch_bounds__(256, 2) k_narrow(const StepArgs a) {
     __shared__ double alphas[kAlphas];
@@ -858,8 +858,8 @@ __global__ void __launch_bounds__(256, 2) k_narrow(const StepArgs a) {
         if (a.pr.profiling) {   // statistics for the bandwidth accounting (lookups per scene) and decision flips
             const int s = scene_of(a.bd.scene_start, a.bd.n_scenes, A);
             atomicAdd(&a.out.stats[s].n_grid_lookups, lookups);
-            if (kF32) atomicAdd(&a.out.stats[s].n_grid_lookups32, lookups32);
-            if (kF32 && (a.pr.profiling & 2)) {   // the check against the plain FP64 search, on request
+            if (kF32) {   // the check against the plain FP64 search
+                atomicAdd(&a.out.stats[s].n_grid_lookups32, lookups32);
                 int n64 = 0, accept64 = 0;
                 uint32_t trace64 = 0u;
                 fw_check64(g, alphas, ps, qB, max_it, tol, envelope, n64, trace64, accept64);
@@ -4083,9 +4083,9 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     // narrow phase
     // The search on the FP32 grid copy makes the FP64 search's decisions (near-ties go to FP64 lookups), so it finds the
     // same contacts; with FP64 lookups rid of their divisions it is the slower one, for its error bounds and second
-    // lookups (512 piles with a grid per body 1284 against 710 us, 4096-body lattice 213 against 137).  It runs where its
-    // own statistics are asked for: the lookups on the copy and the decision flips of a profiled step.
-    if (pr->precision != RB_PRECISION_FP64 && sh->grid32 && prof) {
+    // lookups (512 piles with a grid per body 1284 against 710 us, 4096-body lattice 213 against 137).  It runs only
+    // where it is checked against the FP64 search (profiling bit 2); every other step, profiled or not, runs the latter.
+    if (pr->precision != RB_PRECISION_FP64 && sh->grid32 && (pr->profiling & 2)) {
         k_narrow<true><<<narrow_blocks, narrow_threads, 0, st>>>(a); note_launch();
     } else {
         k_narrow<false><<<narrow_blocks, narrow_threads, 0, st>>>(a); note_launch();

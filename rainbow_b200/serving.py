@@ -39,10 +39,12 @@ def _shape_key(scene, k):
 
 
 class ShapeLibrary:
-    """Shapes resident on the device for every batch of a server, stored once per distinct shape."""
+    """Shapes resident on the device for every batch of a server, stored once per distinct shape.  With grid32 there
+    is an FP32 copy of the grids too, which only steps profiled with bit 2 read (rb_shapes.grid32)."""
 
-    def __init__(self, device):
+    def __init__(self, device, grid32=False):
         self.device = torch.device(device)
+        self.grid32 = grid32
         self.index = {}
         self.V, self.T, self.G, self.meta = [], [], [], []
         self.nv, self.nt = [], []
@@ -88,13 +90,14 @@ class ShapeLibrary:
             "g_off": off([len(g) for g in self.G], np.int64).to(dev),
             "grid_meta": torch.from_numpy(np.concatenate(self.meta)).to(dev, torch.float64),
         }
-        self.t["grid32"] = self.t["grid"].float()   # the FP32 modes' contact search reads this copy
         sh = N.RbShapes()
         sh.n_shapes = len(self.V)
         for f in ("V", "v_off", "T", "t_off", "grid", "g_off", "grid_meta"):
             setattr(sh, f, self.t[f].data_ptr())
         sh.max_shape_triangles = max(self.nt)
-        sh.grid32 = self.t["grid32"].data_ptr()
+        if self.grid32:
+            self.t["grid32"] = self.t["grid"].float()
+            sh.grid32 = self.t["grid32"].data_ptr()
         self.rb_shapes = sh
         self._dirty = False
 
@@ -351,7 +354,7 @@ class Server:
         self.budget = int(hbm_fraction * total)
         self.max_active_bodies = max_active_bodies
         self.caps_per_body = list(caps_per_body)
-        self.library = ShapeLibrary(device)
+        self.library = ShapeLibrary(device, grid32=bool(rb_params.profiling & 2))
         self.pool = {}
         self._next = None          # the next tick's plan, made while the current step runs
         self.queue = deque()

@@ -297,9 +297,6 @@ class DeviceWorld:
             setattr(sh, f, T["shape_" + f].data_ptr())
         sh.grid_meta = T["shape_grid_meta"].data_ptr()
         sh.max_shape_triangles = int(np.diff(P["shape_t_off"]).max())
-        # FP32 copy of the grids for the contact search of the FP32 precision modes (FP64 steps ignore it)
-        T["shape_grid32"] = T["shape_grid"].float()
-        sh.grid32 = T["shape_grid32"].data_ptr()
         self.rb_shapes = sh
         bd = N.RbBodies()
         bd.n_bodies, bd.n_scenes = self.n_bodies, self.n_scenes
@@ -366,6 +363,11 @@ class DeviceWorld:
     def launch(self, rb_params, stream=None):
         """Enqueue one step of every scene (asynchronous; the caller checks ``status()`` when it syncs)."""
         st = stream if stream is not None else torch.cuda.current_stream(self.device)
+        if rb_params.profiling & 2 and not self.rb_shapes.grid32:   # the check's FP32 copy of the grids, made when asked for
+            with torch.cuda.stream(st):
+                self.tensors["shape_grid32"] = self.tensors["shape_grid"].float()
+            st.synchronize()   # steps on other streams may read it next
+            self.rb_shapes.grid32 = self.tensors["shape_grid32"].data_ptr()
         rc = self.lib.rb_step(ctypes.byref(self.rb_shapes), ctypes.byref(self.rb_bodies), ctypes.byref(self.caps),
                               ctypes.byref(rb_params), ctypes.byref(self.rb_outputs), self.t_ws.data_ptr(),
                               self.workspace_bytes, ctypes.c_void_p(st.cuda_stream))

@@ -91,3 +91,22 @@ def test_residual_intervals_beyond_the_sweeps(interval):
     assert st.fp32_sweeps == st1.fp32_sweeps == 40 and st.n_contacts == 20
     np.testing.assert_array_equal(sol, sol1)
     np.testing.assert_array_equal(u, u1)
+
+
+def test_profiled_steps_run_the_contact_search_of_the_others():
+    """Profiling alone does not change the kernels that are timed: an FP32 step searches the FP64 grids, with as many
+    lookups as the FP64 step's, and a world holds no FP32 copy of its grids.  Bit 2 asks for the check, which makes it."""
+    from rainbow_b200 import world as W
+    a = chips(20)
+    w = W.DeviceWorld([a], device="cuda:0", max_iterations=200)
+    x0, u0 = w.state()
+    seen = []
+    for precision, profiling in (("fp64", 1), ("fp32", 0), ("fp32", 1), ("fp32", 3)):
+        assert not w.rb_shapes.grid32
+        w.set_state(x0, u0)
+        assert w.step(W.make_rb_params(W.params_from_vector(a["params"]), precision=precision, profiling=profiling,
+                                       termination="residual_fixed_r")) == 0
+        st = w.stats()[0]
+        seen.append((st.n_grid_lookups, st.n_grid_lookups32, st.n_contacts))
+    assert seen[0] == seen[2] and seen[0][0] > 0 and seen[1] == (0, 0, 20)
+    assert seen[3][1] > 0 and w.rb_shapes.grid32
