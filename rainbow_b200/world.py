@@ -433,9 +433,10 @@ class DeviceWorld:
                                  self.t_csol[:4 * K]]
         sizes = [-(-t.numel() * t.element_size() // 64) * 64 for t in parts]
         total = sum(sizes)
-        stage = getattr(self, "h_stage", None)
+        # the staging belongs to this call until it is put back: another thread's call meanwhile makes its own
+        stage = self.__dict__.pop("h_stage", None)
         if stage is None or stage.numel() < total:
-            stage = self.h_stage = torch.empty(total + total // 2 + 4096, dtype=torch.uint8, pin_memory=True)
+            stage = torch.empty(total + total // 2 + 4096, dtype=torch.uint8, pin_memory=True)
         host, at = [], 0
         for t, size in zip(parts, sizes):
             h = stage[at:at + t.numel() * t.element_size()].view(t.dtype)
@@ -445,6 +446,7 @@ class DeviceWorld:
             at += size
         torch.cuda.current_stream(self.device).synchronize()
         out = [h.numpy().copy() for h in host]
+        self.h_stage = stage
         ids, p, n, g, sol = out[-5:]
         return out[:-5], dict(ids=ids.reshape(K, 2), p=p.reshape(K, 3), n=n.reshape(K, 3), g=g, sol=sol)
 
