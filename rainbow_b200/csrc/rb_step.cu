@@ -4116,9 +4116,15 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     const int smem_bodies = std::min(std::max(bd->max_scene_bodies, 0), kSolveSmemBodies - 1) + 1;   // + 1: fixed bodies
     const size_t block_smem = (size_t)6 * sizeof(double) * smem_bodies;
     const int bg = bd->n_scenes < 148 * 16 ? bd->n_scenes : 148 * 16;
-    // a scene that has an SM to itself takes as many warps as the registers allow (255 a thread), so that wide levels
-    // and the rebuilds of w have them; more scenes than SMs share them, two or four blocks to an SM
-    const int solve_threads = bd->n_scenes <= 148 ? kSolveBlock : bd->n_scenes <= 2 * 148 ? kSolveBlock / 2 : kSolveBlock / 4;
+    // Threads of a scene's block: a scene that has an SM to itself takes as many warps as the registers allow (255 a
+    // thread), so that wide levels and the rebuilds of w have them; more scenes than SMs share them, two or four blocks
+    // to an SM, where the accumulators leave room for as many.  A batch whose largest scene is more than four times the
+    // mean waits for that scene: it takes the most threads too.  (400 piles of up to 200 bodies and one of 5000: 454 ms a
+    // step by the number of scenes alone, 131 so; 300 of up to 40 and one of 1500: 729 and 251; 300 piles of up to 200:
+    // 73 either way, with 64 threads.)
+    const int share = (int)std::min<size_t>((bd->n_scenes + 147) / 148, (227 * 1024) / (block_smem + 2048));
+    const bool uneven = (int64_t)bd->max_scene_bodies * bd->n_scenes > 4 * (int64_t)N;
+    const int solve_threads = share <= 1 || uneven ? kSolveBlock : share == 2 ? kSolveBlock / 2 : kSolveBlock / 4;
     if (pr->precision != RB_PRECISION_FP64) {
         k_fp32_classes<<<1, 1024, 0, st>>>(a, small_slab, mid_slab); note_launch();
         // FP32 phase, four size classes side by side: warp teams with small slabs (28 KB unless tuned), warp
