@@ -1199,7 +1199,9 @@ __device__ __forceinline__ SceneRange scene_range(const StepArgs& a, int s) {
     return R;
 }
 
+// the larger one, or NaN once either is (v: the largest so far)
 __device__ __forceinline__ double nanmax(double v, double t) { return (t > v || t != t) ? t : v; }
+__device__ __forceinline__ float nanmax(float v, float t) { return (t > v || t != t) ? t : v; }
 
 struct WarpGroup {
     __device__ __forceinline__ int rank() const { return threadIdx.x & 31; }
@@ -2827,8 +2829,7 @@ __device__ __noinline__ float s32_residual(const G g, const S32Scene f) {
         const float fr = pn <= 0.0f ? 0.0f : (sqr <= radius * radius ? zq : zq * (radius * rsqrtf(sqr)));
         const float d = x - (q == 0 ? pn : fr);
         if (at < f.K) {
-            m = fmaxf(m, fabsf(d));
-            if (d != d) m = d;
+            m = nanmax(m, fabsf(d));
             xm = fmaxf(xm, fabsf(x));
         }
     }
@@ -3394,8 +3395,7 @@ __device__ __forceinline__ double s32_correct(const StepArgs& a, const G& g, con
         const int kind = prox_factor(z, a.ws.mu[k], pn, scale);
         const double d = x - (q == 0 ? pn : prox_apply(kind, scale, zq));
         if (at < K) {
-            m = fmax(m, fabs(d));
-            if (d != d) m = d;
+            m = nanmax(m, fabs(d));
             xm = fmax(xm, fabs(x));
         }
     }

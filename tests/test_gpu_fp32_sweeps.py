@@ -110,3 +110,33 @@ def test_profiled_steps_run_the_contact_search_of_the_others():
         seen.append((st.n_grid_lookups, st.n_grid_lookups32, st.n_contacts))
     assert seen[0] == seen[2] and seen[0][0] > 0 and seen[1] == (0, 0, 20)
     assert seen[3][1] > 0 and w.rb_shapes.grid32
+
+
+@pytest.mark.parametrize("count,scheme", [(40, "rigid_gauss_seidel"), (40, "parallel_jacobi"), (600, "rigid_gauss_seidel"),
+                                          (1500, "rigid_gauss_seidel")])
+@pytest.mark.parametrize("precision", ["fp32", "fp32_refine"])
+def test_a_nan_impulse_is_never_reported_as_a_residual(count, scheme, precision):
+    """One body with a NaN velocity among others: a NaN in its contact's impulses, whichever lanes and warps test it, makes
+    the residual NaN and is no convergence.  (FP32 Gauss-Seidel sweeps leave one in the friction rows; a Jacobi sweep and
+    the FP64 prox put zero there.)"""
+    from rainbow_b200 import _native as N, world as W
+    a = chips(count)
+    out = []
+    for bad in (False, True):
+        a = dict(a, body_v=a["body_v"].copy())
+        if bad:
+            a["body_v"][3] = np.nan
+        w = W.DeviceWorld([a], device="cuda:0", max_iterations=24)
+        rp = W.make_rb_params(W.params_from_vector(a["params"]), termination="residual_fixed_r", residual_tolerance=1e-6,
+                              residual_interval=4, precision=precision, scheme=scheme)
+        rp.max_iterations = 24
+        assert w.step(rp) == (N.STATUS_NONFINITE if bad else 0)
+        out.append((w.stats()[0], w.contacts()["sol"].reshape(-1, 4)))
+    (good_st, good), (bad_st, bad) = out
+    assert bad_st.n_contacts == good_st.n_contacts > count // 2
+    assert np.isfinite(good).all() and np.isfinite(good_st.residual)
+    assert np.isnan(bad).any(axis=1).sum() == (precision == "fp32" and scheme == "rigid_gauss_seidel")
+    if np.isnan(bad).any():
+        assert np.isnan(bad_st.residual) and bad_st.exitcode == 0
+    else:
+        np.testing.assert_array_equal(bad[2], 0.0)
