@@ -117,16 +117,6 @@ __device__ __forceinline__ void make_orthonormal_vectors(d3 nin, d3& t, d3& b, d
     b = d3{bb.x / lb, bb.y / lb, bb.z / lb};
     t = cross_np(b, n);
 }
-// prox_operators.py:14 prox_sphere
-__device__ __forceinline__ void prox_sphere(double zs, double zt, double ztau, double mu, double xn, double* o) {
-    if (xn <= 0.0) { o[0] = 0.0; o[1] = 0.0; o[2] = 0.0; return; }
-    const double radius = mu * xn;
-    const double sqr = zs * zs + zt * zt + ztau * ztau;
-    if (sqr <= radius * radius) { o[0] = zs; o[1] = zt; o[2] = ztau; return; }
-    const double scale = radius / sqrt(sqr);
-    o[0] = zs * scale; o[1] = zt * scale; o[2] = ztau * scale;
-}
-
 // whether two positive doubles, given by their high words, both lie in 2^+-500: the sequences below then keep their
 // residuals exact (0x20b: the exponent field of 2^-500; 0x3e8: 1000 binades)
 __device__ __forceinline__ bool mid_range(int hi_a, int hi_v) {

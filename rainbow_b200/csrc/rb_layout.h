@@ -32,8 +32,8 @@ struct Workspace {
     double* clu;         // 6 NC cluster boxes
     // pairs
     int32_t* pairs;      // 2P
-    int32_t* pair_items; // P+1 candidate triangles per pair -> offsets
-    int32_t* pair_itemsA;// P   of which from side A
+    int32_t* pair_items; // P+1 first candidate triangle of each pair
+    int32_t* pair_n_items; // P their number
     int32_t* pair_cont;  // P+1 contacts per pair -> offsets
     int32_t* pair_ovl;   // P   overlapping leaf pairs per pair (profiling statistic)
     // items
@@ -48,7 +48,8 @@ struct Workspace {
     int32_t* bc_list;    // 2K
     double* J;           // 48K
     double* WJT;         // 48K
-    float* c32;          // 52K   compact FP32 contacts of the scenes whose copy does not fit in shared memory
+    float* c32;          // 52K   compact FP32 contacts of the scenes whose copy does not fit in shared memory; the FP64
+                         //       solve of a scene keeps its per-contact metas and steps in its room
     uint32_t* blist32;   // 2K    ... their per-body contact lists
     uint16_t* pos32;     // K     ... and level-order positions
     float* body32;       // 16N   ... and, for scenes with too many bodies for the slab, their body records
@@ -78,7 +79,7 @@ struct Workspace {
     int32_t* counters;   // 16
 };
 
-enum Counter { kNPairs = 0, kNItems = 1, kNRaw = 2, kNContacts = 3, kMidNext = 4 };
+enum Counter { kNPairs = 0, kNItems = 1, kNContacts = 3, kMidNext = 4 };
 
 inline size_t align_up(size_t v) { return (v + 255) & ~size_t(255); }
 
@@ -98,7 +99,7 @@ inline size_t layout(Workspace* ws, char* base, int64_t N, int64_t NV, int64_t N
     take(w->w, 6 * N); take(w->w2, 6 * N);
     take(w->pair_cnt, N + 1); take(w->bc_ptr, N + 1); take(w->bc_fill, N);
     take(w->Vw, 3 * NV); take(w->clu, 6 * NC);
-    take(w->pairs, 2 * P); take(w->pair_items, P + 1); take(w->pair_itemsA, P); take(w->pair_cont, P + 1); take(w->pair_ovl, P);
+    take(w->pairs, 2 * P); take(w->pair_items, P + 1); take(w->pair_n_items, P); take(w->pair_cont, P + 1); take(w->pair_ovl, P);
     take(w->item_pair, C); take(w->item_tri, C); take(w->item_flag, C);
     take(w->item_p, 3 * C); take(w->item_n, 3 * C); take(w->item_g, C);
     take(w->lohi, 2 * K); take(w->bc_list, 2 * K);

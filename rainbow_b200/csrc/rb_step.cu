@@ -68,7 +68,7 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 
 // ---------------------------------------------------------------------------------------------------------
 // device-wide exclusive scan of int32 counts (three phases; the element count may live on the device)
-// data[0..n) -> exclusive prefix sums, data[n] = total, *total_out = total
+// data[0..n) -> exclusive prefix sums, data[n] = total, which ScanTotal may also put into a counter
 // ---------------------------------------------------------------------------------------------------------
 // with a device count, n_host is the capacity the count is clamped to
 __device__ __forceinline__ int scan_n(const int32_t* n_dev, int n_host) { return n_dev ? min(*n_dev, n_host) : n_host; }
@@ -420,7 +420,7 @@ __device__ __forceinline__ void mid_arrays(int max_clusters, int warp, int16_t*&
 }
 
 // writes a pair's candidates, the set bits of both sides' masks, in ascending (side, triangle) order, in room reserved
-// with one atomic: pair_items[p] = first candidate of the pair, pair_itemsA[p] = their number (one warp)
+// with one atomic: pair_items[p] = first candidate of the pair, pair_n_items[p] = their number (one warp)
 __device__ __forceinline__ void mid_emit(const StepArgs& a, int p, int nA, int nB, const int16_t* listA, const int16_t* listB,
                                          const uint32_t* maskA, const uint32_t* maskB, int n_ovl) {
     const int lane = threadIdx.x & 31;
@@ -431,7 +431,7 @@ __device__ __forceinline__ void mid_emit(const StepArgs& a, int p, int nA, int n
     int pos = 0;
     if (lane == 0) pos = atomicAdd(a.ws.counters + kNItems, cnt);
     pos = __shfl_sync(0xffffffffu, pos, 0);
-    if (lane == 0) { a.ws.pair_items[p] = pos; a.ws.pair_itemsA[p] = cnt; a.ws.pair_ovl[p] = n_ovl; }
+    if (lane == 0) { a.ws.pair_items[p] = pos; a.ws.pair_n_items[p] = cnt; a.ws.pair_ovl[p] = n_ovl; }
     if (pos + cnt > a.caps.item_capacity) return;   // k_narrow aborts the step
     for (int side = 0; side < 2; ++side) {
         const int n = side ? nB : nA;
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kBlock) k_mid(const StepArgs a, int max_cluste
             if (lane == 0) {
                 atomicOr(a.out.status, RB_STATUS_MESH_TOO_LARGE);
                 atomicOr(a.ws.counters + kAbort, RB_STATUS_MESH_TOO_LARGE);
-                a.ws.pair_items[p] = 0; a.ws.pair_itemsA[p] = 0; a.ws.pair_ovl[p] = 0;
+                a.ws.pair_items[p] = 0; a.ws.pair_n_items[p] = 0; a.ws.pair_ovl[p] = 0;
             }
             continue;
         }
@@ -888,7 +888,7 @@ __global__ void __launch_bounds__(kBlock) k_dedup(const StepArgs a) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int n_pairs = a.ws.counters[kNPairs];
     for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n_pairs; p += (gridDim.x * blockDim.x) >> 5) {
-        const int i0 = a.ws.pair_items[p], i1 = i0 + a.ws.pair_itemsA[p];
+        const int i0 = a.ws.pair_items[p], i1 = i0 + a.ws.pair_n_items[p];
         int kept = 0;
         for (int c0 = i0; c0 < i1;) {
             // the next accepted candidates, as many whole chunks of 32 as there is room for
@@ -2480,8 +2480,8 @@ __device__ void solve_scene_body(const StepArgs& a, const G& g, int s, int post,
 //
 // Compact form.  A contact's Jacobian rows are [lin_lo | ang_lo | lin_hi | ang_hi] with lin_hi = -lin_lo
 // (the frame direction, zero on the torsion row) and W J^T = (m^-1 lin, I_w^-1 ang) per body, so a contact
-// stores per row q: lin_lo (3), ang_lo (3), ang_hi (3), b, 1/diag and x -- 12 floats, 48 per contact -- and mu, in a
-// record of kS32Floats, and a body stores its accumulator w (6), m^-1, a fixed flag and the world inverse
+// stores per row q three float4s, (lin_lo, b), (ang_lo, 1/diag) and (ang_hi, mu), and its four impulses in one more, in a
+// record of kS32Floats; a body stores its accumulator w (6), m^-1, a fixed flag and the world inverse
 // inertia (6, symmetric), in a record of kS32BodyFloats (all fixed bodies share one with m^-1 = I^-1 = 0).  The update
 // of w after a contact changes by dx is m^-1 sum_q lin_q dx_q (negated on the hi side) and I^-1 sum_q ang_q dx_q.
 //
@@ -2632,21 +2632,23 @@ __device__ __forceinline__ uint32_t c32_at(int piece, int q) { return 64u * piec
 constexpr uint32_t kX32 = 192;
 
 // Warps that sweep a step of a scene of these levels: the number (a power of two, up to max_warps) with the least cost.
-// A level of up to eight contacts a warp is a step of quads and a wider one steps of a lane per contact, or, with the
-// rows in L2 (in_l2), more steps of quads.  The cycles of a step, in tens: by turns 400-420 with quads
-// (14 to 600 contacts, one or two warps a step) and 515 with lanes (547 contacts on six levels); in L2 those that fit
-// 200 sweeps over 1565 contacts by one, two and four warps (27256, 16884, 9525 us).
+// In a slab (one or two warps) a level of up to eight contacts a warp is a step of quads and a wider one steps of a lane
+// per contact; in tens of cycles a step by turns takes 400-420 with quads (14 to 600 contacts) and 515 with lanes (547
+// contacts on six levels).  With the rows in L2 (in_l2; scenes with too many bodies for the ring, whose warps are given)
+// wide levels are cut into more steps of quads.  200 sweeps of 5441 contacts on 193 levels with one, two, four and eight
+// warps: 82.0, 53.3, 38.8 and 40.3 ms; of 7503 on 201: 133, 78.6, 52.8, 52.0; of 3288 on 70: 32.8, 19.7, 13.3, 12.4;
+// of 1248 on 56: 5.4, 5.3, 5.5, 5.3.  The rule takes eight in the first three, so it is off the best by 4 % at most there.
 // Every warp of the block counts for itself.
 __device__ __forceinline__ int s32_warps(const int* ptr, int L, int max_warps, bool in_l2) {
     int cost[4] = {0, 0, 0, 0};
-    const int quads[4] = {in_l2 ? 120 : 40, in_l2 ? 125 : 42, in_l2 ? 112 : 60, in_l2 ? 140 : 90};
-    const int lanes[4] = {50, 52, 70, 100};
+    const int quads[4] = {in_l2 ? 120 : 40, in_l2 ? 125 : 42, 112, 140};   // the last two in L2 alone
+    const int lanes[2] = {50, 52};
     for (int l = threadIdx.x & 31; l < L; l += 32) {
         const int n = ptr[l + 1] - ptr[l];
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
             const int q = 8 << w;
-            cost[w] += in_l2 ? (n + q - 1) / q * quads[w] : n <= q ? quads[w] : (n + 4 * q - 1) / (4 * q) * lanes[w];
+            cost[w] += in_l2 ? (n + q - 1) / q * quads[w] : n <= q ? quads[w] : (n + 4 * q - 1) / (4 * q) * lanes[w & 1];
         }
     }
     int best = 1, least = INT_MAX;
@@ -3682,7 +3684,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_solve_blocks(const StepArgs a, 
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// integration (state_storage.py:239 velocity_update, :251 position_update): thread per body
+// integration (state_storage.py:239 velocity_update, :251 position_update)
 // ---------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void position_update(double* xb, const double* ub, double dt) {
     for (int i = 0; i < 3; ++i) xb[i] = xb[i] + ub[i] * dt;
@@ -3756,7 +3758,7 @@ __global__ void k_post_apply(const StepArgs a) {
     if (moves && d == 0) position_update(a.bd.x + 7 * b, dr, 1.0);
 }
 
-// energies and largest penetration (state_storage.py:188, contacts.py:222): thread per scene, body order
+// energies and largest penetration (state_storage.py:188, contacts.py:222)
 // one warp per scene: the deepest gap and the pair / candidate counts by warp reductions (order-free), the
 // energy sums by lane 0 in body order (their rounding follows state_storage.py:188-237)
 __device__ __forceinline__ void scene_summary(const StepArgs& a, int s) {
@@ -3769,7 +3771,7 @@ __device__ __forceinline__ void scene_summary(const StepArgs& a, int s) {
     const int p0 = a.ws.pair_cnt[R.b0], p1 = a.ws.pair_cnt[R.b1];
     int ovl = 0, cand = 0;
     if (a.pr.profiling)
-        for (int p = p0 + lane; p < p1; p += 32) { ovl += a.ws.pair_ovl[p]; cand += a.ws.pair_itemsA[p]; }
+        for (int p = p0 + lane; p < p1; p += 32) { ovl += a.ws.pair_ovl[p]; cand += a.ws.pair_n_items[p]; }
     for (int o = 16; o > 0; o >>= 1) {
         ovl += __shfl_xor_sync(0xffffffffu, ovl, o);
         cand += __shfl_xor_sync(0xffffffffu, cand, o);
@@ -4074,7 +4076,7 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
         const int max_clusters = (sh->max_shape_triangles + 31) / 32;
         const size_t mid_smem = (size_t)kWarpsPerBlock * 3 * sizeof(uint32_t) * max_clusters;
         k_mid<<<mid_blocks, kBlock, mid_smem, st>>>(a, max_clusters); note_launch();
-        // no pair of single-cluster shapes (up to 32 triangles) is a wide one
+        // shapes of up to four clusters (128 triangles) make no wide pair
         if (max_clusters * max_clusters > kMidLight) {
             k_mid_wide<<<148 * 4, 32 * kMidWideWarps, mid_wide_bytes(max_clusters), st>>>(a, max_clusters); note_launch();
         }
