@@ -12,7 +12,6 @@ namespace rb {
 
 struct d3 { double x, y, z; };
 
-__device__ __forceinline__ d3 mk(double x, double y, double z) { return d3{x, y, z}; }
 __device__ __forceinline__ d3 ld3(const double* p) { return d3{p[0], p[1], p[2]}; }
 __device__ __forceinline__ void st3(double* p, d3 a) { p[0] = a.x; p[1] = a.y; p[2] = a.z; }
 __device__ __forceinline__ d3 sub(d3 a, d3 b) { return d3{a.x - b.x, a.y - b.y, a.z - b.z}; }

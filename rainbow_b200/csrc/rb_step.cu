@@ -2627,8 +2627,7 @@ struct GlPtr {
     __device__ __forceinline__ void set(float4 v) const { *reinterpret_cast<float4*>(p) = v; }
 };
 constexpr uint32_t kC32 = sizeof(float) * kS32Floats, kB32 = sizeof(float) * kS32BodyFloats;   // record strides
-// a contact record's offsets: piece j (0..2) of row q, and the impulses
-__device__ __forceinline__ uint32_t c32_at(int piece, int q) { return 64u * piece + 16u * q; }
+// a contact record's offsets: piece j (0..2) of row q at 64 j + 16 q, and the impulses
 constexpr uint32_t kX32 = 192;
 
 // Warps that sweep a step of a scene of these levels: the number (a power of two, up to max_warps) with the least cost.
