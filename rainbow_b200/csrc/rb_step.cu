@@ -4118,14 +4118,16 @@ int rb_step(const rb_shapes* sh, const rb_bodies* bd, const rb_caps* caps, const
     const size_t block_smem = (size_t)6 * sizeof(double) * smem_bodies;
     const int bg = bd->n_scenes < 148 * 16 ? bd->n_scenes : 148 * 16;
     // Threads of a scene's block: a scene that has an SM to itself takes as many warps as the registers allow (255 a
-    // thread), so that wide levels and the rebuilds of w have them; more scenes than SMs share them, two or four blocks
-    // to an SM, where the accumulators leave room for as many.  A batch whose largest scene is more than four times the
-    // mean waits for that scene: it takes the most threads too.  (400 piles of up to 200 bodies and one of 5000: 454 ms a
-    // step by the number of scenes alone, 131 so; 300 of up to 40 and one of 1500: 729 and 251; 300 piles of up to 200:
-    // 73 either way, with 64 threads.)
+    // thread), so that wide levels and the rebuilds of w have them; more scenes than SMs share them, two blocks to an SM
+    // or, with scenes so small or so many that two warps each do better, four, where the accumulators leave room for as
+    // many.  A batch whose largest scene is more than four times the mean waits for that scene: it takes the most threads
+    // too.  (Measured, ms a step with 128 and with 64 threads: 300 piles of 8-200 bodies 57 and 74, 600 101 and 128, 1500
+    // 67.8 and 68.7, 4000 107 and 105; 600 piles of 30-60 bodies 66 and 54, 600 of 4-30 25.7 and 25.4, 1500 20.4 and 17.2.
+    // 400 piles of up to 200 bodies and one of 5000: 454 with 64, 131 with 256; 300 of up to 40 and one of 1500: 729, 251.)
     const int share = (int)std::min<size_t>((bd->n_scenes + 147) / 148, (227 * 1024) / (block_smem + 2048));
     const bool uneven = (int64_t)bd->max_scene_bodies * bd->n_scenes > 4 * (int64_t)N;
-    const int solve_threads = share <= 1 || uneven ? kSolveBlock : share == 2 ? kSolveBlock / 2 : kSolveBlock / 4;
+    const bool small = bd->max_scene_bodies <= 64 || bd->n_scenes > 8 * 148;
+    const int solve_threads = share <= 1 || uneven ? kSolveBlock : share == 2 || !small ? kSolveBlock / 2 : kSolveBlock / 4;
     if (pr->precision != RB_PRECISION_FP64) {
         k_fp32_classes<<<1, 1024, 0, st>>>(a, small_slab, mid_slab); note_launch();
         // FP32 phase, four size classes side by side: warp teams with small slabs (28 KB unless tuned), warp

@@ -29,3 +29,17 @@ def test_a_large_scene_among_small_ones(n_small, big):
             wx, wu = xs[s0[k]:s0[k + 1]], us[s0[k]:s0[k + 1]]
         np.testing.assert_array_equal(x[st[i]:st[i + 1]], wx)
         np.testing.assert_array_equal(u[st[i]:st[i + 1]], wu)
+
+
+@pytest.mark.parametrize("n_scenes,bodies", [(297, 63), (297, 66), (1184, 66), (1185, 66)])
+def test_even_batches_of_small_and_larger_scenes(n_scenes, bodies):
+    from rainbow_b200 import world as W
+    one = chips(bodies - 1)
+    rp = W.make_rb_params(W.params_from_vector(one["params"]))
+    many, alone = W.DeviceWorld([one] * n_scenes, device="cuda:0"), W.DeviceWorld(one, device="cuda:0")
+    for _ in range(2):
+        assert [w.step(rp) for w in (many, alone)] == [0, 0]
+    (x, u), (x1, u1) = many.state(), alone.state()
+    assert alone.stats()[0].n_contacts > bodies // 2
+    np.testing.assert_array_equal(x.reshape(n_scenes, bodies, 7), np.broadcast_to(x1, (n_scenes, bodies, 7)))
+    np.testing.assert_array_equal(u.reshape(n_scenes, bodies, 6), np.broadcast_to(u1, (n_scenes, bodies, 6)))
